@@ -114,7 +114,9 @@ __global__ void k_cell_keys(StepArgs a) {
 }
 
 // ------------------------------------------------------------------- scan
-// Exclusive scan of cell_count[0, ncells) into cell_start[0, ncells].
+// Exclusive scan of cell_count[0, ncells) into cell_start[0, ncells].  A grid
+// larger than the cell arrays has raised the status in k_grid_setup: nothing
+// is read or written then (the step is run again once the arrays have grown).
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanChunk = kScanThreads * kScanItems;
@@ -146,9 +148,10 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *smem, int &total
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_blocks(const int *in, int *out, int *sums, const long long *np_dev,
-                                                              long long n_static) {
+                                                              const DevStatus *status) {
     __shared__ int smem[32];
-    long long n = np_dev ? *np_dev : n_static;
+    if (status->code) return;
+    long long n = *np_dev;
     long long base = (long long)blockIdx.x * kScanChunk;
     int v[kScanItems];
     int local = 0;
@@ -169,8 +172,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_blocks(const int *in, int
     if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_sums(int *sums, int nblocks) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(int *sums, int nblocks, const DevStatus *status) {
     __shared__ int smem[32];
+    if (status->code) return;
     int carry = 0;
     for (int base = 0; base < nblocks; base += kScanThreads) {
         int idx = base + threadIdx.x;
@@ -183,8 +187,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(int *sums, int nbloc
     if (threadIdx.x == 0) sums[nblocks] = carry;
 }
 
-__global__ void k_scan_add(int *out, const int *sums, const long long *np_dev, long long n_static, int nblocks) {
-    long long n = np_dev ? *np_dev : n_static;
+__global__ void k_scan_add(int *out, const int *sums, const long long *np_dev, int nblocks, const DevStatus *status) {
+    if (status->code) return;
+    long long n = *np_dev;
     long long base = (long long)blockIdx.x * kScanChunk;
     int add = sums[blockIdx.x];
     for (int k = threadIdx.x; k < kScanChunk; k += blockDim.x) {
@@ -195,12 +200,12 @@ __global__ void k_scan_add(int *out, const int *sums, const long long *np_dev, l
 }
 
 static void device_exclusive_scan(const int *in, int *out, int *sums, const long long *n_dev, long long cap,
-                                  cudaStream_t s) {
+                                  const DevStatus *status, cudaStream_t s) {
     int nblocks = (int)((cap + kScanChunk - 1) / kScanChunk);
     if (nblocks < 1) nblocks = 1;
-    k_scan_blocks<<<nblocks, kScanThreads, 0, s>>>(in, out, sums, n_dev, cap);
-    k_scan_sums<<<1, kScanThreads, 0, s>>>(sums, nblocks);
-    k_scan_add<<<nblocks, 256, 0, s>>>(out, sums, n_dev, cap, nblocks);
+    k_scan_blocks<<<nblocks, kScanThreads, 0, s>>>(in, out, sums, n_dev, status);
+    k_scan_sums<<<1, kScanThreads, 0, s>>>(sums, nblocks, status);
+    k_scan_add<<<nblocks, 256, 0, s>>>(out, sums, n_dev, nblocks, status);
 }
 
 // --------------------------------------------------------------- scatter
@@ -377,7 +382,7 @@ void launch_grid_setup(const StepArgs &a, cudaStream_t s) { k_grid_setup<<<1, 32
 void launch_cell_build(const StepArgs &a, cudaStream_t s) {
     cudaMemsetAsync(a.cell_count, 0, sizeof(int) * (size_t)a.cell_cap, s);
     k_cell_keys<<<grid_blocks(a.n, 256), 256, 0, s>>>(a);
-    device_exclusive_scan(a.cell_count, a.cell_start, a.scan_sums, &a.grid->ncells, a.cell_cap, s);
+    device_exclusive_scan(a.cell_count, a.cell_start, a.scan_sums, &a.grid->ncells, a.cell_cap, a.status, s);
     k_cell_scatter<<<grid_blocks(a.n, 256), 256, 0, s>>>(a);
     {
         long long b = (a.cell_cap + 7) / 8;   // 8 warps (cells) per block
