@@ -326,8 +326,11 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepAr
 #pragma unroll
                 for (int l = 0; l < 3; ++l) acc[n] = fma(massj * ds[3 * sym_index(n, m) + l], invB[l][m], acc[n]);
     }
+    // the corrected form's acceleration was formed from complete sums on every lane
+    if (DISC == 0) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) acc[c] = sub_sum<L>(acc[c]);
+        for (int c = 0; c < 3; ++c) acc[c] = sub_sum<L>(acc[c]);
+    }
     // per-particle tail on lane 0 of each sub-warp
     if (live && lane == 0) {
         const int i = a.cell_list[t];

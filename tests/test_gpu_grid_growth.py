@@ -23,7 +23,7 @@ def split_bar(gap_cells):
 
 
 @pytest.mark.parametrize("precision", [_abi.PREC_FP64_EXACT, _abi.PREC_MIXED])
-@pytest.mark.parametrize("gap", [6000, 9000])
+@pytest.mark.parametrize("gap", [8000, 25000])
 def test_grid_grows(precision, gap):
     deck = split_bar(gap)
     bystander = Solver(taylor_bar(dx=0.8e-3), _abi.PREC_FP64_EXACT)
