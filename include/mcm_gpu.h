@@ -308,14 +308,15 @@ int mcm_gpu_adjoint_backward(mcm_gpu_handle *h, const double *xbar, const double
  * combined over a different number of block partials.  Zero fields keep the
  * current value. */
 typedef struct {
-    int search_threads;      /* threads per block of the search: 64, 128 or 256 */
+    int search_threads;      /* threads per block of the search: 64 or 128 (256 runs as 128) */
     int pair_threads;        /* threads per block of the gathers: 64, 128 or 256 */
     int pair_blocks_per_sm;  /* blocks per SM the gathers' persistent grid is sized for: 1..16 (reported as
                                 0 while it is the blocks resident per SM, the default) */
     int nbr_stride;          /* neighbour-table row width in entries (rounded up to 4; still regrown
                                 when a list outgrows it) */
-    int search_kind;         /* 1: one thread per particle (the default), 2: one warp per particle,
-                                3: one warp per cell (candidates staged in shared memory) */
+    int search_kind;         /* 1: by size, one thread per particle for bodies that fill the GPU, four or
+                                eight lanes per particle for smaller ones (the default), 2: eight lanes
+                                per particle, 3: one warp per cell (candidates staged in shared memory) */
     int pair_kind;           /* mixed-precision strain and momentum gathers: 1 neighbour records
                                 through L1 (the default), 2 each block's rows of neighbour cells
                                 staged in shared memory (the same sums) */

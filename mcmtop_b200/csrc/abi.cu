@@ -68,10 +68,6 @@ DevParams make_params(const mcm_gpu_config &c, int nmat) {
     p.contact = (c.contacttype > 0 && nmat > 1) ? 1 : 0;
     p.skin = c.nbr_skin > 0.0 ? c.nbr_skin : 0.0;
     p.kahan = (c.precision == MCM_PREC_MIXED && c.compensated_sums) ? 1 : 0;
-    // the sums of the FP64-fast and mixed steps do not follow the reference's
-    // neighbour order: their cells are kept in x order, which lets the search
-    // window each row of cells in x
-    p.xsort = c.precision != MCM_PREC_FP64_EXACT ? 1 : 0;
     p.veloc_opt = c.veloc_opt;
     for (int k = 0; k < 3; ++k) p.base_a[k] = c.baseaccel ? c.base_a[k] : 0.0;
     DevPlanes &pl = p.planes;
@@ -120,7 +116,10 @@ int alloc_particles(mcm_gpu_handle *h) {
     if ((st = dalloc(h, &h->A.cell_list, np))) return st;
     if ((st = dalloc(h, &h->A.cpos, np))) return st;
     if ((st = dalloc(h, &h->A.cposf, np))) return st;
-    if (h->A.prm.xsort && (st = dalloc(h, &h->A.cposg, np))) return st;
+    if ((st = dalloc(h, &h->A.snx, 4 * (np + 32)))) return st;   // the search reads groups of four past the end
+    h->A.sny = h->A.snx + (np + 32);
+    h->A.snz = h->A.sny + (np + 32);
+    h->A.snh = h->A.snz + (np + 32);
     if ((st = dalloc(h, &h->A.cmat, np))) return st;
     if ((st = dalloc(h, &h->A.ckey, np))) return st;
     if ((st = dalloc(h, &h->A.reorder_tmp, np))) return st;
@@ -698,6 +697,7 @@ int mcm_gpu_create(const mcm_gpu_config *cfg, const mcm_gpu_material *mats, int 
     h->A.npad = h->npad;
     h->A.nmat = nmat;
     h->A.split_mode = 1;
+    h->A.share = 1;
     h->A.prm = make_params(h->cfg, nmat);
     h->A.prm.asym = cap_model ? 1 : 0;
     // materials
@@ -761,7 +761,7 @@ int mcm_gpu_destroy(mcm_gpu_handle *h) {
     void *ptrs[] = {h->d_fields, h->d_stage, h->A.frec0, h->A.gfrec1, h->A.gfrec2,
                     h->d_ints, h->d_mats, h->d_scalars, h->d_nppermat,
                     h->A.key, h->A.cell_list, h->A.nnbr, h->A.gnnbr, h->A.rec0, h->A.rec1, h->A.rec2,
-                    h->A.cpos, h->A.cposf, h->A.cposg, h->A.cmat, h->A.ckey, h->A.reorder_tmp, h->A.reorder_grp, h->A.nidx,
+                    h->A.cpos, h->A.cposf, h->A.snx, h->A.cmat, h->A.ckey, h->A.reorder_tmp, h->A.reorder_grp, h->A.nidx,
                     h->A.red, h->A.cell_count, h->A.cell_start, h->A.scan_sums, h->A.gcell,
                     h->A.layer_count, h->A.layer_off, h->A.gx, h->A.gy, h->A.gz, h->A.gvx, h->A.gvy,
                     h->A.gvz, h->A.gmass, h->A.gh, h->A.ghold, h->A.grho, h->A.gpar, h->A.gmat, h->A.gflip,

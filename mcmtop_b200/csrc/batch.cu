@@ -178,7 +178,9 @@ int capture(mcm_gpu_batch *b) {
                 if (b->lane_of[k] != l) continue;
                 mcm_gpu_handle *h = b->bodies[k];
                 h->stream = b->lane_streams[l];
+                h->A.share = std::min(b->lanes, nb);
                 enqueue_iteration(h);
+                h->A.share = 1;
                 h->stream = own[k];
             }
         for (int l = 0; l < b->lanes; ++l) {

@@ -73,6 +73,7 @@ __global__ void k_grid_setup(StepArgs a) {
         if (c1 == 1 || c1 == 2) g.gridlim[i] = g.gridlim[i] + 1;
     }
     g.pad = 0;
+    for (int i = 0; i < 3; ++i) g.cell[i] = 1.0 / g.gridsize[i];
     g.ncells = (long long)g.gridlim[0] * g.gridlim[1] * g.gridlim[2];
     if (bad || g.ncells >= (1LL << 31)) {
         raise_status(a.status, MCM_EGRID_TOO_LARGE);
@@ -80,7 +81,8 @@ __global__ void k_grid_setup(StepArgs a) {
         a.status->req_cells = g.ncells;
         raise_status(a.status, MCM_EGRID_OVERFLOW);
     }
-    g.hcut = 0.0;   // raised by k_cell_records
+    g.hcut = 0.0;                                     // raised by k_cell_records
+    g.hmin = __longlong_as_double(0x7fffffffffffffffll);   // lowered by k_cell_records
     *a.grid = g;
     *a.ngp = 0;
     *a.n_inside = 0;
@@ -233,16 +235,18 @@ __global__ void k_cell_scatter(StepArgs a) {
     }
 }
 
-// Candidate records in cell order (positions at neighbour time).
-// Candidate records in cell order: FP64 position and h, and an FP32 copy of
-// the position relative to the origin of the particle's own cell, which the
-// search uses to decide all but the near-tie candidates.
-__global__ void __launch_bounds__(256) k_cell_records(StepArgs a) {
-    __shared__ unsigned long long smax[8];
+// Candidate records in cell order (positions at neighbour time): FP64 position
+// and h, and the FP32 coordinates by which the search decides all but the
+// near-tie candidates: negated, one array each, x relative to the grid origin
+// (the candidates of a row's two or three cells share one frame in x), y and z
+// relative to the origin of the particle's own cell.  cposf (all three
+// relative to the cell, h) is kept for the searches that read it.
+__global__ void __launch_bounds__(256) k_cell_records(StepArgs a, int with_cposf) {
+    __shared__ unsigned long long smax[8], smin[8];
     if (a.status->code) return;
     const double *X = a.F.f[FX], *Y = a.F.f[FY], *Z = a.F.f[FZ], *H = a.F.f[FH];
     const DevGrid g = *a.grid;
-    unsigned long long hbits = 0ull;   // h > 0: the bit pattern orders like the value
+    unsigned long long hbits = 0ull, lbits = ~0ull;   // h > 0: the bit pattern orders like the value
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x) {
         int i = a.cell_list[p];
         const double x = X[i], y = Y[i], z = Z[i], h = H[i];
@@ -260,29 +264,37 @@ __global__ void __launch_bounds__(256) k_cell_records(StepArgs a) {
             r.z = (float)(z - cell_origin(g, 2, bz));
             const unsigned long long hb = (unsigned long long)__double_as_longlong(h);
             hbits = hb > hbits ? hb : hbits;
+            lbits = hb < lbits ? hb : lbits;
         }
-        a.cposf[p] = r;
-        // the windowed search's copy: x relative to the grid origin, so that the
-        // candidates of a row's two or three cells share one frame in x
-        if (a.cposg) a.cposg[p] = make_float4((float)(x - g.gridmin[0]), r.y, r.z, r.w);
+        if (with_cposf) a.cposf[p] = r;
+        a.snx[p] = -(float)(x - g.gridmin[0]);
+        a.sny[p] = -r.y;
+        a.snz[p] = -r.z;
+        a.snh[p] = r.w;
     }
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long v = __shfl_xor_sync(0xffffffffu, hbits, o);
+        const unsigned long long u = __shfl_xor_sync(0xffffffffu, lbits, o);
         hbits = v > hbits ? v : hbits;
+        lbits = u < lbits ? u : lbits;
     }
-    if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = hbits;
+    if ((threadIdx.x & 31) == 0) { smax[threadIdx.x >> 5] = hbits; smin[threadIdx.x >> 5] = lbits; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) hbits = smax[w] > hbits ? smax[w] : hbits;
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
+            hbits = smax[w] > hbits ? smax[w] : hbits;
+            lbits = smin[w] < lbits ? smin[w] : lbits;
+        }
         atomicMax(reinterpret_cast<unsigned long long *>(&a.grid->hcut), hbits);
+        atomicMin(reinterpret_cast<unsigned long long *>(&a.grid->hmin), lbits);
     }
 }
 
 // Per-cell order: descending reference index (head insertion in
 // MCM/mcm_setuplist.f90:126-130 over i = 1..np ascending), the order of the
-// reference's lists.  With xsort (steps whose sums do not follow that order)
-// ascending x, ties by descending reference index: a row of x-adjacent cells
-// is then one x-sorted range, which the search windows in x.
+// reference's lists.  (Ascending x, which lets a search window its rows,
+// measured slower for every later kernel of the FP64-fast and mixed steps:
+// 1.25 against 1.23 ms per mixed step of the 685 824-particle bar.)
 // One warp per cell: each lane takes one of the cell's particles (cells of up
 // to 32, the common case) or up to kSortPer of them, and counts how many of
 // the cell's particles come before each (a rank sort: the order is total, so
@@ -290,14 +302,9 @@ __global__ void __launch_bounds__(256) k_cell_records(StepArgs a) {
 // written back.  Cells of more than 32 * kSortPer particles are sorted by
 // insertion in one lane.
 constexpr int kSortPer = 4;
-__device__ __forceinline__ bool cell_before(bool xs, double xa, int oa, double xb, int ob) {
-    return xs ? (xa < xb || (xa == xb && oa > ob)) : oa > ob;
-}
 __global__ void __launch_bounds__(256) k_cell_sort(StepArgs a) {
     if (a.status->code) return;
     const long long ncells = a.grid->ncells;
-    const bool xs = a.prm.xsort != 0;
-    const double *X = a.F.f[FX];
     const int lane = threadIdx.x & 31;
     const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
     for (long long c = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += nw) {
@@ -309,42 +316,33 @@ __global__ void __launch_bounds__(256) k_cell_sort(StepArgs a) {
             const bool on = lane < n;
             const int v = on ? a.cell_list[s + lane] : 0;
             const int o = on ? a.F.orig[v] : 0;
-            const double x = (on && xs) ? X[v] : 0.0;
             int rank = 0;
-            for (int k = 0; k < n; ++k) {
-                const double xb = __shfl_sync(0xffffffffu, x, k);
-                const int ob = __shfl_sync(0xffffffffu, o, k);
-                rank += cell_before(xs, xb, ob, x, o) ? 1 : 0;
-            }
+            for (int k = 0; k < n; ++k) rank += __shfl_sync(0xffffffffu, o, k) > o ? 1 : 0;
             __syncwarp();
             if (on) a.cell_list[s + rank] = v;
             __syncwarp();
         } else if (n <= 32 * kSortPer) {
             int v[kSortPer], o[kSortPer], rank[kSortPer];
-            double x[kSortPer];
 #pragma unroll
             for (int u = 0; u < kSortPer; ++u) {
                 const int j = lane + 32 * u;
                 v[u] = j < n ? a.cell_list[s + j] : 0;
                 o[u] = j < n ? a.F.orig[v[u]] : 0;
-                x[u] = (j < n && xs) ? X[v[u]] : 0.0;
                 rank[u] = 0;
             }
             for (int k0 = 0; k0 < n; k0 += 32) {
                 // the chunk's keys, one per lane, broadcast by shuffles
                 const int uk = k0 >> 5;
-                double xk = 0.0;
                 int ok = 0;
 #pragma unroll
                 for (int u = 0; u < kSortPer; ++u)
-                    if (u == uk) { xk = x[u]; ok = o[u]; }
+                    if (u == uk) ok = o[u];
                 const int m = n - k0 < 32 ? n - k0 : 32;
                 for (int k = 0; k < m; ++k) {
-                    const double xb = __shfl_sync(0xffffffffu, xk, k);
                     const int ob = __shfl_sync(0xffffffffu, ok, k);
 #pragma unroll
                     for (int u = 0; u < kSortPer; ++u)
-                        if (lane + 32 * u < n && cell_before(xs, xb, ob, x[u], o[u])) ++rank[u];
+                        if (lane + 32 * u < n && ob > o[u]) ++rank[u];
                 }
             }
             __syncwarp();
@@ -356,12 +354,9 @@ __global__ void __launch_bounds__(256) k_cell_sort(StepArgs a) {
             for (int k = s + 1; k < e; ++k) {
                 const int v = a.cell_list[k];
                 const int ov = a.F.orig[v];
-                const double xv = xs ? X[v] : 0.0;
                 int m = k - 1;
-                while (m >= s) {
-                    const int u = a.cell_list[m];
-                    if (!cell_before(xs, xv, ov, xs ? X[u] : 0.0, a.F.orig[u])) break;
-                    a.cell_list[m + 1] = u;
+                while (m >= s && a.F.orig[a.cell_list[m]] < ov) {
+                    a.cell_list[m + 1] = a.cell_list[m];
                     --m;
                 }
                 a.cell_list[m + 1] = v;
@@ -389,7 +384,8 @@ void launch_cell_build(const StepArgs &a, cudaStream_t s) {
         if (b > 148LL * 8) b = 148LL * 8;
         k_cell_sort<<<(unsigned)(b < 1 ? 1 : b), 256, 0, s>>>(a);
     }
-    k_cell_records<<<grid_blocks(a.n, 256) < 148 * 8 ? grid_blocks(a.n, 256) : 148 * 8, 256, 0, s>>>(a);
+    k_cell_records<<<grid_blocks(a.n, 256) < 148 * 8 ? grid_blocks(a.n, 256) : 148 * 8, 256, 0, s>>>(
+        a, a.search_kind == 3 || a.prm.skin > 0.0 ? 1 : 0);
 }
 
 // ------------------------------------------------------------- re-sorting
@@ -595,17 +591,25 @@ void launch_ghosts(const StepArgs &a, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------ search
-// MCM/mcm_ll_neighbours.f90:96-299.  One thread per cell-order position t;
-// the threads of a warp (neighbouring positions, mostly one cell) walk the
-// same rows, so their candidate loads hit the same cache lines.  Candidates
-// are visited in the reference order (rows of the 27-cell neighbourhood in
-// z, y order, cells in x order, each cell's contiguous range of positions),
-// and accepted ones are appended to t's list in that order.  The distance
-// test runs first in FP32 on positions relative to cell origins; only
-// candidates within a narrow band around the cutoff (or all accepted ones
-// when the FP64 minimum distance is wanted) are decided by the reference's
-// FP64 expression, so the sets are the reference's.  Cells whose box lies
-// beyond h_i + max h cannot hold a neighbour and are skipped.
+// MCM/mcm_ll_neighbours.f90:96-299.  The candidates of the particle at
+// cell-order position t are the cells of its 27-cell neighbourhood in z, y, x
+// order, each a contiguous range of positions in the reference's order, so
+// appending the accepted ones in position order gives the reference's lists.
+//
+// Two phases.  First every candidate is reduced to one bit: groups of four
+// aligned positions are read as three 16-byte loads (negated x, y and z lie in
+// arrays of their own), the distances of two candidates are formed by one
+// packed FP32 instruction each, with the cutoff as the chain's starting value,
+// so the sign of the result is the decision and a funnel shift moves it into
+// the mask: about 6 instructions a candidate, without divergence or stores.
+// Then the set bits (one candidate in six) are walked in position order and
+// written.  The FP32 decision is final outside a narrow band around the
+// cutoff, wider than the FP32 rounding; a mask with a candidate inside the
+// band (a signed integer minimum over the results finds it: of the negative
+// floats those nearest zero are the smallest integers) is walked through the
+// reference's FP64 expression before it is written, as all are when the FP64
+// minimum distance is wanted.  Cells whose box lies beyond h_i + max h cannot
+// hold a neighbour and are left out.
 
 __device__ __forceinline__ double exact_d2(double4 a, double4 b) {
     double d = __dsub_rn(b.x, a.x);
@@ -617,433 +621,545 @@ __device__ __forceinline__ double exact_d2(double4 a, double4 b) {
     return s;
 }
 
-// Variants of the search, fixed at compile time so that the candidate loop of
-// the common case (one material, no repulsive contact, no minimum distance)
-// tests none of these flags per candidate.
-enum { kSrchContact = 1, kSrchTwoPass = 2, kSrchMind = 4, kSrchXWin = 8 };
+// Variants of the search, fixed at compile time so that the common case (one
+// material, no repulsive contact, no minimum distance) tests none of them.
+enum { kSrchContact = 1, kSrchTwoPass = 2, kSrchMind = 4 };
 
-template <int V>
-__global__ void __launch_bounds__(256, 4) k_search(StepArgs a) {
-    constexpr bool contact = (V & kSrchContact) != 0;   // contacttype > 0: other materials -> contact list
-    constexpr bool two_pass = (V & kSrchTwoPass) != 0;  // kernel contact between materials: own material first
-    constexpr bool want_mind = (V & kSrchMind) != 0;    // FP64 minimum distance (tcrit option 2, diagnostics)
-    constexpr bool xwin = (V & kSrchXWin) != 0;         // cells in x order: each row windowed in x
-    if (a.status->code) return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= a.n) return;
-    const int np = a.npad;
-    const int cap = a.nstride;
-    const int key = a.ckey[t];
-    const int i = a.cell_list[t];
-    const bool with_self = (a.prm.disctype == 1);
-    int nn = 0, gn = 0, nc = 0, gcn = 0;
-    double mind = 1.0e20;
-    if (key >= 0) {
-        const DevGrid g = *a.grid;
-        int bx, by, bz;
-        cell_coords(key, g.gridlim, bx, by, bz);
-        const int lo1 = by > 1 ? by - 1 : 1, hi1 = by < g.gridlim[1] ? by + 1 : g.gridlim[1];
-        const int lo2 = bz > 1 ? bz - 1 : 1, hi2 = bz < g.gridlim[2] ? bz + 1 : g.gridlim[2];
-        const bool has_l = bx > 1, has_r = bx < g.gridlim[0];
-        const double4 xi = a.cpos[t];
-        const float4 ui = a.cposf[t];
-        const float cs[3] = {(float)(1.0 / g.gridsize[0]), (float)(1.0 / g.gridsize[1]), (float)(1.0 / g.gridsize[2])};
-        const float csm = fmaxf(cs[0], fmaxf(cs[1], cs[2]));
-        // FP32 decision band around the cutoff: the FP32 rounding of d2 and
-        // (h_i + h_j)^2 (a few hundred ulps of csm^2 at most) stays far inside it
-        const float kb = 2.44140625e-4f * csm * csm;
-        const float khi = 1.0f + 2.44140625e-4f, klo = 1.0f - 2.44140625e-4f;
-        const float reach = ui.w + (float)g.hcut;
-        const float reach2 = reach * reach * 1.0009765625f + 9.765625e-4f * csm * csm;
-        // this particle relative to the origins of the left, own and right cell of a row
-        const float qxl = ui.x + cs[0], qxr = ui.x - cs[0];
-        const float gxl = fmaxf(ui.x, 0.0f), gxr = fmaxf(cs[0] - ui.x, 0.0f);
-        // windowed rows: x relative to the grid origin (one frame for the whole
-        // row); its rounding (up to gridlim(1) cells of magnitude) widens the
-        // decision band by gridlim(1) 2^-16 cell^2, 32 times that error's bound
-        const float ugx = xwin ? a.cposg[t].x : 0.0f;
-        const float kbx = kb + (xwin ? (float)g.gridlim[0] * 1.52587890625e-5f * csm * csm : 0.0f);
-        const int mati = a.cmat[t];
-        unsigned *out = a.nidx + (size_t)t * cap;
-        // MCM/mcm_ll_neighbours.f90:150-174, 238-267: other materials'
-        // particles are appended after the own material's with kernel contact
-        // (a second walk), and form the contact list otherwise (the same walk,
-        // each list in walk order)
-        unsigned *cout = contact ? a.cidx + (size_t)t * a.cstride : nullptr;
-        // Windowed common case: accepted entries collect in four registers and
-        // leave as one 16-byte store per four (t's row starts at t * cap
-        // entries, cap a multiple of 4), so a warp's lanes, whose rows lie cap
-        // entries apart, send a quarter of the scattered store requests.
-        const bool vec = (cap & 3) == 0;
-        unsigned b0 = 0u, b1 = 0u, b2 = 0u, b3 = 0u;
-#pragma unroll 1
-        for (int pass = 0; pass < (two_pass ? 2 : 1); ++pass) {
-            for (int nz = lo2; nz <= hi2; ++nz) {
-                const float qz = ui.z + (float)(bz - nz) * cs[2];
-                const float gz = fmaxf(nz < bz ? ui.z : (nz > bz ? cs[2] - ui.z : 0.0f), 0.0f);
-                for (int my = lo1; my <= hi1; ++my) {
-                    const float qy = ui.y + (float)(by - my) * cs[1];
-                    const float gy = fmaxf(my < by ? ui.y : (my > by ? cs[1] - ui.y : 0.0f), 0.0f);
-                    const float gyz = gy * gy + gz * gz;
-                    if (gyz > reach2) continue;
-                    // the row's x-adjacent cells are contiguous in position
-                    // order: one range from the first to the last cell whose
-                    // box is within reach (the own cell always is)
-                    const int kc = (int)cell_key(bx, my, nz, g.gridlim);
-                    const int s1 = a.cell_start[kc], s2 = a.cell_start[kc + 1];
-                    const int rb = (has_l && !(gyz + gxl * gxl > reach2)) ? a.cell_start[kc - 1] : s1;
-                    const int re = (has_r && !(gyz + gxr * gxr > reach2)) ? a.cell_start[kc + 2] : s2;
-                    const unsigned code_yz = (unsigned)(3 * (my - by + 1) + 9 * (nz - bz + 1));
-                    int pb = rb, pe = re;
-                    if (xwin) {
-                        // the row is x-sorted: candidates farther than rxw in x
-                        // are beyond reach (with a margin for FP32 rounding);
-                        // the window's ends by bisection
-                        const float rxw = sqrtf(fmaxf(reach2 - gyz, 0.0f)) * 1.0009765625f + 9.765625e-4f * csm;
-                        int hi = re;
-                        while (pb < hi) {
-                            const int mid = (pb + hi) >> 1;
-                            if (ugx - a.cposg[mid].x > rxw) pb = mid + 1;
-                            else hi = mid;
-                        }
-                        int lo = pb;
-                        while (lo < pe) {
-                            const int mid = (lo + pe) >> 1;
-                            if (ugx - a.cposg[mid].x < -rxw) pe = mid;
-                            else lo = mid + 1;
-                        }
-                    }
-                    if constexpr (xwin && !contact && !two_pass && !want_mind) {
-                        // windowed rows, one material, no minimum distance: the
-                        // accept path is a predicated store, so the lanes stay
-                        // converged (measured: 1.41 against 1.46 ms on the 2M
-                        // bar; on the unwindowed rows of the reference order it
-                        // is slower than the branching loop)
-                        for (int p = pb; p < pe; ++p) {
-                            const float4 c = a.cposg[p];
-                            const float dx = ugx - c.x, dy = qy - c.y, dz = qz - c.z;
-                            const float d2f = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                            const float hsf = ui.w + c.w;
-                            const float r2f = hsf * hsf;
-                            bool in = d2f < fmaf(r2f, khi, kbx) && p != t;
-                            if (in && d2f > fmaf(r2f, klo, -kbx)) {
-                                // near tie: the reference's FP64 test
-                                const double4 cd = a.cpos[p];
-                                const double hs = __dadd_rn(cd.w, xi.w);
-                                in = exact_d2(xi, cd) < __dmul_rn(hs, hs);
-                            }
-                            const unsigned entry = (unsigned)p | ((code_yz + (p < s1 ? 0u : (p >= s2 ? 2u : 1u))) << 26);
-                            if (vec) {
-                                if (in) { b0 = b1; b1 = b2; b2 = b3; b3 = entry; }
-                                nn += in ? 1 : 0;
-                                if (in && (nn & 3) == 0 && nn <= cap)
-                                    *reinterpret_cast<uint4 *>(out + (nn - 4)) = make_uint4(b0, b1, b2, b3);
-                            } else {
-                                if (in && nn < cap) out[nn] = entry;
-                                nn += in ? 1 : 0;
-                            }
-                        }
-                    } else {
-                    for (int p = pb; p < pe; ++p) {
-                        const float4 c = a.cposf[p];
-                        const bool left = p < s1, right = p >= s2;
-                        const float qx = left ? qxl : (right ? qxr : ui.x);
-                        const float dx = qx - c.x, dy = qy - c.y, dz = qz - c.z;
-                        const float d2f = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                        const float hsf = ui.w + c.w;
-                        const float r2f = hsf * hsf;
-                        if (d2f >= fmaf(r2f, khi, kb)) continue;
-                        if (p == t) continue;
-                        double d2 = 0.0;
-                        if (want_mind || d2f > fmaf(r2f, klo, -kb)) {
-                            // near tie (or mindist wanted): the reference's FP64 test
-                            const double4 cd = a.cpos[p];
-                            d2 = exact_d2(xi, cd);
-                            const double hs = __dadd_rn(cd.w, xi.w);
-                            if (!(d2 < __dmul_rn(hs, hs))) continue;
-                        }
-                        const unsigned code = (code_yz + (left ? 0u : (right ? 2u : 1u))) << 26;
-                        if (contact) {
-                            if (a.cmat[p] != mati) {
-                                if (nc < a.cstride) cout[nc] = (unsigned)p | code;
-                                ++nc;
-                                continue;
-                            }
-                        } else if (two_pass) {
-                            if ((a.cmat[p] == mati) != (pass == 0)) continue;
-                        }
-                        if (want_mind) mind = fmin(mind, d2);
-                        if (nn < cap) out[nn] = (unsigned)p | code;
-                        ++nn;
-                    }
-                    }
-                }
-            }
-        }
-        if constexpr (xwin && !contact && !two_pass && !want_mind) {
-            if (vec) {
-                // the last nn % 4 accepted entries are still in b(4 - nn % 4) .. b3
-                const int r = nn & 3;
-                if (r >= 3 && nn - 3 < cap) out[nn - 3] = b1;
-                if (r >= 2 && nn - 2 < cap) out[nn - 2] = b2;
-                if (r >= 1 && nn - 1 < cap) out[nn - 1] = b3;
-            }
-        }
-        if (nn > cap) {
-            atomicMax(&a.status->req_stride, nn);
-            raise_status(a.status, MCM_ENBR_OVERFLOW, i);
-        }
-        if (contact && nc > a.cstride) {
-            atomicMax(&a.status->req_cstride, nc);
-            raise_status(a.status, MCM_ENBR_OVERFLOW, i);
-        }
-        // ghosts: only neighbourhoods that reach a ghost layer
-        if (a.prm.boundary) {
-            const int lo0 = has_l ? bx - 1 : bx, hi0 = has_r ? bx + 1 : bx;
-            const DevPlanes &pl = a.prm.planes;
-            const bool near = (lo0 == 1 && pl.code[0][0]) || (hi0 == g.gridlim[0] && pl.code[1][0]) ||
-                              (lo1 == 1 && pl.code[0][1]) || (hi1 == g.gridlim[1] && pl.code[1][1]) ||
-                              (lo2 == 1 && pl.code[0][2]) || (hi2 == g.gridlim[2] && pl.code[1][2]);
-            if (near) {
-#pragma unroll 1
-                for (int pass = 0; pass < (two_pass ? 2 : 1); ++pass) {
-                    for (int nz = lo2; nz <= hi2; ++nz)
-                        for (int my = lo1; my <= hi1; ++my)
-                            for (int lx = lo0; lx <= hi0; ++lx) {
-                                const int2 gc = a.gcell[(int)cell_key(lx, my, nz, g.gridlim)];
-                                for (int r = 0; r < gc.y; ++r) {
-                                    const int q = gc.x + gc.y - 1 - r;   // chain order: newest first
-                                    const double4 c = make_double4(a.gx[q], a.gy[q], a.gz[q], a.gh[q]);
-                                    const double d2 = exact_d2(xi, c);
-                                    const double hs = __dadd_rn(c.w, xi.w);
-                                    if (d2 < __dmul_rn(hs, hs)) {
-                                        if (contact) {
-                                            if (a.gmat[q] != mati) {
-                                                if (gcn < a.gcstride) a.gcont[(size_t)gcn * np + t] = q;
-                                                ++gcn;
-                                                continue;
-                                            }
-                                        } else if (two_pass) {
-                                            if ((a.gmat[q] == mati) != (pass == 0)) continue;
-                                        }
-                                        mind = fmin(mind, d2);
-                                        if (gn < a.gstride) a.gnbr[(size_t)gn * np + t] = q;
-                                        ++gn;
-                                    }
-                                }
-                            }
-                }
-                if (gn > a.gstride) {
-                    atomicMax(&a.status->req_gstride, gn);
-                    raise_status(a.status, MCM_ENBR_OVERFLOW, i);
-                }
-                if (contact && gcn > a.gcstride) {
-                    atomicMax(&a.status->req_gcstride, gcn);
-                    raise_status(a.status, MCM_ENBR_OVERFLOW, i);
-                }
-            }
-        }
-        mind = sqrt(mind);
-    }
-    if (with_self) nn += 1;   // MCM/mcm_ll_neighbours.f90:288-299 (for every particle)
-    a.nnbr[t] = nn;
-    a.gnnbr[t] = gn;
-    if (contact) { a.ncont[t] = nc; a.gncont[t] = gcn; }
-    if (want_mind) a.F.f[FMINDIST][i] = mind;
-    atomicMax(&a.status->max_nbr, nn);
-    atomicMax(&a.status->max_gnbr, gn);
+// What the search of one particle needs of it and of the grid.
+struct Seeker {
+    double4 xi;
+    float qx, ux, uy, uz;     // x relative to the grid origin; x, y, z to the own cell's
+    float cs[3];              // cell size
+    float hi, reach2, kb;     // own h; squared box reach; decision band
+    bool uni;                 // one smoothing length for all
+    float thr;                // then: minus the upper cutoff
+    int tie_at;               // results below this as signed integers lie in the band
+    int key, gl0, gl1;        // own cell, the grid's extent in x and y
+    int bx, by, bz, lo1, hi1, lo2, hi2;
+    bool has_l, has_r;
+    // key of the own cell's neighbour in row (my, nz)
+    __device__ __forceinline__ int row_key(int my, int nz) const { return key + gl0 * ((my - by) + gl1 * (nz - bz)); }
+};
+constexpr float kRelBand = 3.814697265625e-6f;   // 2^-18
+
+__device__ __forceinline__ Seeker make_seeker(const StepArgs &a, const DevGrid &g, int t, int key) {
+    Seeker k;
+    k.key = key;
+    k.gl0 = g.gridlim[0];
+    k.gl1 = g.gridlim[1];
+    cell_coords(key, g.gridlim, k.bx, k.by, k.bz);
+    k.lo1 = k.by > 1 ? k.by - 1 : 1;
+    k.hi1 = k.by < g.gridlim[1] ? k.by + 1 : g.gridlim[1];
+    k.lo2 = k.bz > 1 ? k.bz - 1 : 1;
+    k.hi2 = k.bz < g.gridlim[2] ? k.bz + 1 : g.gridlim[2];
+    k.has_l = k.bx > 1;
+    k.has_r = k.bx < g.gridlim[0];
+    k.xi = a.cpos[t];
+    for (int d = 0; d < 3; ++d) k.cs[d] = (float)g.cell[d];
+    const float csm = fmaxf(k.cs[0], fmaxf(k.cs[1], k.cs[2]));
+    k.hi = (float)k.xi.w;
+    k.qx = -a.snx[t];
+    k.uy = -a.sny[t];
+    k.uz = -a.snz[t];
+    k.ux = (float)(k.xi.x - cell_origin(g, 0, k.bx));
+    // With u = 2^-24 the coordinates, their differences and the sum of squares
+    // round by less than (4 gridlim(1) + 30) u cell^2 and the cutoff by 5 u of
+    // itself: the band is 4 and 8 times that.
+    k.kb = (1.52587890625e-5f + (float)g.gridlim[0] * 9.5367431640625e-7f) * csm * csm;
+    const float reach = k.hi + (float)g.hcut;
+    k.reach2 = reach * reach * 1.0009765625f + 9.765625e-4f * csm * csm;
+    k.uni = g.hmin == g.hcut;
+    const float r = k.hi + k.hi;
+    k.thr = -(r * r * (1.0f + kRelBand) + k.kb);
+    k.tie_at = __float_as_int(-(reach * reach * (2.0f * kRelBand) * 1.0009765625f + 2.0f * k.kb));
+    return k;
+}
+// squared y-z distance of the row (my, nz)'s boxes
+__device__ __forceinline__ float row_gap2(const Seeker &k, int my, int nz) {
+    const float gz = fmaxf(nz < k.bz ? k.uz : (nz > k.bz ? k.cs[2] - k.uz : 0.0f), 0.0f);
+    const float gy = fmaxf(my < k.by ? k.uy : (my > k.by ? k.cs[1] - k.uy : 0.0f), 0.0f);
+    return gy * gy + gz * gz;
 }
 
-// The same search with one warp per position t (search_kind 2; on the
-// 2 034 720-particle bar it takes 2.1x the time of k_search, whose threads
-// share candidate rows through L1, so it is only a tuning alternative for
-// small bodies).  The lanes take consecutive
-// candidates of a row (the up to three cells of a row are contiguous in
-// position order), so every lane runs the same loop and the candidate loads
-// are coalesced.  Accepted candidates are compacted with a ballot in lane
-// order, which is position order, so t's list is the one k_search builds:
-// rows in z, y order, cells in x order, positions ascending.  The FP32
-// decision and the FP64 tie test are k_search's expressions.
-__global__ void __launch_bounds__(256) k_search_warp(StepArgs a) {
-    if (a.status->code) return;
-    const int lane = threadIdx.x & 31;
-    const int t = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
-    if (t >= a.n) return;                       // warp-uniform
-    const unsigned below = (1u << lane) - 1u;
+// The decision bits of groups g0 .. g0 + m - 1 (1 <= m <= 8), candidate c at
+// bit 31 - c; least: the signed minimum over the results.  Groups are taken
+// two at a time, so one group past the range may be read (the arrays are
+// padded) and positions outside the caller's range have to be masked off.
+// UNI: one smoothing length; otherwise the candidate's own h enters the cutoff.
+template <bool UNI>
+__device__ __forceinline__ unsigned group_bits(const StepArgs &a, int g0, int m, float qx, float qy, float qz,
+                                               const Seeker &k, int &least) {
+    const float4 *X = reinterpret_cast<const float4 *>(a.snx) + g0;
+    const float4 *Y = reinterpret_cast<const float4 *>(a.sny) + g0;
+    const float4 *Z = reinterpret_cast<const float4 *>(a.snz) + g0;
+    const float4 *H = reinterpret_cast<const float4 *>(a.snh) + g0;
+    const float2 qx2 = make_float2(qx, qx), qy2 = make_float2(qy, qy), qz2 = make_float2(qz, qz);
+    const float2 thr = make_float2(k.thr, k.thr), hi2 = make_float2(k.hi, k.hi);
+    const float2 rel = make_float2(-(1.0f + kRelBand), -(1.0f + kRelBand)), band = make_float2(-k.kb, -k.kb);
+    unsigned bits = 0u;
+    const int turns = (m + 1) >> 1;
+#pragma unroll 1
+    for (int j = 0; j < turns; ++j) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const float4 x = __ldg(X + 2 * j + u), y = __ldg(Y + 2 * j + u), z = __ldg(Z + 2 * j + u);
+            float2 t0 = thr, t1 = thr;
+            if (!UNI) {
+                const float4 h = __ldg(H + 2 * j + u);
+                const float2 h0 = __fadd2_rn(hi2, make_float2(h.x, h.y)), h1 = __fadd2_rn(hi2, make_float2(h.z, h.w));
+                t0 = __ffma2_rn(__fmul2_rn(h0, rel), h0, band);
+                t1 = __ffma2_rn(__fmul2_rn(h1, rel), h1, band);
+            }
+            const float2 dx0 = __fadd2_rn(qx2, make_float2(x.x, x.y)), dx1 = __fadd2_rn(qx2, make_float2(x.z, x.w));
+            const float2 dy0 = __fadd2_rn(qy2, make_float2(y.x, y.y)), dy1 = __fadd2_rn(qy2, make_float2(y.z, y.w));
+            const float2 dz0 = __fadd2_rn(qz2, make_float2(z.x, z.y)), dz1 = __fadd2_rn(qz2, make_float2(z.z, z.w));
+            t0 = __ffma2_rn(dz0, dz0, t0);
+            t1 = __ffma2_rn(dz1, dz1, t1);
+            t0 = __ffma2_rn(dy0, dy0, t0);
+            t1 = __ffma2_rn(dy1, dy1, t1);
+            t0 = __ffma2_rn(dx0, dx0, t0);
+            t1 = __ffma2_rn(dx1, dx1, t1);
+            const int i0 = __float_as_int(t0.x), i1 = __float_as_int(t0.y);
+            const int i2 = __float_as_int(t1.x), i3 = __float_as_int(t1.y);
+            bits = __funnelshift_l((unsigned)i0, bits, 1);
+            bits = __funnelshift_l((unsigned)i1, bits, 1);
+            bits = __funnelshift_l((unsigned)i2, bits, 1);
+            bits = __funnelshift_l((unsigned)i3, bits, 1);
+            least = min(least, min(min(i0, i1), min(i2, i3)));
+        }
+    }
+    return bits << (32 - 8 * turns);
+}
+
+// The bits of the positions of [pb, pe) in the 32 from p0 = 4 g0 on, without t
+// itself; those in the decision band settled by the reference's FP64
+// expression, which also gives the minimum distance (of the own material's
+// particles with repulsive contact).
+template <int V>
+__device__ __forceinline__ unsigned accept_bits(const StepArgs &a, const Seeker &k, int t, int mati, int g0, int m,
+                                                int pb, int pe, float qy, float qz, double &mind) {
+    constexpr bool want_mind = (V & kSrchMind) != 0;
+    const int p0 = 4 * g0;
+    int least = 0x7fffffff;
+    unsigned bits = k.uni ? group_bits<true>(a, g0, m, k.qx, qy, qz, k, least)
+                          : group_bits<false>(a, g0, m, k.qx, qy, qz, k, least);
+    if (p0 < pb) bits &= 0xffffffffu >> (pb - p0);
+    if (pe - p0 < 32) bits &= ~(0xffffffffu >> (pe - p0));
+    if ((unsigned)(t - p0) < 32u) bits &= ~(0x80000000u >> (t - p0));
+    if (want_mind || least < k.tie_at) {
+        unsigned left = bits;
+        while (left) {
+            const int c = __clz(left);
+            left &= ~(0x80000000u >> c);
+            const double4 cd = a.cpos[p0 + c];
+            const double d2 = exact_d2(k.xi, cd);
+            const double hs = __dadd_rn(cd.w, k.xi.w);
+            if (!(d2 < __dmul_rn(hs, hs))) bits &= ~(0x80000000u >> c);
+            else if (want_mind && (!(V & kSrchContact) || a.cmat[p0 + c] == mati)) mind = fmin(mind, d2);
+        }
+    }
+    return bits;
+}
+
+// The set bits that belong to particles of other materials.
+__device__ __forceinline__ unsigned other_bits(const StepArgs &a, unsigned bits, int p0, int mati) {
+    unsigned oth = 0u, left = bits;
+    while (left) {
+        const int c = __clz(left);
+        left &= ~(0x80000000u >> c);
+        if (a.cmat[p0 + c] != mati) oth |= 0x80000000u >> c;
+    }
+    return oth;
+}
+
+// Ghost neighbours (and contacts) of t, found by the G lanes of grp together:
+// only neighbourhoods that reach a ghost layer have any; a cell's ghosts are
+// visited newest first (the reference's chain order).
+template <int V, int G>
+__device__ __forceinline__ void search_ghosts(const StepArgs &a, const Seeker &k, int t, int i,
+                                              int mati, int sub, unsigned grp, int &gn, int &gcn, double &mind) {
+    constexpr bool contact = (V & kSrchContact) != 0;
+    constexpr bool two_pass = (V & kSrchTwoPass) != 0;
+    const int lo0 = k.has_l ? k.bx - 1 : k.bx, hi0 = k.has_r ? k.bx + 1 : k.bx;
+    const DevPlanes &pl = a.prm.planes;
+    const bool near = (lo0 == 1 && pl.code[0][0]) || (hi0 == k.gl0 && pl.code[1][0]) ||
+                      (k.lo1 == 1 && pl.code[0][1]) || (k.hi1 == k.gl1 && pl.code[1][1]) ||
+                      (k.lo2 == 1 && pl.code[0][2]) || (k.hi2 == a.grid->gridlim[2] && pl.code[1][2]);
+    if (!near) return;
     const int np = a.npad;
-    const int cap = a.nstride;
-    const int key = a.ckey[t];
-    const int i = a.cell_list[t];
-    const bool with_self = (a.prm.disctype == 1);
-    const bool want_mind = (a.prm.tcrit_opt == 2 || a.prm.diag);
-    int nn = 0, gn = 0, nc = 0, gcn = 0;
-    double mind = 1.0e20;
-    const bool contact = a.prm.contact != 0;
-    if (key >= 0) {
-        const DevGrid g = *a.grid;
-        int bx, by, bz;
-        cell_coords(key, g.gridlim, bx, by, bz);
-        const int lo0 = bx > 1 ? bx - 1 : 1, hi0 = bx < g.gridlim[0] ? bx + 1 : g.gridlim[0];
-        const int lo1 = by > 1 ? by - 1 : 1, hi1 = by < g.gridlim[1] ? by + 1 : g.gridlim[1];
-        const int lo2 = bz > 1 ? bz - 1 : 1, hi2 = bz < g.gridlim[2] ? bz + 1 : g.gridlim[2];
-        const double4 xi = a.cpos[t];
-        const float4 ui = a.cposf[t];
-        const float cs[3] = {(float)(1.0 / g.gridsize[0]), (float)(1.0 / g.gridsize[1]), (float)(1.0 / g.gridsize[2])};
-        const float csm = fmaxf(cs[0], fmaxf(cs[1], cs[2]));
-        const float kb = 2.44140625e-4f * csm * csm;
-        const float khi = 1.0f + 2.44140625e-4f, klo = 1.0f - 2.44140625e-4f;
-        const float reach = ui.w + (float)g.hcut;
-        const float reach2 = reach * reach * 1.0009765625f + 9.765625e-4f * csm * csm;
-        const int mati = a.cmat[t];
-        unsigned *out = a.nidx + (size_t)t * cap;
-        // x extent of the rows: the own column always, a side column when its
-        // box can hold a neighbour (the test of k_search's cell loop)
-        const float gxl = ui.x, gxr = fmaxf(cs[0] - ui.x, 0.0f);
-        unsigned *cout = contact ? a.cidx + (size_t)t * a.cstride : nullptr;
-        const int passes = (a.nmat > 1 && a.prm.contacttype == 0) ? 2 : 1;
-        for (int pass = 0; pass < passes; ++pass) {
-            for (int nz = lo2; nz <= hi2; ++nz) {
-                const float qz = ui.z + (float)(bz - nz) * cs[2];
-                const float gz = fmaxf(nz < bz ? ui.z : (nz > bz ? cs[2] - ui.z : 0.0f), 0.0f);
-                for (int my = lo1; my <= hi1; ++my) {
-                    const float qy = ui.y + (float)(by - my) * cs[1];
-                    const float gy = fmaxf(my < by ? ui.y : (my > by ? cs[1] - ui.y : 0.0f), 0.0f);
-                    const float gyz = gy * gy + gz * gz;
-                    if (gyz > reach2) continue;
-                    const int lf = (lo0 < bx && !(gyz + fmaxf(gxl, 0.0f) * fmaxf(gxl, 0.0f) > reach2)) ? lo0 : bx;
-                    const int ll = (hi0 > bx && !(gyz + gxr * gxr > reach2)) ? hi0 : bx;
-                    const int kf = (int)cell_key(lf, my, nz, g.gridlim);
-                    const int cb = a.cell_start[kf];
-                    const int ce = a.cell_start[kf + (ll - lf) + 1];
-                    // first positions of the second and third cell of the range
-                    const int s1 = a.cell_start[kf + 1];
-                    const int s2 = (ll - lf >= 2) ? a.cell_start[kf + 2] : ce;
-                    const unsigned code_yz = (unsigned)(3 * (my - by + 1) + 9 * (nz - bz + 1));
-                    for (int base = cb; base < ce; base += 32) {
-                        const int p = base + lane;
-                        bool acc = false, accc = false;
-                        double d2 = 0.0;
-                        int lx = lf;
-                        if (p < ce) {
-                            lx = lf + (p >= s1 ? 1 : 0) + (p >= s2 ? 1 : 0);
-                            const float4 c = a.cposf[p];
-                            const float qx = ui.x + (float)(bx - lx) * cs[0];
-                            const float dx = qx - c.x, dy = qy - c.y, dz = qz - c.z;
-                            const float d2f = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                            const float hsf = ui.w + c.w;
-                            const float r2f = hsf * hsf;
-                            acc = (d2f < fmaf(r2f, khi, kb)) && (p != t);
-                            if (acc && (d2f > fmaf(r2f, klo, -kb) || want_mind)) {
-                                const double4 cd = a.cpos[p];
-                                d2 = exact_d2(xi, cd);
-                                const double hs = __dadd_rn(cd.w, xi.w);
-                                acc = d2 < __dmul_rn(hs, hs);
-                            }
-                            if (acc && contact) {
-                                accc = (a.cmat[p] != mati);
-                                acc = !accc;
-                            } else if (acc && a.nmat > 1) {
-                                acc = ((a.cmat[p] == mati) == (pass == 0));
-                            }
+    const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
+#pragma unroll 1
+    for (int pass = 0; pass < (two_pass ? 2 : 1); ++pass) {
+        for (int nz = k.lo2; nz <= k.hi2; ++nz)
+            for (int my = k.lo1; my <= k.hi1; ++my)
+                for (int lx = lo0; lx <= hi0; ++lx) {
+                    const int2 gc = a.gcell[k.row_key(my, nz) + lx - k.bx];
+                    for (int r0 = 0; r0 < gc.y; r0 += G) {
+                        const int r = r0 + sub;
+                        const int q = gc.x + gc.y - 1 - r;
+                        bool in = false, inc = false;
+                        if (r < gc.y) {
+                            const double4 c = make_double4(a.gx[q], a.gy[q], a.gz[q], a.gh[q]);
+                            const double d2 = exact_d2(k.xi, c);
+                            const double hs = __dadd_rn(c.w, k.xi.w);
+                            in = d2 < __dmul_rn(hs, hs);
+                            if (contact && in && a.gmat[q] != mati) { inc = true; in = false; }
+                            if (two_pass && in) in = (a.gmat[q] == mati) == (pass == 0);
+                            if (in) mind = fmin(mind, d2);
                         }
-                        const unsigned bal = __ballot_sync(0xffffffffu, acc);
-                        if (acc) {
-                            if (want_mind) mind = fmin(mind, d2);
-                            const int pos = nn + __popc(bal & below);
-                            if (pos < cap) out[pos] = (unsigned)p | ((code_yz + (unsigned)(lx - bx + 1)) << 26);
-                        }
-                        nn += __popc(bal);
-                        if (contact) {
-                            const unsigned cbal = __ballot_sync(0xffffffffu, accc);
-                            if (accc) {
-                                const int pos = nc + __popc(cbal & below);
-                                if (pos < a.cstride) cout[pos] = (unsigned)p | ((code_yz + (unsigned)(lx - bx + 1)) << 26);
+                        if (G == 1) {
+                            if (in) {
+                                if (gn < a.gstride) a.gnbr[(size_t)gn * np + t] = q;
+                                ++gn;
                             }
-                            nc += __popc(cbal);
+                            if (contact && inc) {
+                                if (gcn < a.gcstride) a.gcont[(size_t)gcn * np + t] = q;
+                                ++gcn;
+                            }
+                        } else {
+                            const unsigned bal = __ballot_sync(grp, in) & grp;
+                            const int at = gn + __popc(bal & below);
+                            if (in && at < a.gstride) a.gnbr[(size_t)at * np + t] = q;
+                            gn += __popc(bal);
+                            if (contact) {
+                                const unsigned cb = __ballot_sync(grp, inc) & grp;
+                                const int ac = gcn + __popc(cb & below);
+                                if (inc && ac < a.gcstride) a.gcont[(size_t)ac * np + t] = q;
+                                gcn += __popc(cb);
+                            }
                         }
                     }
                 }
-            }
-        }
-        // ghosts: only neighbourhoods that reach a ghost layer; a cell's ghosts
-        // are visited newest first (the chain order of the reference)
-        if (a.prm.boundary) {
-            const DevPlanes &pl = a.prm.planes;
-            const bool near = (lo0 == 1 && pl.code[0][0]) || (hi0 == g.gridlim[0] && pl.code[1][0]) ||
-                              (lo1 == 1 && pl.code[0][1]) || (hi1 == g.gridlim[1] && pl.code[1][1]) ||
-                              (lo2 == 1 && pl.code[0][2]) || (hi2 == g.gridlim[2] && pl.code[1][2]);
-            if (near) {
-                const int gpasses = (a.nmat > 1 && a.prm.contacttype == 0) ? 2 : 1;
-                for (int pass = 0; pass < gpasses; ++pass) {
-                    for (int nz = lo2; nz <= hi2; ++nz)
-                        for (int my = lo1; my <= hi1; ++my)
-                            for (int lx = lo0; lx <= hi0; ++lx) {
-                                const int2 gc = a.gcell[(int)cell_key(lx, my, nz, g.gridlim)];
-                                for (int base = 0; base < gc.y; base += 32) {
-                                    const int r = base + lane;
-                                    bool acc = false, accc = false;
-                                    double d2 = 0.0;
-                                    int q = 0;
-                                    if (r < gc.y) {
-                                        q = gc.x + gc.y - 1 - r;
-                                        const double4 c = make_double4(a.gx[q], a.gy[q], a.gz[q], a.gh[q]);
-                                        d2 = exact_d2(xi, c);
-                                        const double hs = __dadd_rn(c.w, xi.w);
-                                        acc = d2 < __dmul_rn(hs, hs);
-                                        if (acc && contact) {
-                                            accc = (a.gmat[q] != mati);
-                                            acc = !accc;
-                                        } else if (acc && a.nmat > 1) {
-                                            acc = ((a.gmat[q] == mati) == (pass == 0));
-                                        }
-                                    }
-                                    const unsigned bal = __ballot_sync(0xffffffffu, acc);
-                                    if (acc) {
-                                        mind = fmin(mind, d2);
-                                        const int pos = gn + __popc(bal & below);
-                                        if (pos < a.gstride) a.gnbr[(size_t)pos * np + t] = q;
-                                    }
-                                    gn += __popc(bal);
-                                    if (contact) {
-                                        const unsigned cbal = __ballot_sync(0xffffffffu, accc);
-                                        if (accc) {
-                                            const int pos = gcn + __popc(cbal & below);
-                                            if (pos < a.gcstride) a.gcont[(size_t)pos * np + t] = q;
-                                        }
-                                        gcn += __popc(cbal);
-                                    }
-                                }
-                            }
-                }
-            }
-        }
-        for (int o = 16; o > 0; o >>= 1) mind = fmin(mind, __shfl_xor_sync(0xffffffffu, mind, o));
-        mind = sqrt(mind);
     }
-    if (lane != 0) return;
-    if (nn > cap) {
-        atomicMax(&a.status->req_stride, nn);
+    if (sub == 0 && gn > a.gstride) {
+        atomicMax(&a.status->req_gstride, gn);
         raise_status(a.status, MCM_ENBR_OVERFLOW, i);
     }
-    if (gn > a.gstride) {
-        atomicMax(&a.status->req_gstride, gn);
+    if (contact && sub == 0 && gcn > a.gcstride) {
+        atomicMax(&a.status->req_gcstride, gcn);
+        raise_status(a.status, MCM_ENBR_OVERFLOW, i);
+    }
+}
+
+// Counts of t, and the largest of a warp's for the status.
+template <int V>
+__device__ __forceinline__ void search_counts(const StepArgs &a, int t, int i, int nn, int gn, int nc, int gcn, double mind) {
+    a.nnbr[t] = nn;
+    a.gnnbr[t] = gn;
+    if (V & kSrchContact) { a.ncont[t] = nc; a.gncont[t] = gcn; }
+    if (V & kSrchMind) a.F.f[FMINDIST][i] = mind;
+}
+__device__ __forceinline__ void search_max(const StepArgs &a, int nn, int gn) {
+    const int mn = __reduce_max_sync(0xffffffffu, nn), mg = __reduce_max_sync(0xffffffffu, gn);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&a.status->max_nbr, mn);
+        atomicMax(&a.status->max_gnbr, mg);
+    }
+}
+__device__ __forceinline__ void list_overflow(const StepArgs &a, int i, int nn, int nc, bool contact) {
+    if (nn > a.nstride) {
+        atomicMax(&a.status->req_stride, nn);
         raise_status(a.status, MCM_ENBR_OVERFLOW, i);
     }
     if (contact && nc > a.cstride) {
         atomicMax(&a.status->req_cstride, nc);
         raise_status(a.status, MCM_ENBR_OVERFLOW, i);
     }
-    if (contact && gcn > a.gcstride) {
-        atomicMax(&a.status->req_gcstride, gcn);
-        raise_status(a.status, MCM_ENBR_OVERFLOW, i);
+}
+
+// One thread per particle (bodies that fill the chip).  The lanes of a warp walk
+// the nine rows together (they lie in one or two cells, so their rows mostly
+// are the same ones), 32 candidates to a mask, and collect their entries in
+// shared memory, entry k of lane l at word 33 k + l.  When a lane has no room
+// for the next mask the whole warp moves the collected entries on, eight lanes
+// to a particle, each with one 16-byte store per four entries (rows start at
+// multiples of 4); up to three stay behind.
+constexpr int kSrchKeep = 36;   // entries a lane can hold
+template <int V>
+__global__ void __launch_bounds__(128, 8) k_search(StepArgs a) {
+    constexpr bool contact = (V & kSrchContact) != 0;   // contacttype > 0: other materials -> contact list
+    constexpr bool two_pass = (V & kSrchTwoPass) != 0;  // kernel contact between materials: own material first
+    constexpr unsigned kAll = 0xffffffffu;
+    extern __shared__ unsigned stage_all[];             // 33 kSrchKeep words per warp
+    if (a.status->code) return;
+    const int lane = threadIdx.x & 31;
+    unsigned *keep = stage_all + (threadIdx.x >> 5) * (33 * kSrchKeep) + lane;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int cap = a.nstride;
+    const int key = t < a.n ? a.ckey[t] : kNoCell;
+    const bool live = key >= 0;
+    Seeker k;
+    if (live) k = make_seeker(a, *a.grid, t, key);
+    const int mati = (live && (contact || two_pass)) ? a.cmat[t] : 0;
+    int nn = 0, held = 0;   // entries in the list (a multiple of 4) and in keep
+    int nc = 0, gn = 0, gcn = 0;
+    double mind = 1.0e20;
+    unsigned *row0 = a.nidx + (size_t)(t - lane) * cap;   // list of the warp's first particle
+    auto move_on = [&]() {
+        __syncwarp();
+        const int quads = held >> 2;
+#pragma unroll 1
+        for (int p0 = 0; p0 < 32; p0 += 4) {
+            const int p = p0 + (lane >> 3), q = lane & 7;
+            const int nq = __shfl_sync(kAll, quads, p), at = __shfl_sync(kAll, nn, p);
+            const unsigned *src = keep - lane + p;
+            unsigned *dst = row0 + (size_t)p * cap + at;
+            for (int i = q; i < nq; i += 8) {
+                const uint4 v = make_uint4(src[33 * (4 * i)], src[33 * (4 * i + 1)], src[33 * (4 * i + 2)], src[33 * (4 * i + 3)]);
+                if (at + 4 * i + 4 <= cap) *reinterpret_cast<uint4 *>(dst + 4 * i) = v;
+            }
+        }
+        __syncwarp();
+        const int left = held & 3;
+        for (int i = 0; i < left; ++i) keep[33 * i] = keep[33 * (4 * quads + i)];
+        nn += 4 * quads;
+        held = left;
+    };
+    const float gxl = fmaxf(k.ux, 0.0f), gxr = fmaxf(k.cs[0] - k.ux, 0.0f);
+    int others = 0;   // two_pass: neighbours of other materials, appended by a second walk
+#pragma unroll 1
+    for (int pass = 0; pass < (two_pass ? 2 : 1); ++pass) {
+        if (two_pass && pass == 1 && !__any_sync(kAll, others > 0)) break;
+#pragma unroll 1
+        for (int row = 0; row < 9; ++row) {
+            const int dy = row % 3 - 1, dz = row / 3 - 1;
+            int pb = 0, pe = 0, s1 = 0, s2 = 0;
+            float qy = 0.0f, qz = 0.0f;
+            if (live && !(two_pass && pass == 1 && others == 0)) {
+                const int my = k.by + dy, nz = k.bz + dz;
+                const float gyz = row_gap2(k, my, nz);
+                if (my >= k.lo1 && my <= k.hi1 && nz >= k.lo2 && nz <= k.hi2 && !(gyz > k.reach2)) {
+                    const int kc = k.row_key(my, nz);
+                    s1 = a.cell_start[kc];
+                    s2 = a.cell_start[kc + 1];
+                    pb = (k.has_l && !(gyz + gxl * gxl > k.reach2)) ? a.cell_start[kc - 1] : s1;
+                    pe = (k.has_r && !(gyz + gxr * gxr > k.reach2)) ? a.cell_start[kc + 2] : s2;
+                    qy = k.uy - (float)dy * k.cs[1];
+                    qz = k.uz - (float)dz * k.cs[2];
+                }
+            }
+            const unsigned code = (unsigned)(3 * row) << 26;
+            const int ge = pb < pe ? (pe + 3) >> 2 : 0;
+#pragma unroll 1
+            for (int g0 = pb >> 2; __any_sync(kAll, g0 < ge); g0 += 8) {
+                unsigned bits = 0u;
+                if (g0 < ge) bits = accept_bits<V>(a, k, t, mati, g0, min(8, ge - g0), pb, pe, qy, qz, mind);
+                if (contact || two_pass) {
+                    unsigned oth = other_bits(a, bits, 4 * g0, mati);
+                    bits &= ~oth;
+                    if (two_pass && pass == 0) others += __popc(oth);
+                    if (two_pass && pass == 1) bits = oth;
+                    if (contact) {
+                        while (oth) {
+                            const int b = __clz(oth);
+                            oth &= ~(0x80000000u >> b);
+                            const int p = 4 * g0 + b;
+                            unsigned e = (unsigned)p + code;
+                            if (p >= s1) e += 1u << 26;
+                            if (p >= s2) e += 1u << 26;
+                            if (nc < a.cstride) a.cidx[(size_t)t * a.cstride + nc] = e;
+                            ++nc;
+                        }
+                    }
+                }
+                if (__any_sync(kAll, held + __popc(bits) > kSrchKeep)) move_on();
+                unsigned *to = keep + 33 * held;
+                held += __popc(bits);
+                while (bits) {
+                    const int b = __clz(bits);
+                    bits ^= 0x80000000u >> b;
+                    const int p = 4 * g0 + b;
+                    unsigned e = (unsigned)p + code;
+                    if (p >= s1) e += 1u << 26;
+                    if (p >= s2) e += 1u << 26;
+                    *to = e;
+                    to += 33;
+                }
+            }
+        }
     }
-    if (with_self) nn += 1;   // MCM/mcm_ll_neighbours.f90:288-299 (for every particle)
-    a.nnbr[t] = nn;
-    a.gnnbr[t] = gn;
-    if (contact) { a.ncont[t] = nc; a.gncont[t] = gcn; }
-    if (want_mind) a.F.f[FMINDIST][i] = mind;
-    atomicMax(&a.status->max_nbr, nn);
-    atomicMax(&a.status->max_gnbr, gn);
+    move_on();
+    for (int i = 0; i < held; ++i)
+        if (nn + i < cap) a.nidx[(size_t)t * cap + nn + i] = keep[33 * i];
+    nn += held;
+    if (t < a.n) {
+        const int i = a.cell_list[t];
+        if (live) {
+            list_overflow(a, i, nn, nc, contact);
+            if (a.prm.boundary) search_ghosts<V, 1>(a, k, t, i, mati, 0, 0u, gn, gcn, mind);
+            mind = sqrt(mind);
+        }
+        if (a.prm.disctype == 1) nn += 1;   // MCM/mcm_ll_neighbours.f90:288-299 (for every particle)
+        search_counts<V>(a, t, i, nn, gn, nc, gcn, mind);
+    }
+    search_max(a, nn, gn);
+}
+
+// G lanes per particle (bodies too small to fill the chip with one thread per
+// particle).  A row's three cells are one contiguous range; each lane takes a
+// run of its groups, and the lanes' counts give each where its entries begin.
+// The three rows of a plane are decided before any is written, so that their
+// loads overlap.
+template <int V, int G>
+__global__ void __launch_bounds__(128, 6) k_search_lanes(StepArgs a) {
+    constexpr bool contact = (V & kSrchContact) != 0;
+    constexpr bool two_pass = (V & kSrchTwoPass) != 0;
+    constexpr bool want_mind = (V & kSrchMind) != 0;
+    if (a.status->code) return;
+    const int t = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) / G);
+    const int sub = threadIdx.x % G;
+    // the G lanes of a particle take every branch below together
+    const unsigned grp = ((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
+    const int cap = a.nstride;
+    int nn = 0, gn = 0;
+    if (t < a.n) {
+        const int key = a.ckey[t];
+        const int i = a.cell_list[t];
+        int nc = 0, gcn = 0;
+        double mind = 1.0e20;
+        if (key >= 0) {
+            const Seeker k = make_seeker(a, *a.grid, t, key);
+            const int mati = (contact || two_pass) ? a.cmat[t] : 0;
+            unsigned *out = a.nidx + (size_t)t * cap;
+            unsigned *cout = contact ? a.cidx + (size_t)t * a.cstride : nullptr;
+            const float gxl = fmaxf(k.ux, 0.0f), gxr = fmaxf(k.cs[0] - k.ux, 0.0f);
+            // exclusive sums over the lanes; total gets the sum
+            auto scan = [&](int v, int &total) {
+                int x = v;
+#pragma unroll
+                for (int o = 1; o < G; o <<= 1) {
+                    const int y = __shfl_up_sync(grp, x, o, G);
+                    if (sub >= o) x += y;
+                }
+                total = __shfl_sync(grp, x, G - 1, G);
+                return x - v;
+            };
+            auto write = [&](unsigned set, int at, unsigned *list, int room, int p0, int s1, int s2, unsigned code) {
+                while (set) {
+                    const int b = __clz(set);
+                    set &= ~(0x80000000u >> b);
+                    const int p = p0 + b;
+                    unsigned e = (unsigned)p + (code << 26);
+                    if (p >= s1) e += 1u << 26;
+                    if (p >= s2) e += 1u << 26;
+                    if (at < room) list[at] = e;
+                    ++at;
+                }
+            };
+            int others = 0;
+#pragma unroll 1
+            for (int pass = 0; pass < (two_pass ? 2 : 1); ++pass) {
+                if (two_pass && pass == 1 && others == 0) break;
+#pragma unroll 1
+                for (int nz = k.lo2; nz <= k.hi2; ++nz) {
+                    const float qz = k.uz + (float)(k.bz - nz) * k.cs[2];
+                    int rb[3], re[3], s1[3], s2[3], most = 0;
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) {
+                        const int my = k.by - 1 + r;
+                        rb[r] = re[r] = s1[r] = s2[r] = 0;
+                        const float gyz = row_gap2(k, my, nz);
+                        if (my < k.lo1 || my > k.hi1 || gyz > k.reach2) continue;
+                        const int kc = k.row_key(my, nz);
+                        s1[r] = a.cell_start[kc];
+                        s2[r] = a.cell_start[kc + 1];
+                        rb[r] = (k.has_l && !(gyz + gxl * gxl > k.reach2)) ? a.cell_start[kc - 1] : s1[r];
+                        re[r] = (k.has_r && !(gyz + gxr * gxr > k.reach2)) ? a.cell_start[kc + 2] : s2[r];
+                        if (rb[r] < re[r]) most = max(most, ((re[r] + 3) >> 2) - (rb[r] >> 2));
+                    }
+                    if (most == 0) continue;
+                    if (most <= 8 * G) {
+                        unsigned bits[3], oth[3];
+                        int p0[3];
+#pragma unroll
+                        for (int r = 0; r < 3; ++r) {
+                            const int gb = rb[r] >> 2, ge = (re[r] + 3) >> 2;
+                            const int per = (ge - gb + G - 1) / G;
+                            const int g0 = gb + sub * per, m = rb[r] < re[r] ? min(per, ge - g0) : 0;
+                            p0[r] = 4 * g0;
+                            bits[r] = oth[r] = 0u;
+                            if (m > 0)
+                                bits[r] = accept_bits<V>(a, k, t, mati, g0, m, rb[r], min(re[r], 4 * (g0 + m)),
+                                                         k.uy + (float)(1 - r) * k.cs[1], qz, mind);
+                        }
+                        if (contact || two_pass) {
+#pragma unroll
+                            for (int r = 0; r < 3; ++r) {
+                                oth[r] = other_bits(a, bits[r], p0[r], mati);
+                                bits[r] &= ~oth[r];
+                                if (two_pass && pass == 0) others += __popc(oth[r]);
+                                if (two_pass && pass == 1) bits[r] = oth[r];
+                            }
+                        }
+                        // three counts of at most 32 G <= 256 in one word
+                        int tot;
+                        const int ex = scan(__popc(bits[0]) | __popc(bits[1]) << 10 | __popc(bits[2]) << 20, tot);
+                        int at = nn;
+#pragma unroll
+                        for (int r = 0; r < 3; ++r) {
+                            write(bits[r], at + ((ex >> (10 * r)) & 1023), out, cap, p0[r], s1[r], s2[r],
+                                  (unsigned)(3 * r + 9 * (nz - k.bz + 1)));
+                            at += (tot >> (10 * r)) & 1023;
+                        }
+                        nn = at;
+                        if (contact) {
+                            const int cx = scan(__popc(oth[0]) | __popc(oth[1]) << 10 | __popc(oth[2]) << 20, tot);
+                            at = nc;
+#pragma unroll
+                            for (int r = 0; r < 3; ++r) {
+                                write(oth[r], at + ((cx >> (10 * r)) & 1023), cout, a.cstride, p0[r], s1[r], s2[r],
+                                      (unsigned)(3 * r + 9 * (nz - k.bz + 1)));
+                                at += (tot >> (10 * r)) & 1023;
+                            }
+                            nc = at;
+                        }
+                    } else {
+                        // rows of more than 32 G candidates: sub-runs of 8 groups per lane, row by row
+                        for (int r = 0; r < 3; ++r) {
+                            const unsigned code = (unsigned)(3 * r + 9 * (nz - k.bz + 1));
+                            const float qy = k.uy + (float)(1 - r) * k.cs[1];
+                            // (dynamic r: the row's values by selection)
+                            const int b = r == 0 ? rb[0] : (r == 1 ? rb[1] : rb[2]);
+                            const int e = r == 0 ? re[0] : (r == 1 ? re[1] : re[2]);
+                            const int f1 = r == 0 ? s1[0] : (r == 1 ? s1[1] : s1[2]);
+                            const int f2 = r == 0 ? s2[0] : (r == 1 ? s2[1] : s2[2]);
+                            const int ge = (e + 3) >> 2;
+                            if (b >= e) continue;
+                            for (int gw = b >> 2; gw < ge; gw += 8 * G) {
+                                const int g0 = gw + 8 * sub, m = min(8, ge - g0);
+                                unsigned bits = 0u, oth = 0u;
+                                if (m > 0) bits = accept_bits<V>(a, k, t, mati, g0, m, b, e, qy, qz, mind);
+                                if (contact || two_pass) {
+                                    oth = other_bits(a, bits, 4 * g0, mati);
+                                    bits &= ~oth;
+                                    if (two_pass && pass == 0) others += __popc(oth);
+                                    if (two_pass && pass == 1) bits = oth;
+                                }
+                                int tot;
+                                int ex = scan(__popc(bits), tot);
+                                write(bits, nn + ex, out, cap, 4 * g0, f1, f2, code);
+                                nn += tot;
+                                if (contact) {
+                                    ex = scan(__popc(oth), tot);
+                                    write(oth, nc + ex, cout, a.cstride, 4 * g0, f1, f2, code);
+                                    nc += tot;
+                                }
+                            }
+                        }
+                    }
+                }
+                if (two_pass) others = __reduce_add_sync(grp, others);
+            }
+            if (sub == 0) list_overflow(a, i, nn, nc, contact);
+            if (a.prm.boundary) search_ghosts<V, G>(a, k, t, i, mati, sub, grp, gn, gcn, mind);
+            if (want_mind)
+                for (int o = G / 2; o > 0; o >>= 1) mind = fmin(mind, __shfl_xor_sync(grp, mind, o, G));
+            mind = sqrt(mind);
+        }
+        if (a.prm.disctype == 1) nn += 1;   // MCM/mcm_ll_neighbours.f90:288-299 (for every particle)
+        if (sub == 0) search_counts<V>(a, t, i, nn, gn, nc, gcn, mind);
+    }
+    search_max(a, nn, gn);
 }
 
 // The same search with one warp per cell (search_kind 3): the lanes are the
@@ -1515,40 +1631,44 @@ void launch_skin_search(const StepArgs &a, cudaStream_t s) {
     k_skin_filter<<<nb, 256, 0, s>>>(a);
 }
 
+// Lanes per particle of the search: one thread per particle is the cheapest
+// walk where it fills the chip, but its chain of nine rows takes 65 us however
+// few particles there are.  Measured (us a search, 1 / 4 / 8 lanes, taylor
+// bars, mixed): 16 848 particles 62 / 48 / 34, 38 880: 70 / 53 / 55, 68 120:
+// 75 / 68 / 85, 131 544: 89 / 115 / 152, 685 824: 340 / 546 / 766.  Bodies of a
+// batch fill the chip together, so the particles of all that run at the same
+// time count.
+constexpr int kSearch8Below = 24000, kSearch4Below = 64000;
+template <int V, int G>
+static void launch_lanes(const StepArgs &a, int threads, cudaStream_t s) {
+    k_search_lanes<V, G><<<(unsigned)(((long long)a.n * G + threads - 1) / threads), threads, 0, s>>>(a);
+}
+template <int V>
+static void launch_search_v(const StepArgs &a, cudaStream_t s) {
+    const int threads = search_threads_of(a) < 128 ? search_threads_of(a) : 128;
+    const long long n = (long long)a.n * a.share;
+    if (a.search_kind == 2 || n < kSearch8Below) launch_lanes<V, 8>(a, threads, s);
+    else if (n < kSearch4Below) launch_lanes<V, 4>(a, threads, s);
+    else k_search<V><<<(a.n + threads - 1) / threads, threads, (threads / 32) * 33 * kSrchKeep * sizeof(unsigned), s>>>(a);
+}
+
 void launch_search(const StepArgs &a, cudaStream_t s) {
-    const int threads = search_threads_of(a);
     if (a.search_kind == 3) {
         // grid-stride over the cells (ncells is on the device): up to 16 blocks per SM
         long long b = (a.cell_cap + kCellWarps - 1) / kCellWarps;
         if (b > 148LL * 16) b = 148LL * 16;
         k_search_cell<<<(unsigned)(b < 1 ? 1 : b), kCellWarps * 32, 0, s>>>(a);
-    } else if (a.search_kind == 2) {
-        const long long lanes = 32LL * a.n;
-        k_search_warp<<<(unsigned)((lanes + threads - 1) / threads), threads, 0, s>>>(a);
-    } else {
-        const bool mind = a.prm.tcrit_opt == 2 || a.prm.diag;
-        const int v = (a.prm.contact ? kSrchContact : 0) | ((a.nmat > 1 && a.prm.contacttype == 0) ? kSrchTwoPass : 0) |
-                      (mind ? kSrchMind : 0);
-        const unsigned nb = (unsigned)((a.n + threads - 1) / threads);
-        if (a.prm.xsort) {
-            switch (v) {
-                case 0: k_search<kSrchXWin><<<nb, threads, 0, s>>>(a); break;
-                case kSrchContact: k_search<kSrchXWin | kSrchContact><<<nb, threads, 0, s>>>(a); break;
-                case kSrchTwoPass: k_search<kSrchXWin | kSrchTwoPass><<<nb, threads, 0, s>>>(a); break;
-                case kSrchMind: k_search<kSrchXWin | kSrchMind><<<nb, threads, 0, s>>>(a); break;
-                case kSrchContact | kSrchMind: k_search<kSrchXWin | kSrchContact | kSrchMind><<<nb, threads, 0, s>>>(a); break;
-                default: k_search<kSrchXWin | kSrchTwoPass | kSrchMind><<<nb, threads, 0, s>>>(a); break;
-            }
-        } else {
-            switch (v) {
-                case 0: k_search<0><<<nb, threads, 0, s>>>(a); break;
-                case kSrchContact: k_search<kSrchContact><<<nb, threads, 0, s>>>(a); break;
-                case kSrchTwoPass: k_search<kSrchTwoPass><<<nb, threads, 0, s>>>(a); break;
-                case kSrchMind: k_search<kSrchMind><<<nb, threads, 0, s>>>(a); break;
-                case kSrchContact | kSrchMind: k_search<kSrchContact | kSrchMind><<<nb, threads, 0, s>>>(a); break;
-                default: k_search<kSrchTwoPass | kSrchMind><<<nb, threads, 0, s>>>(a); break;
-            }
-        }
+        return;
+    }
+    const bool mind = a.prm.tcrit_opt == 2 || a.prm.diag;
+    switch ((a.prm.contact ? kSrchContact : 0) | ((a.nmat > 1 && a.prm.contacttype == 0) ? kSrchTwoPass : 0) |
+            (mind ? kSrchMind : 0)) {
+        case 0: launch_search_v<0>(a, s); break;
+        case kSrchContact: launch_search_v<kSrchContact>(a, s); break;
+        case kSrchTwoPass: launch_search_v<kSrchTwoPass>(a, s); break;
+        case kSrchMind: launch_search_v<kSrchMind>(a, s); break;
+        case kSrchContact | kSrchMind: launch_search_v<kSrchContact | kSrchMind>(a, s); break;
+        default: launch_search_v<kSrchTwoPass | kSrchMind>(a, s); break;
     }
 }
 

@@ -52,6 +52,8 @@ struct DevGrid {
     int pad;
     long long ncells;
     double hcut;      // largest h of the particles in cells (bounds the search reach)
+    double hmin;      // smallest h of the particles in cells
+    double cell[3];   // cell size 1 / gridsize
 };
 
 // Boundary planes (MCM/mcm_init_boundary.f90:28-116).
@@ -72,7 +74,6 @@ struct DevParams {
     int contacttype;  // 0: particles of other materials are neighbours (kernel contact); > 0: contacts
     int contact;      // contacttype > 0 with more than one material: contact lists and repulsion are built
     int kahan;        // mixed precision: pair sums compensated per lane (Kahan) before the lane combination
-    int xsort;        // each cell's particles in ascending x (FP64-fast, mixed); else descending reference index
     double drelax_scale, tssf, hmax;
     double skin;      // > 0: neighbour lists filtered from skin lists kept within h_i + h_j + skin * hmax
     double base_a[3];
@@ -112,7 +113,7 @@ __host__ __device__ inline long long cell_key(int bx, int by, int bz, const int 
 
 // Lower corner of cell b (1-based) along axis d of the grid.
 __host__ __device__ inline double cell_origin(const DevGrid &g, int d, int b) {
-    return g.gridmin[d] + (double)(b - 1) * (1.0 / g.gridsize[d]);
+    return g.gridmin[d] + (double)(b - 1) * g.cell[d];
 }
 
 __device__ __forceinline__ void raise_status(DevStatus *st, int code, int idx = -1) {

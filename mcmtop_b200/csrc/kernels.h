@@ -15,6 +15,7 @@ struct StepArgs {
     int ghost_cap;    // ghost storage
     long long cell_cap;   // cell-array storage
     int layer_cap;    // scratch for one boundary layer
+    int share;        // bodies of this one's size that run on the GPU at the same time (a batch's lanes)
     int split_mode;   // 1: step_a/b/c entry points (dt supplied by the host); 0: fused run
     DevParams prm;
     const DevMaterial *mats;
@@ -33,8 +34,8 @@ struct StepArgs {
     int *cell_list;   // npad: position -> state index
     int *n_inside;    // particles inside the grid (device counter)
     double4 *cpos;    // per position: x, y, z, h at neighbour time
-    float4 *cposf;    // per position: x, y, z relative to the cell origin (FP32), h
-    float4 *cposg;    // x-ordered steps, per position: x relative to the grid origin, y, z relative to the cell origin (FP32), h
+    float4 *cposf;    // per position: x, y, z relative to the cell origin (FP32), h (for search_kind 3 and the skin lists)
+    float *snx, *sny, *snz, *snh;   // per position, FP32: -(x relative to the grid origin), -(y), -(z) relative to the cell origin, h
     int *cmat;        // per position: material
     int *ckey;        // per position: cell key or -1
     int *scan_sums;   // block sums of the scan
@@ -83,7 +84,7 @@ struct StepArgs {
     int red_blocks;   // capacity of red in blocks (partial vectors)
     // launch shape, chosen by mcm_gpu_set_tuning or mcm_gpu_autotune (0: default)
     int search_threads;   // threads per block of the neighbour search
-    int search_kind;      // 0 or 1: one thread per particle (k_search); 2: one warp per particle (k_search_warp);
+    int search_kind;      // 0 or 1: lanes per particle by size (k_search, k_search_lanes); 2: eight lanes;
                           // 3: one warp per cell (k_search_cell)
     int pair_threads;     // threads per block of the cooperative strain and momentum gathers
     int pair_bps;         // blocks per SM the cooperative gathers' persistent grid is sized for (0: resident)
@@ -195,6 +196,6 @@ inline int pair_blocks_of(const StepArgs &a, int lanes, const void *kernel) {
     if (a.red_blocks > 0 && b > a.red_blocks) b = a.red_blocks;
     return b < 1 ? 1 : b;
 }
-inline int search_threads_of(const StepArgs &a) { return a.search_threads > 0 ? a.search_threads : 256; }
+inline int search_threads_of(const StepArgs &a) { return a.search_threads > 0 ? a.search_threads : 128; }
 
 }  // namespace mcm
