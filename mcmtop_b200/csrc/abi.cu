@@ -115,8 +115,9 @@ int alloc_particles(mcm_gpu_handle *h) {
     if ((st = dalloc(h, &h->A.key, np))) return st;
     if ((st = dalloc(h, &h->A.cell_list, np))) return st;
     if ((st = dalloc(h, &h->A.cpos, np))) return st;
-    if ((st = dalloc(h, &h->A.cposf, np))) return st;
-    if ((st = dalloc(h, &h->A.snx, 4 * (np + 32)))) return st;   // the search reads groups of four past the end
+    // the search's coordinates (it reads groups of four past the end), and cposf behind them
+    if ((st = dalloc(h, &h->A.snx, 4 * (np + 32) + 4 * np))) return st;
+    h->A.cposf = (float4 *)(h->A.snx + 4 * (np + 32));
     h->A.sny = h->A.snx + (np + 32);
     h->A.snz = h->A.sny + (np + 32);
     h->A.snh = h->A.snz + (np + 32);
@@ -761,7 +762,7 @@ int mcm_gpu_destroy(mcm_gpu_handle *h) {
     void *ptrs[] = {h->d_fields, h->d_stage, h->A.frec0, h->A.gfrec1, h->A.gfrec2,
                     h->d_ints, h->d_mats, h->d_scalars, h->d_nppermat,
                     h->A.key, h->A.cell_list, h->A.nnbr, h->A.gnnbr, h->A.rec0, h->A.rec1, h->A.rec2,
-                    h->A.cpos, h->A.cposf, h->A.snx, h->A.cmat, h->A.ckey, h->A.reorder_tmp, h->A.reorder_grp, h->A.nidx,
+                    h->A.cpos, h->A.snx, h->A.cmat, h->A.ckey, h->A.reorder_tmp, h->A.reorder_grp, h->A.nidx,
                     h->A.red, h->A.cell_count, h->A.cell_start, h->A.scan_sums, h->A.gcell,
                     h->A.layer_count, h->A.layer_off, h->A.gx, h->A.gy, h->A.gz, h->A.gvx, h->A.gvy,
                     h->A.gvz, h->A.gmass, h->A.gh, h->A.ghold, h->A.grho, h->A.gpar, h->A.gmat, h->A.gflip,

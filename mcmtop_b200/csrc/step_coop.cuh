@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepAr
             const Entry e = entry_at(a, t, k, nreal, self, spos);
             const double4 xj = e.kind ? a.grec0[e.idx] : a.rec0[e.idx];
             const double4 r2 = e.kind ? a.grec2[e.idx] : a.rec2[e.idx];
-            const double Volj = r2.z / r2.w;
+            const double Volj = r2.w;
             const double ih = inv_havg(xi.w, xj.w, ihi);
             const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
             double d[3];
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepAr
             const Entry e = entry_at(a, t, k, nreal, self, spos);
             const double4 xj = e.kind ? a.grec0[e.idx] : a.rec0[e.idx];
             const double4 r2 = e.kind ? a.grec2[e.idx] : a.rec2[e.idx];
-            const double Volj = r2.z / r2.w;
+            const double Volj = r2.w;
             const double ih = inv_havg(xi.w, xj.w, ihi);
             const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
             double d[3];

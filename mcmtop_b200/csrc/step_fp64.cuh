@@ -199,90 +199,6 @@ __global__ void k_strain_prep(StepArgs a) {
     }
 }
 
-template <int DISC>
-__device__ __forceinline__ void strain_gather(const StepArgs &a, const DevGrid &g, int t, const double4 xi,
-                                              const double4 vi, double gv[3][3]) {
-    if (DISC == 0) {
-        // MCM/mcm_oldstrain.f90:34-54
-        auto body = [&](const double4 xj, const double4 vj) {
-            double Volj = vj.w;
-            double havg = 0.5 * (xi.w + xj.w);
-            double d[3];
-            gradw(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z, havg, d[0], d[1], d[2]);
-            const double dv[3] = {vj.x - vi.x, vj.y - vi.y, vj.z - vi.z};
-#pragma unroll
-            for (int n = 0; n < 3; ++n) {
-                double tt = Volj * dv[n];
-#pragma unroll
-                for (int m = 0; m < 3; ++m) gv[n][m] = gv[n][m] + tt * d[m];
-            }
-        };
-        for_each_neighbour(
-            a, g, t, [&](int p, bool) { body(a.rec0[p], a.rec1[p]); }, [&](int q) { body(a.grec0[q], a.grec1[q]); });
-    } else {
-        // MCM/mcm_corr_strain.f90:51-134 (three passes, kernel centred at i)
-        double sum_w = 0.0, sg[3] = {0.0, 0.0, 0.0};
-        auto pass1 = [&](const double4 xj, const double4 vj) {
-            double Volj = vj.w;
-            double havg = 0.5 * (xi.w + xj.w);
-            double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-            double w = kernelw(dx, dy, dz, havg);
-            double d[3];
-            gradw(dx, dy, dz, havg, d[0], d[1], d[2]);
-            sum_w = sum_w + Volj * w;
-#pragma unroll
-            for (int l = 0; l < 3; ++l) sg[l] = sg[l] + Volj * d[l];
-        };
-        for_each_neighbour(
-            a, g, t, [&](int p, bool) { pass1(a.rec0[p], a.rec1[p]); }, [&](int q) { pass1(a.grec0[q], a.grec1[q]); });
-        double B[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        const double sw2 = sum_w * sum_w;
-        auto pass2 = [&](const double4 xj, const double4 vj) {
-            double Volj = vj.w;
-            double havg = 0.5 * (xi.w + xj.w);
-            double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-            double w = kernelw(dx, dy, dz, havg);
-            double d[3];
-            gradw(dx, dy, dz, havg, d[0], d[1], d[2]);
-            double cg[3];
-#pragma unroll
-            for (int m = 0; m < 3; ++m) cg[m] = (d[m] * sum_w - w * sg[m]) / sw2;
-            const double xr[3] = {xj.x - xi.x, xj.y - xi.y, xj.z - xi.z};
-#pragma unroll
-            for (int m = 0; m < 3; ++m)
-#pragma unroll
-                for (int n = 0; n < 3; ++n) B[n][m] = B[n][m] + Volj * xr[n] * cg[m];
-        };
-        for_each_neighbour(
-            a, g, t, [&](int p, bool) { pass2(a.rec0[p], a.rec1[p]); }, [&](int q) { pass2(a.grec0[q], a.grec1[q]); });
-        double invB[3][3];
-        inverse3(B, invB);
-        auto pass3 = [&](const double4 xj, const double4 vj) {
-            double Volj = vj.w;
-            double havg = 0.5 * (xi.w + xj.w);
-            double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-            double w = kernelw(dx, dy, dz, havg);
-            double d[3];
-            gradw(dx, dy, dz, havg, d[0], d[1], d[2]);
-            double cg[3];
-#pragma unroll
-            for (int m = 0; m < 3; ++m) cg[m] = (d[m] * sum_w - w * sg[m]) / sw2;
-            double c2[3];
-#pragma unroll
-            for (int n = 0; n < 3; ++n) c2[n] = invB[n][0] * cg[0] + invB[n][1] * cg[1] + invB[n][2] * cg[2];
-            const double vv[3] = {vj.x, vj.y, vj.z};
-#pragma unroll
-            for (int n = 0; n < 3; ++n) {
-                double tt = Volj * vv[n];
-#pragma unroll
-                for (int m = 0; m < 3; ++m) gv[n][m] = gv[n][m] + tt * c2[m];
-            }
-        };
-        for_each_neighbour(
-            a, g, t, [&](int p, bool) { pass3(a.rec0[p], a.rec1[p]); }, [&](int q) { pass3(a.grec0[q], a.grec1[q]); });
-    }
-}
-
 __device__ __forceinline__ double block_min(double v, double *sm) {
     for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -293,37 +209,6 @@ __device__ __forceinline__ double block_min(double v, double *sm) {
         for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
     }
     return v;
-}
-
-// ------------------------------------------------------------ strain rate
-// MCM/mcm_oldstrain.f90 / mcm_corr_strain.f90 for the particle at position t:
-// rod, spin and trace go to the state's diagnostic arrays, which the
-// constitutive kernel reads (this keeps the gather kernel small enough to
-// keep many warps resident).
-template <int DISC>
-__global__ void __launch_bounds__(kRedThreads) k_strain(StepArgs a) {
-    if (skip_step(a)) return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= a.n) return;
-    const int i = a.cell_list[t];
-    const DevGrid g = *a.grid;
-    const double4 xi = a.rec0[t], vi = a.rec1[t];
-    double gv[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    strain_gather<DISC>(a, g, t, xi, vi, gv);
-    double *const *f = a.F.f;
-    const double r11 = 0.5 * (gv[0][0] + gv[0][0]);
-    const double r22 = 0.5 * (gv[1][1] + gv[1][1]);
-    const double r33 = 0.5 * (gv[2][2] + gv[2][2]);
-    f[FR11][i] = r11;
-    f[FR22][i] = r22;
-    f[FR33][i] = r33;
-    f[FR12][i] = 0.5 * (gv[0][1] + gv[1][0]);
-    f[FR13][i] = 0.5 * (gv[0][2] + gv[2][0]);
-    f[FR23][i] = 0.5 * (gv[1][2] + gv[2][1]);
-    f[FW12][i] = 0.5 * (gv[0][1] - gv[1][0]);
-    f[FW13][i] = 0.5 * (gv[0][2] - gv[2][0]);
-    f[FW23][i] = 0.5 * (gv[1][2] - gv[2][1]);
-    f[FTR][i] = r11 + r22 + r33;
 }
 
 // ------------------------------------------------- variable smoothing length
@@ -457,7 +342,7 @@ __global__ void k_rep_cont(StepArgs a) {
 
 // --------------------------------------------------------- momentum prep
 // Gather records: x, h; (sigma - q)/rho^2 (MCM/mcm_oldacceleration.f90:79-80);
-// mass.  Ghost stresses follow MCM/mcm_update_ghost_stress.f90:28-41 (all
+// mass and V = m/rho (the corrected sums').  Ghost stresses follow MCM/mcm_update_ghost_stress.f90:28-41 (all
 // off-diagonals negated) with the ghost's own density from its creation.
 __global__ void k_mom_prep(StepArgs a) {
     if (skip_step(a)) return;
@@ -470,7 +355,7 @@ __global__ void k_mom_prep(StepArgs a) {
         a.rec0[p] = make_double4(f[FX][i], f[FY][i], f[FZ][i], f[FH][i]);
         a.rec1[p] = make_double4((f[FS11][i] - q) / r2, (f[FS22][i] - q) / r2, (f[FS33][i] - q) / r2,
                                  (f[FS12][i] - 0.0) / r2);
-        a.rec2[p] = make_double4((f[FS13][i] - 0.0) / r2, (f[FS23][i] - 0.0) / r2, f[FMASS][i], rho);
+        a.rec2[p] = make_double4((f[FS13][i] - 0.0) / r2, (f[FS23][i] - 0.0) / r2, f[FMASS][i], f[FMASS][i] / rho);
         if (a.prm.asym)
             a.rec3[p] = make_double4((f[FL21][i] - 0.0) / r2, (f[FL31][i] - 0.0) / r2, (f[FL32][i] - 0.0) / r2, 0.0);
     }
@@ -484,134 +369,12 @@ __global__ void k_mom_prep(StepArgs a) {
             a.grec0[g] = make_double4(a.gx[g], a.gy[g], a.gz[g], a.gh[g]);
             a.grec1[g] = make_double4((f[FS11][j] - q) / r2, (f[FS22][j] - q) / r2, (f[FS33][j] - q) / r2,
                                       ((-f[FS12][j]) - (-0.0)) / r2);
-            a.grec2[g] = make_double4(((-f[FS13][j]) - (-0.0)) / r2, ((-f[FS23][j]) - (-0.0)) / r2, a.gmass[g], rho);
+            a.grec2[g] = make_double4(((-f[FS13][j]) - (-0.0)) / r2, ((-f[FS23][j]) - (-0.0)) / r2, a.gmass[g],
+                                      a.gmass[g] / rho);
             if (a.prm.asym)
                 a.grec3[g] = make_double4(((-f[FL21][j]) - (-0.0)) / r2, ((-f[FL31][j]) - (-0.0)) / r2,
                                           ((-f[FL32][j]) - (-0.0)) / r2, 0.0);
         }
-    }
-}
-
-__device__ __forceinline__ void sym_from_rec(const double4 &r1, const double4 &r2, double A[3][3]) {
-    A[0][0] = r1.x; A[1][1] = r1.y; A[2][2] = r1.z;
-    A[0][1] = A[1][0] = r1.w;
-    A[0][2] = A[2][0] = r2.x;
-    A[1][2] = A[2][1] = r2.y;
-}
-
-// The lower triangle from the asymmetric record (cap model, prm.asym).
-__device__ __forceinline__ void lower_from_rec(const double4 &r3, double A[3][3]) {
-    A[1][0] = r3.x;
-    A[2][0] = r3.y;
-    A[2][1] = r3.z;
-}
-
-template <int DISC>
-__device__ __forceinline__ void momentum_gather(const StepArgs &a, const DevGrid &g, int t, double acc[3]) {
-    const double4 xi = a.rec0[t];
-    double Ai[3][3];
-    sym_from_rec(a.rec1[t], a.rec2[t], Ai);
-    const bool asym = a.prm.asym != 0;
-    if (asym) lower_from_rec(a.rec3[t], Ai);
-    if (DISC == 0) {
-        // MCM/mcm_oldacceleration.f90:66-89; sigma(m,n) is read as stored,
-        // both triangles (they differ for the cap model)
-        auto body = [&](const double4 xj, const double4 r1, const double4 r2, const double4 *r3) {
-            double havg = 0.5 * (xi.w + xj.w);
-            double d[3];
-            gradw(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z, havg, d[0], d[1], d[2]);
-            double Aj[3][3];
-            sym_from_rec(r1, r2, Aj);
-            if (r3) lower_from_rec(*r3, Aj);
-            const double massj = r2.z;
-#pragma unroll
-            for (int n = 0; n < 3; ++n) {
-                double ds = 0.0;
-#pragma unroll
-                for (int m = 0; m < 3; ++m) ds = ds + (Aj[m][n] + Ai[m][n]) * d[m];
-                acc[n] = acc[n] + massj * ds;
-            }
-        };
-        for_each_neighbour(
-            a, g, t, [&](int p, bool) { body(a.rec0[p], a.rec1[p], a.rec2[p], asym ? &a.rec3[p] : nullptr); },
-            [&](int q) { body(a.grec0[q], a.grec1[q], a.grec2[q], asym ? &a.grec3[q] : nullptr); });
-    } else {
-        // MCM/mcm_corr_acceleration.f90:63-161 (kernel centred at j; the self
-        // slot k = nnbr is zeroed; the final sum uses the last neighbour's mass)
-        double sum_w = 0.0, sg[3] = {0.0, 0.0, 0.0};
-        double massj = 0.0;
-        auto pass1 = [&](const double4 xj, const double4 r2) {
-            massj = r2.z;
-            double Volj = massj / r2.w;
-            double havg = 0.5 * (xi.w + xj.w);
-            double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-            double w = kernelw(dx, dy, dz, havg);
-            double d[3];
-            gradw(dx, dy, dz, havg, d[0], d[1], d[2]);
-            sum_w = sum_w + Volj * w;
-#pragma unroll
-            for (int l = 0; l < 3; ++l) sg[l] = sg[l] + Volj * d[l];
-        };
-        for_each_neighbour(
-            a, g, t, [&](int p, bool) { pass1(a.rec0[p], a.rec2[p]); }, [&](int q) { pass1(a.grec0[q], a.grec2[q]); });
-        double B[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        const double sw2 = sum_w * sum_w;
-        auto pass2 = [&](const double4 xj, const double4 r2) {
-            massj = r2.z;
-            double Volj = massj / r2.w;
-            double havg = 0.5 * (xi.w + xj.w);
-            double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-            double w = kernelw(dx, dy, dz, havg);
-            double d[3];
-            gradw(dx, dy, dz, havg, d[0], d[1], d[2]);
-            double cg[3];
-#pragma unroll
-            for (int m = 0; m < 3; ++m) cg[m] = (d[m] * sum_w - w * sg[m]) / sw2;
-            const double xr[3] = {dx, dy, dz};
-#pragma unroll
-            for (int m = 0; m < 3; ++m)
-#pragma unroll
-                for (int n = 0; n < 3; ++n) B[n][m] = B[n][m] + Volj * xr[n] * cg[m];
-        };
-        for_each_neighbour(
-            a, g, t, [&](int p, bool) { pass2(a.rec0[p], a.rec2[p]); }, [&](int q) { pass2(a.grec0[q], a.grec2[q]); });
-        double invB[3][3];
-        inverse3(B, invB);
-        // deltasig(m,n,l) is symmetric in (m,n): keep 6 x 3 accumulators
-        double ds[6][3];
-#pragma unroll
-        for (int u = 0; u < 6; ++u) ds[u][0] = ds[u][1] = ds[u][2] = 0.0;
-        auto pass3 = [&](const double4 xj, const double4 r1, const double4 r2, bool self_slot) {
-            massj = r2.z;
-            double havg = 0.5 * (xi.w + xj.w);
-            double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-            double w = kernelw(dx, dy, dz, havg);
-            double d[3];
-            gradw(dx, dy, dz, havg, d[0], d[1], d[2]);
-            double cg[3];
-#pragma unroll
-            for (int m = 0; m < 3; ++m) cg[m] = (d[m] * sum_w - w * sg[m]) / sw2;
-            double Aj[3][3];
-            sym_from_rec(r1, r2, Aj);
-#pragma unroll
-            for (int u = 0; u < 6; ++u) {
-                const int m = (u < 3) ? u : (u == 5 ? 1 : 0);
-                const int n = (u < 3) ? u : (u == 3 ? 1 : 2);
-                double dsig = Aj[m][n] + Ai[m][n];
-                if (self_slot) dsig = 0.0;
-#pragma unroll
-                for (int l = 0; l < 3; ++l) ds[u][l] = ds[u][l] + dsig * cg[l];
-            }
-        };
-        for_each_neighbour(
-            a, g, t, [&](int p, bool self) { pass3(a.rec0[p], a.rec1[p], a.rec2[p], self); },
-            [&](int q) { pass3(a.grec0[q], a.grec1[q], a.grec2[q], false); });
-#pragma unroll
-        for (int n = 0; n < 3; ++n)
-#pragma unroll
-            for (int m = 0; m < 3; ++m)
-#pragma unroll
-                for (int l = 0; l < 3; ++l) acc[n] = acc[n] + massj * ds[sym_index(n, m)][l] * invB[l][m];
     }
 }
 
@@ -678,84 +441,6 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &a, int i, con
     f[FVX][i] = v[0]; f[FVY][i] = v[1]; f[FVZ][i] = v[2];
     f[FVABS][i] = vabs;
     f[FX][i] = xo[0]; f[FY][i] = xo[1]; f[FZ][i] = xo[2];
-}
-
-// ----------------------------------------------- momentum + integration
-// Writes a (split path), adds base accelerations and displacement BCs
-// (MCM/mcm_boundcond.f90:23-62), block partial energy sums
-// (MCM/mcm_calctotale.f90:33-51) and, when integrate is set and the run has
-// not terminated, the velocity and position update with block bbox partials.
-template <int DISC>
-__global__ void __launch_bounds__(kRedThreads) k_momentum(StepArgs a, int integrate) {
-    __shared__ double sm[32];
-    if (skip_step(a)) return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nm = a.nmat;
-    double acc[3] = {0.0, 0.0, 0.0};
-    int mati = 0;
-    double ke = 0.0, ie = 0.0, mo[3] = {0.0, 0.0, 0.0};
-    double x[3] = {1.0e20, 1.0e20, 1.0e20};
-    double xmax[3] = {-1.0e20, -1.0e20, -1.0e20};
-    const bool do_int = integrate && !a.time->ended;
-    if (t < a.n) {
-        const int i = a.cell_list[t];
-        double *const *f = a.F.f;
-        const DevGrid g = *a.grid;
-        // MCM/mcm_oldacceleration.f90:49-51, mcm_corr_acceleration.f90:45-49
-        if (a.prm.contact)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) acc[j] = acc[j] + f[FRPX + j][i];
-        momentum_gather<DISC>(a, g, t, acc);
-        if (a.prm.baseaccel)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) acc[j] = acc[j] + a.prm.base_a[j];
-        switch (a.F.dispbc[i]) {
-            case 1: acc[0] = 0.0; break;
-            case 2: acc[1] = 0.0; break;
-            case 3: acc[2] = 0.0; break;
-            case 4: acc[0] = 0.0; acc[1] = 0.0; break;
-            case 5: acc[1] = 0.0; acc[2] = 0.0; break;
-            case 6: acc[0] = 0.0; acc[2] = 0.0; break;
-            case 7: acc[0] = 0.0; acc[1] = 0.0; acc[2] = 0.0; break;
-            default: break;
-        }
-        if (a.split_mode || a.prm.diag || a.prm.veloc_opt) { f[FAX][i] = acc[0]; f[FAY][i] = acc[1]; f[FAZ][i] = acc[2]; }
-        mati = a.F.mat[i];
-        const double mass = f[FMASS][i], vabs = f[FVABS][i];
-        ke = 0.5 * mass * (vabs * vabs);
-        mo[0] = mass * fabs(f[FVX][i]);
-        mo[1] = mass * fabs(f[FVY][i]);
-        mo[2] = mass * fabs(f[FVZ][i]);
-        ie = f[FE][i];
-        if (do_int) {
-            double xn[3];
-            integrate_particle(a, i, acc, a.time->dt, a.time->dtold, xn);
-            x[0] = xn[0]; x[1] = xn[1]; x[2] = xn[2];
-            xmax[0] = xn[0]; xmax[1] = xn[1]; xmax[2] = xn[2];
-        }
-    }
-    // per-block partials: [5*nmat energies][6 bbox]
-    const int stride = 5 * nm + 6;
-    double *out = a.red + (size_t)blockIdx.x * stride;
-    for (int m = 1; m <= nm; ++m) {
-        bool mine = (mati == m);
-        double v0 = block_sum(mine ? ke : 0.0, sm);
-        double v1 = block_sum(mine ? ie : 0.0, sm);
-        double v2 = block_sum(mine ? mo[0] : 0.0, sm);
-        double v3 = block_sum(mine ? mo[1] : 0.0, sm);
-        double v4 = block_sum(mine ? mo[2] : 0.0, sm);
-        if (threadIdx.x == 0) {
-            out[5 * (m - 1) + 0] = v0; out[5 * (m - 1) + 1] = v1;
-            out[5 * (m - 1) + 2] = v2; out[5 * (m - 1) + 3] = v3; out[5 * (m - 1) + 4] = v4;
-        }
-    }
-    if (do_int) {
-        for (int d = 0; d < 3; ++d) {
-            double lo = block_minmax(x[d], sm, false);
-            double hi = block_minmax(xmax[d], sm, true);
-            if (threadIdx.x == 0) { out[5 * nm + d] = lo; out[5 * nm + 3 + d] = hi; }
-        }
-    }
 }
 
 // Split path: velocity and position update after the host's output phase.
@@ -1005,7 +690,9 @@ __global__ void __launch_bounds__(kRedThreads) k_init_critts(StepArgs a) {
 }  // namespace MCM_FLAVOUR_NS
 }  // namespace mcm
 
-#if !MCM_EXACT
+#if MCM_EXACT
+#include "step_exact.cuh"
+#else
 #include "step_coop.cuh"
 #endif
 
@@ -1020,15 +707,23 @@ static inline int nblk(int n, int t) { return (n + t - 1) / t; }
 constexpr int kCoopLanes = 4;
 static inline int gs_blocks(int n) { int b = nblk(n, 256); return b > 148 * 16 ? 148 * 16 : (b < 1 ? 1 : b); }
 
+#if MCM_EXACT
+// Lanes per particle of the in-order sums; the particles of all the bodies
+// that run at the same time fill the chip.
+static int seq_lanes(const StepArgs &a) { return (long long)a.n * a.share < kSeqLanesBelow ? 8 : 1; }
+#endif
+
 void launch_strain_prep(const StepArgs &a, cudaStream_t s) {
     k_strain_prep<<<gs_blocks(a.n > a.ghost_cap ? a.n : a.ghost_cap), 256, 0, s>>>(a);
 }
 
 void launch_strain(const StepArgs &a, cudaStream_t s) {
 #if MCM_EXACT
-    int blocks = nblk(a.n, kRedThreads);
-    if (a.prm.disctype == 0) k_strain<0><<<blocks, kRedThreads, 0, s>>>(a);
-    else k_strain<1><<<blocks, kRedThreads, 0, s>>>(a);
+    const int lanes = seq_lanes(a);
+    void (*kern)(StepArgs) = a.prm.disctype == 0 ? (lanes == 1 ? k_strain_seq<0, 1> : k_strain_seq<0, 8>)
+                                                 : (lanes == 1 ? k_strain_seq<1, 1> : k_strain_seq<1, 8>);
+    const int threads = seq_threads(lanes);
+    kern<<<nblk(a.n, threads / lanes), threads, 0, s>>>(a);
 #else
     constexpr int L = kCoopLanes;
     void (*kern)(StepArgs) = a.prm.disctype == 0 ? k_strain_coop<L, 0> : k_strain_coop<L, 1>;
@@ -1050,9 +745,16 @@ void launch_rep_cont(const StepArgs &a, cudaStream_t s) { k_rep_cont<<<gs_blocks
 
 int launch_momentum(const StepArgs &a, cudaStream_t s, int integrate) {
 #if MCM_EXACT
-    int blocks = nblk(a.n, kRedThreads);
-    if (a.prm.disctype == 0) k_momentum<0><<<blocks, kRedThreads, 0, s>>>(a, integrate);
-    else k_momentum<1><<<blocks, kRedThreads, 0, s>>>(a, integrate);
+    const int lanes = seq_lanes(a);
+    void (*kern)(StepArgs, int) =
+        a.prm.disctype != 0 ? (lanes == 1 ? k_momentum_seq<1, false, 1> : k_momentum_seq<1, false, 8>)
+        : a.prm.asym        ? (lanes == 1 ? k_momentum_seq<0, true, 1> : k_momentum_seq<0, true, 8>)
+                            : (lanes == 1 ? k_momentum_seq<0, false, 1> : k_momentum_seq<0, false, 8>);
+    const int threads = seq_threads(lanes);
+    int blocks = nblk(a.n, threads / lanes);
+    const int wave = 148 * resident_per_sm((const void *)kern, threads);
+    if (blocks > wave) blocks = wave;
+    kern<<<blocks, threads, 0, s>>>(a, integrate);
     return blocks;
 #else
     constexpr int L = kCoopLanes;
