@@ -20,6 +20,14 @@ __device__ __forceinline__ void cell_coords(int key, const int *gl, int &bx, int
 
 constexpr unsigned kPosMask = 0x3ffffffu;   // position bits of a neighbour entry
 
+// A 32-byte record in one load: two 16-byte loads of records 32 bytes apart
+// would each use half of every sector they touch.
+__device__ __forceinline__ double4 ld4(const double4 *p) {
+    double4 r;
+    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    return r;
+}
+
 // Real neighbours stored for position t (the self entry of disctype 1 is not stored).
 __device__ __forceinline__ int stored_neighbours(const StepArgs &a, int t) {
     return a.nnbr[t] - (a.prm.disctype == 1 ? 1 : 0);

@@ -82,8 +82,8 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_strain_coop(StepArgs
     if (live) {
         nreal = stored_neighbours(a, t);
         gn = a.gnnbr[t];
-        xi = a.rec0[t];
-        vi = a.rec1[t];
+        xi = ld4(a.rec0 + t);
+        vi = ld4(a.rec1 + t);
     }
     const unsigned *spos = a.nidx + (size_t)t * a.nstride;
     const int self = (a.prm.disctype == 1) ? 1 : 0;
@@ -93,10 +93,7 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_strain_coop(StepArgs
 #pragma unroll
     for (int u = 0; u < 9; ++u) gv[u] = 0.0;
     if (DISC == 0) {
-        for (int k = lane; k < total; k += L) {
-            const Entry e = entry_at(a, t, k, nreal, self, spos);
-            const double4 xj = e.kind ? a.grec0[e.idx] : a.rec0[e.idx];
-            const double4 vj = e.kind ? a.grec1[e.idx] : a.rec1[e.idx];
+        auto add = [&](const double4 &xj, const double4 &vj) {
             double d[3];
             gradw_ih(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z, inv_havg(xi.w, xj.w, ihi), d[0], d[1], d[2]);
             const double dv[3] = {vj.w * (vj.x - vi.x), vj.w * (vj.y - vi.y), vj.w * (vj.z - vi.z)};
@@ -104,14 +101,23 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_strain_coop(StepArgs
             for (int n = 0; n < 3; ++n)
 #pragma unroll
                 for (int m = 0; m < 3; ++m) gv[3 * n + m] = fma(dv[n], d[m], gv[3 * n + m]);
+        };
+        int k = lane;
+        for (; k < nreal; k += L) {
+            const int p = (int)(spos[k] & kPosMask);
+            add(ld4(a.rec0 + p), ld4(a.rec1 + p));
+        }
+        for (; k < total; k += L) {
+            const int q = a.gnbr[(size_t)(k - nreal) * a.npad + t];
+            add(ld4(a.grec0 + q), ld4(a.grec1 + q));
         }
     } else {
         // MCM/mcm_corr_strain.f90:51-134
         double sw = 0.0, sg0 = 0.0, sg1 = 0.0, sg2 = 0.0;
         for (int k = lane; k < total; k += L) {
             const Entry e = entry_at(a, t, k, nreal, self, spos);
-            const double4 xj = e.kind ? a.grec0[e.idx] : a.rec0[e.idx];
-            const double Volj = e.kind ? a.grec1[e.idx].w : a.rec1[e.idx].w;
+            const double4 xj = ld4((e.kind ? a.grec0 : a.rec0) + e.idx);
+            const double Volj = ld4((e.kind ? a.grec1 : a.rec1) + e.idx).w;
             const double ih = inv_havg(xi.w, xj.w, ihi);
             const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
             double d[3];
@@ -126,8 +132,8 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_strain_coop(StepArgs
         for (int u = 0; u < 9; ++u) B[u] = 0.0;
         for (int k = lane; k < total; k += L) {
             const Entry e = entry_at(a, t, k, nreal, self, spos);
-            const double4 xj = e.kind ? a.grec0[e.idx] : a.rec0[e.idx];
-            const double Volj = e.kind ? a.grec1[e.idx].w : a.rec1[e.idx].w;
+            const double4 xj = ld4((e.kind ? a.grec0 : a.rec0) + e.idx);
+            const double Volj = ld4((e.kind ? a.grec1 : a.rec1) + e.idx).w;
             const double ih = inv_havg(xi.w, xj.w, ihi);
             const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
             double d[3];
@@ -147,8 +153,8 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_strain_coop(StepArgs
         inverse3(Bm, invB);
         for (int k = lane; k < total; k += L) {
             const Entry e = entry_at(a, t, k, nreal, self, spos);
-            const double4 xj = e.kind ? a.grec0[e.idx] : a.rec0[e.idx];
-            const double4 vj = e.kind ? a.grec1[e.idx] : a.rec1[e.idx];
+            const double4 xj = ld4((e.kind ? a.grec0 : a.rec0) + e.idx);
+            const double4 vj = ld4((e.kind ? a.grec1 : a.rec1) + e.idx);
             const double ih = inv_havg(xi.w, xj.w, ihi);
             const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
             double d[3];
@@ -190,7 +196,10 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_strain_coop(StepArgs
 // ------------------------------------------------- momentum + integration
 // Simple SPH: four resident blocks (64 registers) hide the gather latency
 // better than three at 80 (2.37 against 2.65 ms per step on the 2M bar, and
-// 1.58 against 1.87 ms for the strain gather above).
+// 1.58 against 1.87 ms for the strain gather above).  Records come in 32-byte
+// loads and real neighbours in a loop of their own: strain 437 -> 413 us,
+// momentum 590 -> 561 us on the 685 824-particle bar (one thread per particle
+// measured 382 and 561, two neighbours ahead 433 and 553).
 template <int L, int DISC, bool ASYM>
 __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepArgs a, int integrate) {
     __shared__ double sm[32];
@@ -217,10 +226,10 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepAr
     if (live) {
         nreal = stored_neighbours(a, t);
         gn = a.gnnbr[t];
-        xi = a.rec0[t];
-        r1i = a.rec1[t];
-        r2i = a.rec2[t];
-        if (asym) r3i = a.rec3[t];
+        xi = ld4(a.rec0 + t);
+        r1i = ld4(a.rec1 + t);
+        r2i = ld4(a.rec2 + t);
+        if (asym) r3i = ld4(a.rec3 + t);
     }
     const unsigned *spos = a.nidx + (size_t)t * a.nstride;
     const int self = (a.prm.disctype == 1) ? 1 : 0;
@@ -229,32 +238,34 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepAr
     double acc[3] = {0.0, 0.0, 0.0};
     if (DISC == 0) {
         // MCM/mcm_oldacceleration.f90:66-89: a(n) += m_j sum_m (A_j + A_i)(m,n) dW/dx_m
-        for (int k = lane; k < total; k += L) {
-            const Entry e = entry_at(a, t, k, nreal, self, spos);
-            const double4 xj = e.kind ? a.grec0[e.idx] : a.rec0[e.idx];
-            const double4 r1 = e.kind ? a.grec1[e.idx] : a.rec1[e.idx];
-            const double4 r2 = e.kind ? a.grec2[e.idx] : a.rec2[e.idx];
+        auto add = [&](const double4 &xj, const double4 &r1, const double4 &r2, const double4 &r3) {
             double d[3];
             gradw_ih(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z, inv_havg(xi.w, xj.w, ihi), d[0], d[1], d[2]);
             const double s11 = r1.x + r1i.x, s22 = r1.y + r1i.y, s33 = r1.z + r1i.z;
             const double s12 = r1.w + r1i.w, s13 = r2.x + r2i.x, s23 = r2.y + r2i.y;
             double l21 = s12, l31 = s13, l32 = s23;
-            if (asym) {
-                const double4 r3 = e.kind ? a.grec3[e.idx] : a.rec3[e.idx];
-                l21 = r3.x + r3i.x; l31 = r3.y + r3i.y; l32 = r3.z + r3i.z;
-            }
+            if (asym) { l21 = r3.x + r3i.x; l31 = r3.y + r3i.y; l32 = r3.z + r3i.z; }
             const double mj = r2.z;
             acc[0] = fma(mj, s11 * d[0] + l21 * d[1] + l31 * d[2], acc[0]);
             acc[1] = fma(mj, s12 * d[0] + s22 * d[1] + l32 * d[2], acc[1]);
             acc[2] = fma(mj, s13 * d[0] + s23 * d[1] + s33 * d[2], acc[2]);
+        };
+        int k = lane;
+        for (; k < nreal; k += L) {
+            const int p = (int)(spos[k] & kPosMask);
+            add(ld4(a.rec0 + p), ld4(a.rec1 + p), ld4(a.rec2 + p), asym ? ld4(a.rec3 + p) : r3i);
+        }
+        for (; k < total; k += L) {
+            const int q = a.gnbr[(size_t)(k - nreal) * a.npad + t];
+            add(ld4(a.grec0 + q), ld4(a.grec1 + q), ld4(a.grec2 + q), asym ? ld4(a.grec3 + q) : r3i);
         }
     } else {
         // MCM/mcm_corr_acceleration.f90:63-161
         double sw = 0.0, sg0 = 0.0, sg1 = 0.0, sg2 = 0.0;
         for (int k = lane; k < total; k += L) {
             const Entry e = entry_at(a, t, k, nreal, self, spos);
-            const double4 xj = e.kind ? a.grec0[e.idx] : a.rec0[e.idx];
-            const double4 r2 = e.kind ? a.grec2[e.idx] : a.rec2[e.idx];
+            const double4 xj = ld4((e.kind ? a.grec0 : a.rec0) + e.idx);
+            const double4 r2 = ld4((e.kind ? a.grec2 : a.rec2) + e.idx);
             const double Volj = r2.w;
             const double ih = inv_havg(xi.w, xj.w, ihi);
             const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
@@ -270,8 +281,8 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepAr
         for (int u = 0; u < 9; ++u) B[u] = 0.0;
         for (int k = lane; k < total; k += L) {
             const Entry e = entry_at(a, t, k, nreal, self, spos);
-            const double4 xj = e.kind ? a.grec0[e.idx] : a.rec0[e.idx];
-            const double4 r2 = e.kind ? a.grec2[e.idx] : a.rec2[e.idx];
+            const double4 xj = ld4((e.kind ? a.grec0 : a.rec0) + e.idx);
+            const double4 r2 = ld4((e.kind ? a.grec2 : a.rec2) + e.idx);
             const double Volj = r2.w;
             const double ih = inv_havg(xi.w, xj.w, ihi);
             const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
@@ -295,9 +306,9 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepAr
         for (int u = 0; u < 18; ++u) ds[u] = 0.0;
         for (int k = lane; k < total; k += L) {
             const Entry e = entry_at(a, t, k, nreal, self, spos);
-            const double4 xj = e.kind ? a.grec0[e.idx] : a.rec0[e.idx];
-            const double4 r1 = e.kind ? a.grec1[e.idx] : a.rec1[e.idx];
-            const double4 r2 = e.kind ? a.grec2[e.idx] : a.rec2[e.idx];
+            const double4 xj = ld4((e.kind ? a.grec0 : a.rec0) + e.idx);
+            const double4 r1 = ld4((e.kind ? a.grec1 : a.rec1) + e.idx);
+            const double4 r2 = ld4((e.kind ? a.grec2 : a.rec2) + e.idx);
             const double ih = inv_havg(xi.w, xj.w, ihi);
             const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
             double d[3];
@@ -352,7 +363,6 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepAr
             default: break;
         }
         if (a.split_mode || a.prm.diag || a.prm.veloc_opt) { f[FAX][i] = acc[0]; f[FAY][i] = acc[1]; f[FAZ][i] = acc[2]; }
-        const int mati = a.F.mat[i];
         const double mass = f[FMASS][i], vabs = f[FVABS][i];
         const double vals[5] = {0.5 * mass * (vabs * vabs), f[FE][i], mass * fabs(f[FVX][i]),
                                 mass * fabs(f[FVY][i]), mass * fabs(f[FVZ][i])};

@@ -37,13 +37,6 @@ constexpr int seq_threads(int lanes) { return lanes == 1 ? 128 : 256; }
 constexpr int seq_ahead(int lanes) { return lanes == 1 ? 1 : 2; }
 constexpr int seq_blocks(int disc, int lanes) { return lanes == 1 ? (disc ? 4 : 5) : 2; }
 
-// One 32-byte load.
-__device__ __forceinline__ double4 ld4(const double4 *p) {
-    double4 r;
-    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
-    return r;
-}
-
 // a / b, y = RN(1 / b), for a and b well inside the exponent range (in_range).
 __device__ __forceinline__ double quotient(double a, double b, double y) {
     double q = a * y;
