@@ -167,9 +167,11 @@ int alloc_cells(mcm_gpu_handle *h, long long cap) {
     long long nsum = (cap + 4095) / 4096 + 2;
     if ((st = dalloc(h, &h->A.scan_sums, (size_t)nsum))) return st;
     if ((st = dalloc(h, &h->A.gcell, (size_t)cap))) return st;
-    h->A.layer_cap = (int)std::min<long long>(cap, 1LL << 30);
-    if ((st = dalloc(h, &h->A.layer_count, (size_t)h->A.layer_cap))) return st;
-    if ((st = dalloc(h, &h->A.layer_off, (size_t)h->A.layer_cap))) return st;
+    // the six planes' layers: two per axis, each at most half of the cells
+    h->A.layer_cap = h->A.prm.boundary ? (int)std::min<long long>(3 * cap, 1LL << 30) : 1;
+    if ((st = dalloc(h, &h->A.layer_count, 2 * (size_t)h->A.layer_cap + (size_t)h->A.layer_cap / 4096 + 2))) return st;
+    h->A.layer_off = h->A.layer_count + h->A.layer_cap;
+    h->A.layer_sums = h->A.layer_off + h->A.layer_cap;
     return MCM_OK;
 }
 
@@ -350,15 +352,6 @@ int launch_move(mcm_gpu_handle *h) {
     }
 }
 
-int active_planes(const mcm_gpu_handle *h) {
-    int n = 0;
-    for (int p = 0; p < 6; ++p) {
-        int c = h->A.prm.planes.code[p & 1][p >> 1];
-        if ((c == 1 || c == 2) && (p >> 1) < h->A.prm.ndim) ++n;
-    }
-    return n;
-}
-
 // neighbours -> strain -> constitutive -> critts (MCM/mcm_solution.f90:41-53)
 void enqueue_part_a(mcm_gpu_handle *h) {
     StepArgs &a = h->A;
@@ -377,7 +370,7 @@ void enqueue_part_a(mcm_gpu_handle *h) {
         launch_cell_build(a, h->stream);
     }
     if (a.prm.boundary) {
-        Scope sc(h, R_GHOSTS, 3 * active_planes(h));
+        Scope sc(h, R_GHOSTS, 2);
         launch_ghosts(a, h->stream);
     }
     if (a.prm.skin > 0.0) {
@@ -729,7 +722,7 @@ int mcm_gpu_create(const mcm_gpu_config *cfg, const mcm_gpu_material *mats, int 
     h->A.grid = (DevGrid *)p; p += 256;
     h->A.bbox = (double *)p; p += 256;
     h->A.ngp = (int *)p; p += 64;
-    h->A.plane_base = (int *)p; p += 32;
+    h->A.ghost_ticket = (int *)p; p += 32;
     h->A.n_inside = (int *)p; p += 32;
     h->A.hmax = (double *)p; p += 32;
     h->A.skin_d2 = (unsigned long long *)p; p += 32;
@@ -764,7 +757,7 @@ int mcm_gpu_destroy(mcm_gpu_handle *h) {
                     h->A.key, h->A.cell_list, h->A.nnbr, h->A.gnnbr, h->A.rec0, h->A.rec1, h->A.rec2,
                     h->A.cpos, h->A.snx, h->A.cmat, h->A.ckey, h->A.reorder_tmp, h->A.reorder_grp, h->A.nidx,
                     h->A.red, h->A.cell_count, h->A.cell_start, h->A.scan_sums, h->A.gcell,
-                    h->A.layer_count, h->A.layer_off, h->A.gx, h->A.gy, h->A.gz, h->A.gvx, h->A.gvy,
+                    h->A.layer_count, h->A.gx, h->A.gy, h->A.gz, h->A.gvx, h->A.gvy,
                     h->A.gvz, h->A.gmass, h->A.gh, h->A.ghold, h->A.grho, h->A.gpar, h->A.gmat, h->A.gflip,
                     h->A.grec0, h->A.grec1, h->A.grec2, h->A.gnbr, h->A.rec3, h->A.grec3,
                     h->A.cidx, h->A.gcont, h->A.ncont, h->A.gncont,

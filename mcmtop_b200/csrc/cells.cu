@@ -86,6 +86,7 @@ __global__ void k_grid_setup(StepArgs a) {
     *a.grid = g;
     *a.ngp = 0;
     *a.n_inside = 0;
+    *a.ghost_ticket = 0;
 }
 
 // --------------------------------------------------------------- cell keys
@@ -426,168 +427,230 @@ void launch_reorder(const StepArgs &a, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------ ghosts
-// MCM/mcm_ghost_setup.f90:29-284.  Planes in the order xmin xmax ymin ymax
-// zmin zmax; each plane walks the 2-D layer of source cells in the
-// reference's loop order and emits, per source cell, its members in chain
-// order.  A destination cell receives the ghosts of exactly one source cell;
-// its chain order (newest first) is the reverse of the emission order.
+// MCM/mcm_ghost_setup.f90:29-284.  The reference makes the planes' ghosts one
+// plane after the other (xmin xmax ymin ymax zmin zmax): each walks the 2-D
+// layer of cells inside the plane and emits, per source cell, its members in
+// chain order into the cell outside.  A later plane's source cell may itself lie
+// in the layer of an earlier plane and then holds ghosts, newest first.  Where
+// a cell's content comes from follows from its coordinates alone, so all planes
+// are made at once: the layer cells of all planes, in the reference's order,
+// are one sequence; each looks up the cell whose real particles it mirrors and
+// through which planes, one scan over the counts gives the ghosts' numbers, and
+// then every cell writes its ghosts.  Two launches and no waiting of one plane
+// for another (one plane took 20 us and five 84 however few particles).
 
-struct PlaneGeom {
-    int d, side, src, dst, a_dim, b_dim;
-    long long L;
+// The layer cells of the active planes, plane after plane.
+struct Layers {
+    int first[7];   // of each plane's cells in the sequence
+    int gl[3];
 };
-
-__device__ __forceinline__ PlaneGeom plane_geom(const StepArgs &a, int plane) {
-    PlaneGeom p;
-    p.d = plane >> 1;
-    p.side = plane & 1;
-    const int *gl = a.grid->gridlim;
-    int code = a.prm.planes.code[p.side][p.d];
-    if (p.side == 0) p.src = (code == 1) ? 2 : gl[p.d] - 1;
-    else p.src = (code == 1) ? gl[p.d] - 1 : 2;
-    p.dst = (p.side == 0) ? 1 : gl[p.d];
-    if (p.d == 0) { p.a_dim = 2; p.b_dim = 1; }
-    else if (p.d == 1) { p.a_dim = 2; p.b_dim = 0; }
-    else { p.a_dim = 1; p.b_dim = 0; }
-    p.L = (long long)gl[p.a_dim] * gl[p.b_dim];
-    return p;
+__device__ __forceinline__ bool plane_active(const StepArgs &a, int plane) {
+    const int code = a.prm.planes.code[plane & 1][plane >> 1];
+    return (code == 1 || code == 2) && (plane >> 1) < a.prm.ndim;
+}
+__device__ __forceinline__ Layers make_layers(const StepArgs &a) {
+    Layers l;
+    for (int d = 0; d < 3; ++d) l.gl[d] = a.grid->gridlim[d];
+    l.first[0] = 0;
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+        const int d = p >> 1;
+        const int area = l.gl[d == 0 ? 1 : 0] * l.gl[d == 2 ? 1 : 2];   // below 2^31 / 2: an active axis has two layers
+        l.first[p + 1] = l.first[p] + (plane_active(a, p) ? area : 0);
+    }
+    return l;
+}
+__device__ __forceinline__ int layer_key(const Layers &l, const int *c) {
+    return (c[0] - 1) + l.gl[0] * ((c[1] - 1) + l.gl[1] * (c[2] - 1));   // below 2^31
+}
+// Coordinate of the layer that plane (d, side) mirrors.
+__device__ __forceinline__ int source_layer(const StepArgs &a, const Layers &l, int d, int side) {
+    const bool sym = a.prm.planes.code[side][d] == 1;
+    return (side == 0) == sym ? 2 : l.gl[d] - 1;
 }
 
-__device__ __forceinline__ void layer_cells(const StepArgs &a, const PlaneGeom &p, long long t, int &cs, int &cd) {
-    const int *gl = a.grid->gridlim;
-    int bcount = gl[p.b_dim];
-    int aa = (int)(t / bcount) + 1, bb = (int)(t % bcount) + 1;
+// Where layer cell t's ghosts come from: the real particles of cell `from`,
+// mirrored through planes[depth - 1], ..., planes[0] in turn; `to` receives
+// them.  Reals in a cell that also receives ghosts raise MCM_EGHOST_LAYER.
+struct Origin {
+    int from, to, count, depth, planes[3];
+};
+__device__ __forceinline__ Origin origin_of(const StepArgs &a, const Layers &l, int t) {
+    int plane = 0;
+#pragma unroll
+    for (int p = 1; p < 6; ++p)
+        if (t >= l.first[p]) plane = p;
+    const int d = plane >> 1, side = plane & 1;
+    const int ad = d == 2 ? 1 : 2, bd = d == 0 ? 1 : 0;   // the layer's outer and inner axis
+    const int r = t - l.first[plane];
+    const int nb = l.gl[bd];
     int c[3];
-    c[p.a_dim] = aa; c[p.b_dim] = bb;
-    c[p.d] = p.src;
-    cs = (int)cell_key(c[0], c[1], c[2], gl);
-    c[p.d] = p.dst;
-    cd = (int)cell_key(c[0], c[1], c[2], gl);
+    c[ad] = r / nb + 1;
+    c[bd] = r - (c[ad] - 1) * nb + 1;
+    Origin o;
+    c[d] = side == 0 ? 1 : l.gl[d];
+    o.to = layer_key(l, c);
+    c[d] = source_layer(a, l, d, side);
+    o.depth = 1;
+    o.planes[0] = plane;
+    o.count = 0;
+    bool found = false, mixed = false;
+    // down through the earlier planes whose layer the cell lies in
+#pragma unroll
+    for (int e = 2; e >= 0; --e) {
+        if (e >= d) continue;
+        const int es = c[e] == 1 && plane_active(a, 2 * e) ? 0 : (c[e] == l.gl[e] && plane_active(a, 2 * e + 1) ? 1 : -1);
+        if (es < 0) continue;
+        const int k = layer_key(l, c);
+        const int n = a.cell_start[k + 1] - a.cell_start[k];
+        if (n > 0 && !found) {   // reals in a layer cell: they are what is mirrored
+            o.from = k;
+            o.count = n;
+            found = true;
+        }
+        c[e] = source_layer(a, l, e, es);
+        if (!found) {
+            if (o.depth == 1) o.planes[1] = 2 * e + es;
+            else o.planes[2] = 2 * e + es;
+            ++o.depth;
+        }
+    }
+    const int k = layer_key(l, c);
+    const int n = a.cell_start[k + 1] - a.cell_start[k];
+    if (found) {
+        mixed = n > 0;
+    } else {
+        o.from = k;
+        o.count = n;
+    }
+    if (o.count > 0 && (mixed || a.cell_start[o.to + 1] > a.cell_start[o.to]))
+        raise_status(a.status, MCM_EGHOST_LAYER, mixed ? o.from : o.to);
+    return o;
 }
 
-__global__ void k_ghost_count(StepArgs a, int plane) {
-    if (a.status->code) return;
-    PlaneGeom p = plane_geom(a, plane);
-    if (p.L > a.layer_cap) {
+// Counts of the layer cells and their prefix sums: within a chunk in
+// layer_off, over the chunks in layer_sums (by the block that ends last).
+__global__ void __launch_bounds__(kScanThreads) k_ghost_count(StepArgs a) {
+    __shared__ int smem[32];
+    __shared__ int last;
+    if (a.status->code && a.status->code != MCM_EGHOST_LAYER) return;   // EGHOST_LAYER may be this launch's own
+    const Layers l = make_layers(a);
+    const int T = l.first[6];
+    if (T < 0 || T > a.layer_cap) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_status(a.status, MCM_EGRID_OVERFLOW);
         return;
     }
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < p.L; t += (long long)gridDim.x * blockDim.x) {
-        int cs, cd;
-        layer_cells(a, p, t, cs, cd);
-        int nreal = a.cell_start[cs + 1] - a.cell_start[cs];
-        int ng = a.gcell[cs].y;
-        if (nreal > 0 && ng > 0) raise_status(a.status, MCM_EGHOST_LAYER, cs);
-        int cnt = nreal > 0 ? nreal : ng;
-        if (cnt > 0) {
-            int dreal = a.cell_start[cd + 1] - a.cell_start[cd];
-            if (dreal > 0 || a.gcell[cd].y > 0) raise_status(a.status, MCM_EGHOST_LAYER, cd);
-        }
-        a.layer_count[t] = cnt;
+    const int base = blockIdx.x * kScanChunk;
+    const int nblocks = (T + kScanChunk - 1) / kScanChunk;   // blocks that hold layer cells
+    if ((int)blockIdx.x >= nblocks) return;
+    int v[kScanItems];
+    int local = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+        const int t = base + threadIdx.x * kScanItems + k;
+        v[k] = t < T ? origin_of(a, l, t).count : 0;
+        local += v[k];
     }
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_ghost_layer_scan(StepArgs a, int plane) {
-    __shared__ int smem[32];
-    if (a.status->code) return;
-    PlaneGeom p = plane_geom(a, plane);
+    int total;
+    int pre = block_exclusive_scan(local, smem, total);
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+        const int t = base + threadIdx.x * kScanItems + k;
+        if (t < T) {
+            a.layer_count[t] = v[k];
+            a.layer_off[t] = pre;
+        }
+        pre += v[k];
+    }
     int carry = 0;
-    for (long long base = 0; base < p.L; base += kScanThreads) {
-        long long idx = base + threadIdx.x;
-        int v = idx < p.L ? a.layer_count[idx] : 0;
-        int total;
-        int pre = block_exclusive_scan(v, smem, total);
-        if (idx < p.L) a.layer_off[idx] = pre + carry;
+    if (nblocks == 1) {
+        if (threadIdx.x == 0) a.layer_sums[0] = 0;
+        carry = total;
+    } else {
+        if (threadIdx.x == 0) {
+            a.layer_sums[blockIdx.x] = total;
+            __threadfence();
+            last = atomicAdd(a.ghost_ticket, 1) == nblocks - 1;
+        }
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+    }
+    for (int b = 0; nblocks > 1 && b < nblocks; b += kScanThreads) {
+        const int q = b + threadIdx.x;
+        const int n = q < nblocks ? *(volatile int *)(a.layer_sums + q) : 0;
+        const int p = block_exclusive_scan(n, smem, total);
+        if (q < nblocks) a.layer_sums[q] = p + carry;
         carry += total;
     }
     if (threadIdx.x == 0) {
-        int base = *a.ngp;
-        *a.plane_base = base;
-        long long need = (long long)base + carry;
-        if (need > a.ghost_cap) {
-            if (need > a.status->req_ngp) a.status->req_ngp = (int)need;
+        if (carry > a.ghost_cap) {
+            if (carry > a.status->req_ngp) a.status->req_ngp = carry;
             raise_status(a.status, MCM_EGHOST_OVERFLOW);
         }
-        *a.ngp = (int)need;
+        *a.ngp = carry;
     }
 }
 
-__global__ void k_ghost_emit(StepArgs a, int plane) {
+// One warp per layer cell, its lanes over the cell's ghosts.
+__global__ void k_ghost_emit(StepArgs a) {
     if (a.status->code) return;
-    PlaneGeom p = plane_geom(a, plane);
-    const double *mult = a.prm.planes.mult[plane];
-    const double *add = a.prm.planes.add[plane];
-    const int base = *a.plane_base;
-    // axes this plane mirrors (bit d: x_d -> -x_d + add_d); composed along ghost chains
-    const int flips = (mult[0] < 0.0 ? 1 : 0) | (mult[1] < 0.0 ? 2 : 0) | (mult[2] < 0.0 ? 4 : 0);
-    // one warp per layer cell, its lanes over the cell's ghosts (the sources
-    // are real particles or ghosts of earlier planes, so no ghost of this
-    // launch reads another)
+    const Layers l = make_layers(a);
+    const int T = l.first[6];
     const int lane = threadIdx.x & 31;
-    const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long t = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); t < p.L; t += nw) {
-        int cnt = a.layer_count[t];
+    const int nw = gridDim.x * (blockDim.x >> 5);
+    for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < T; t += nw) {
+        const int cnt = a.layer_count[t];
         if (cnt == 0) continue;
-        int cs, cd;
-        layer_cells(a, p, t, cs, cd);
-        int g0 = base + a.layer_off[t];
-        if (lane == 0) a.gcell[cd] = make_int2(g0, cnt);
-        int rs = a.cell_start[cs];
-        int nreal = a.cell_start[cs + 1] - rs;
-        int2 src = a.gcell[cs];
+        const Origin o = origin_of(a, l, t);
+        const int g0 = a.layer_sums[t / kScanChunk] + a.layer_off[t];
+        if (lane == 0) a.gcell[o.to] = make_int2(g0, cnt);
+        const int rs = a.cell_start[o.from];
         for (int r = lane; r < cnt; r += 32) {
-            int g = g0 + r;
-            if (nreal > 0) {
-                // MCM/mcm_ghost_setup.f90:324-355 (create_ghost_from_real)
-                int j = a.cell_list[rs + r];
-                a.gpar[g] = j;
-                a.gflip[g] = flips;
-                a.gmat[g] = a.F.mat[j];
-                a.gmass[g] = a.F.f[FMASS][j];
-                a.gh[g] = a.F.f[FH][j];
-                a.ghold[g] = a.F.f[FHOLD][j];
-                a.grho[g] = a.F.f[FRHO][j];
-                a.gx[g] = a.F.f[FX][j] * mult[0] + add[0];
-                a.gy[g] = a.F.f[FY][j] * mult[1] + add[1];
-                a.gz[g] = a.F.f[FZ][j] * mult[2] + add[2];
-                a.gvx[g] = a.F.f[FVX][j] * mult[0];
-                a.gvy[g] = a.F.f[FVY][j] * mult[1];
-                a.gvz[g] = a.F.f[FVZ][j] * mult[2];
-            } else {
-                // MCM/mcm_ghost_setup.f90:392-423 (create_ghost_from_ghost); chain order = newest first
-                int q = src.x + src.y - 1 - r;
-                a.gpar[g] = a.gpar[q];
-                a.gflip[g] = a.gflip[q] ^ flips;
-                a.gmat[g] = a.gmat[q];
-                a.gmass[g] = a.gmass[q];
-                a.gh[g] = a.gh[q];
-                a.ghold[g] = a.ghold[q];
-                a.grho[g] = a.grho[q];
-                a.gx[g] = a.gx[q] * mult[0] + add[0];
-                a.gy[g] = a.gy[q] * mult[1] + add[1];
-                a.gz[g] = a.gz[q] * mult[2] + add[2];
-                a.gvx[g] = a.gvx[q] * mult[0];
-                a.gvy[g] = a.gvy[q] * mult[1];
-                a.gvz[g] = a.gvz[q] * mult[2];
+            const int g = g0 + r;
+            // MCM/mcm_ghost_setup.f90:324-355 (create_ghost_from_real), :392-423
+            // (create_ghost_from_ghost: the chain's order turns round each time)
+            const int j = a.cell_list[rs + ((o.depth & 1) ? r : cnt - 1 - r)];
+            double x[3] = {a.F.f[FX][j], a.F.f[FY][j], a.F.f[FZ][j]};
+            double v[3] = {a.F.f[FVX][j], a.F.f[FVY][j], a.F.f[FVZ][j]};
+            int flips = 0;
+#pragma unroll
+            for (int q = 2; q >= 0; --q) {
+                if (q >= o.depth) continue;
+                const int plane = o.planes[q];
+                const double *mult = a.prm.planes.mult[plane];
+                const double *add = a.prm.planes.add[plane];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    x[d] = x[d] * mult[d] + add[d];
+                    v[d] = v[d] * mult[d];
+                    // axes mirrored (bit d: x_d -> -x_d + add_d), composed along the chain
+                    if (mult[d] < 0.0) flips ^= 1 << d;
+                }
             }
+            a.gpar[g] = j;
+            a.gflip[g] = flips;
+            a.gmat[g] = a.F.mat[j];
+            a.gmass[g] = a.F.f[FMASS][j];
+            a.gh[g] = a.F.f[FH][j];
+            a.ghold[g] = a.F.f[FHOLD][j];
+            a.grho[g] = a.F.f[FRHO][j];
+            a.gx[g] = x[0];
+            a.gy[g] = x[1];
+            a.gz[g] = x[2];
+            a.gvx[g] = v[0];
+            a.gvy[g] = v[1];
+            a.gvz[g] = v[2];
         }
     }
 }
 
 void launch_ghosts(const StepArgs &a, cudaStream_t s) {
     cudaMemsetAsync(a.gcell, 0, sizeof(int2) * (size_t)a.cell_cap, s);
-    for (int plane = 0; plane < 6; ++plane) {
-        int code = a.prm.planes.code[plane & 1][plane >> 1];
-        if (code != 1 && code != 2) continue;
-        if ((plane >> 1) >= a.prm.ndim) continue;
-        int blocks = grid_blocks(a.layer_cap, 256);
-        if (blocks > 592) blocks = 592;
-        k_ghost_count<<<blocks, 256, 0, s>>>(a, plane);
-        k_ghost_layer_scan<<<1, kScanThreads, 0, s>>>(a, plane);
-        long long eb = ((long long)a.layer_cap + 7) / 8;   // 8 warps (layer cells) per block
-        if (eb > 148LL * 8) eb = 148LL * 8;
-        k_ghost_emit<<<(unsigned)(eb < 1 ? 1 : eb), 256, 0, s>>>(a, plane);
-    }
+    k_ghost_count<<<(unsigned)((a.layer_cap + kScanChunk - 1) / kScanChunk), kScanThreads, 0, s>>>(a);
+    long long eb = ((long long)a.layer_cap + 7) / 8;   // 8 warps (layer cells) per block
+    if (eb > 148LL * 4) eb = 148LL * 4;
+    k_ghost_emit<<<(unsigned)(eb < 1 ? 1 : eb), 256, 0, s>>>(a);
 }
 
 // ------------------------------------------------------------------ search

@@ -14,7 +14,7 @@ struct StepArgs {
     int gstride;      // ghost-neighbour table width (int32 entries)
     int ghost_cap;    // ghost storage
     long long cell_cap;   // cell-array storage
-    int layer_cap;    // scratch for one boundary layer
+    int layer_cap;    // scratch for the planes' layer cells
     int share;        // bodies of this one's size that run on the GPU at the same time (a batch's lanes)
     int split_mode;   // 1: step_a/b/c entry points (dt supplied by the host); 0: fused run
     DevParams prm;
@@ -45,8 +45,8 @@ struct StepArgs {
     int *gpar, *gmat;
     int *gflip;       // per ghost: bit d set if its position is the parent's mirrored along axis d
     int *ngp;         // device ghost counter
-    int *plane_base;  // ghost index base of the plane being built
-    int *layer_count, *layer_off;
+    int *ghost_ticket;                           // blocks of k_ghost_count that have ended
+    int *layer_count, *layer_off, *layer_sums;   // per layer cell of all planes: ghosts, their prefix within a chunk; per chunk
     // neighbour lists, per position p, in the reference order (same-material
     // neighbours, then contacts; rows in z, y order, cells in x order, each
     // cell in descending reference index): entry k of p at
