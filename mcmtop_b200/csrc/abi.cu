@@ -162,7 +162,9 @@ int alloc_particles(mcm_gpu_handle *h) {
 int alloc_cells(mcm_gpu_handle *h, long long cap) {
     int st;
     h->A.cell_cap = cap;
-    if ((st = dalloc(h, &h->A.cell_count, (size_t)cap))) return st;
+    if ((st = dalloc(h, &h->A.cell_count, 2 * (size_t)cap))) return st;
+    h->A.cell_local = h->A.cell_count + cap;
+    CK(cudaMemsetAsync(h->A.cell_count, 0, sizeof(int) * (size_t)cap, h->stream));
     if ((st = dalloc(h, &h->A.cell_start, (size_t)cap + 1))) return st;
     long long nsum = (cap + 4095) / 4096 + 2;
     if ((st = dalloc(h, &h->A.scan_sums, (size_t)nsum))) return st;
@@ -300,12 +302,6 @@ int regrow(mcm_gpu_handle *h, int *grew) {
 int launch_strain(mcm_gpu_handle *h) {
     const int prec = h->cfg.precision;
     {
-        Scope sc(h, R_STRAIN_PREP, 1);
-        if (prec == MCM_PREC_FP64_EXACT) exact::launch_strain_prep(h->A, h->stream);
-        else if (prec == MCM_PREC_MIXED) mixed::launch_strain_prep(h->A, h->stream);
-        else fast::launch_strain_prep(h->A, h->stream);
-    }
-    {
         Scope sc(h, R_STRAIN, 1);
         if (prec == MCM_PREC_FP64_EXACT) exact::launch_strain(h->A, h->stream);
         else if (prec == MCM_PREC_MIXED) mixed::launch_strain(h->A, h->stream);
@@ -365,8 +361,7 @@ void enqueue_part_a(mcm_gpu_handle *h) {
     ++h->steps_enqueued;
     h->have_cells = true;
     {
-        Scope sc(h, R_CELLS, 8);
-        launch_grid_setup(a, h->stream);
+        Scope sc(h, R_CELLS, 4);
         launch_cell_build(a, h->stream);
     }
     if (a.prm.boundary) {
@@ -723,7 +718,8 @@ int mcm_gpu_create(const mcm_gpu_config *cfg, const mcm_gpu_material *mats, int 
     h->A.bbox = (double *)p; p += 256;
     h->A.ngp = (int *)p; p += 64;
     h->A.ghost_ticket = (int *)p; p += 32;
-    h->A.n_inside = (int *)p; p += 32;
+    h->A.n_inside = (int *)p;
+    h->A.scan_ticket = (int *)p + 1; p += 32;
     h->A.hmax = (double *)p; p += 32;
     h->A.skin_d2 = (unsigned long long *)p; p += 32;
     h->A.skin_flags = (int *)p; p += 32;
@@ -874,7 +870,6 @@ int run_search_only(mcm_gpu_handle *h) {
         int st;
         if ((st = reset_status(h))) return st;
         StepArgs &a = h->A;
-        launch_grid_setup(a, h->stream);
         launch_cell_build(a, h->stream);
         if (a.prm.boundary) launch_ghosts(a, h->stream);
         launch_search(a, h->stream);

@@ -18,14 +18,11 @@
 namespace mcm {
 
 // ------------------------------------------------------------- grid set-up
-// MCM/mcm_setuplist.f90:30-81 (one thread).
-__global__ void k_grid_setup(StepArgs a) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (a.status->code) return;
+// MCM/mcm_setuplist.f90:30-81; true when a span has no finite cell count.
+__device__ __forceinline__ bool make_grid(const StepArgs &a, DevGrid &g) {
     const DevParams &P = a.prm;
     const double factor = 2.0;
     const double hmax = a.hmax[0];   // fixed, or the last mcm_update_h's maximum
-    DevGrid g;
     for (int i = 0; i < 3; ++i) {
         g.gridmin[i] = 0.0;
         g.gridlim[i] = 1;
@@ -75,25 +72,38 @@ __global__ void k_grid_setup(StepArgs a) {
     g.pad = 0;
     for (int i = 0; i < 3; ++i) g.cell[i] = 1.0 / g.gridsize[i];
     g.ncells = (long long)g.gridlim[0] * g.gridlim[1] * g.gridlim[2];
-    if (bad || g.ncells >= (1LL << 31)) {
-        raise_status(a.status, MCM_EGRID_TOO_LARGE);
-    } else if (g.ncells > a.cell_cap) {
-        a.status->req_cells = g.ncells;
-        raise_status(a.status, MCM_EGRID_OVERFLOW);
-    }
-    g.hcut = 0.0;                                     // raised by k_cell_records
-    g.hmin = __longlong_as_double(0x7fffffffffffffffll);   // lowered by k_cell_records
-    *a.grid = g;
-    *a.ngp = 0;
-    *a.n_inside = 0;
-    *a.ghost_ticket = 0;
+    g.hcut = 0.0;                                          // raised by k_cell_order
+    g.hmin = __longlong_as_double(0x7fffffffffffffffll);   // lowered by k_cell_order
+    return bad;
 }
 
 // --------------------------------------------------------------- cell keys
-// MCM/mcm_setuplist.f90:110-135: particles outside the grid get no cell.
-__global__ void k_cell_keys(StepArgs a) {
+// The grid (every block forms it for itself, block 0 writes it down), the
+// particles' cells (MCM/mcm_setuplist.f90:110-135: particles outside the grid
+// get none) and the cells' counts.  cell_count is zero on entry: the scatter
+// takes every count down to zero again.
+__global__ void __launch_bounds__(256) k_cell_keys(StepArgs a) {
+    __shared__ DevGrid g;
+    __shared__ int stop;
     if (a.status->code) return;
-    const DevGrid g = *a.grid;
+    if (threadIdx.x == 0) {
+        const bool bad = make_grid(a, g);
+        stop = (bad || g.ncells >= (1LL << 31)) ? MCM_EGRID_TOO_LARGE : g.ncells > a.cell_cap ? MCM_EGRID_OVERFLOW : 0;
+        if (blockIdx.x == 0) {
+            if (stop == MCM_EGRID_OVERFLOW) a.status->req_cells = g.ncells;
+            if (stop) raise_status(a.status, stop);
+            *a.grid = g;
+            *a.ngp = 0;
+            *a.n_inside = 0;
+            *a.scan_ticket = 0;
+            *a.ghost_ticket = 0;
+        }
+    }
+    __syncthreads();
+    if (stop) return;
+    if (a.prm.boundary)
+        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < (int)g.ncells; c += gridDim.x * blockDim.x)
+            a.gcell[c] = make_int2(0, 0);
     const int ndim = a.prm.ndim;
     const double *X[3] = {a.F.f[FX], a.F.f[FY], a.F.f[FZ]};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
@@ -117,9 +127,11 @@ __global__ void k_cell_keys(StepArgs a) {
 }
 
 // ------------------------------------------------------------------- scan
-// Exclusive scan of cell_count[0, ncells) into cell_start[0, ncells].  A grid
-// larger than the cell arrays has raised the status in k_grid_setup: nothing
-// is read or written then (the step is run again once the arrays have grown).
+// Exclusive prefix of cell_count: within a chunk of cells in cell_local, over
+// the chunks in scan_sums (by the block that ends last; the total behind
+// them).  A grid larger than the cell arrays has raised the status in
+// k_cell_keys: nothing is read or written then (the step is run again once the
+// arrays have grown).
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanChunk = kScanThreads * kScanItems;
@@ -150,73 +162,58 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *smem, int &total
     return prefix;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_blocks(const int *in, int *out, int *sums, const long long *np_dev,
-                                                              const DevStatus *status) {
+
+__global__ void __launch_bounds__(kScanThreads) k_cell_scan(StepArgs a) {
     __shared__ int smem[32];
-    if (status->code) return;
-    long long n = *np_dev;
-    long long base = (long long)blockIdx.x * kScanChunk;
+    __shared__ int last;
+    if (a.status->code) return;
+    const int n = (int)a.grid->ncells;
+    const int nblocks = (n + kScanChunk - 1) / kScanChunk;
+    if ((int)blockIdx.x >= nblocks) return;
+    const int base = blockIdx.x * kScanChunk + threadIdx.x * kScanItems;
     int v[kScanItems];
     int local = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        long long idx = base + (long long)threadIdx.x * kScanItems + k;
-        v[k] = (idx < n) ? in[idx] : 0;
+        v[k] = base + k < n ? a.cell_count[base + k] : 0;
         local += v[k];
     }
     int total;
     int pre = block_exclusive_scan(local, smem, total);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        long long idx = base + (long long)threadIdx.x * kScanItems + k;
-        if (idx < n) out[idx] = pre;
+        if (base + k < n) a.cell_local[base + k] = pre;
         pre += v[k];
     }
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan_sums(int *sums, int nblocks, const DevStatus *status) {
-    __shared__ int smem[32];
-    if (status->code) return;
+    if (threadIdx.x == 0) {
+        a.scan_sums[blockIdx.x] = total;
+        __threadfence();
+        last = atomicAdd(a.scan_ticket, 1) == nblocks - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
     int carry = 0;
-    for (int base = 0; base < nblocks; base += kScanThreads) {
-        int idx = base + threadIdx.x;
-        int v = idx < nblocks ? sums[idx] : 0;
-        int total;
-        int pre = block_exclusive_scan(v, smem, total);
-        if (idx < nblocks) sums[idx] = pre + carry;
+    for (int b = 0; b < nblocks; b += kScanThreads) {
+        const int q = b + threadIdx.x;
+        const int w = q < nblocks ? *(volatile int *)(a.scan_sums + q) : 0;
+        const int p = block_exclusive_scan(w, smem, total);
+        if (q < nblocks) a.scan_sums[q] = p + carry;
         carry += total;
     }
-    if (threadIdx.x == 0) sums[nblocks] = carry;
-}
-
-__global__ void k_scan_add(int *out, const int *sums, const long long *np_dev, int nblocks, const DevStatus *status) {
-    if (status->code) return;
-    long long n = *np_dev;
-    long long base = (long long)blockIdx.x * kScanChunk;
-    int add = sums[blockIdx.x];
-    for (int k = threadIdx.x; k < kScanChunk; k += blockDim.x) {
-        long long idx = base + k;
-        if (idx < n) out[idx] += add;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = sums[nblocks];
-}
-
-static void device_exclusive_scan(const int *in, int *out, int *sums, const long long *n_dev, long long cap,
-                                  const DevStatus *status, cudaStream_t s) {
-    int nblocks = (int)((cap + kScanChunk - 1) / kScanChunk);
-    if (nblocks < 1) nblocks = 1;
-    k_scan_blocks<<<nblocks, kScanThreads, 0, s>>>(in, out, sums, n_dev, status);
-    k_scan_sums<<<1, kScanThreads, 0, s>>>(sums, nblocks, status);
-    k_scan_add<<<nblocks, 256, 0, s>>>(out, sums, n_dev, nblocks, status);
+    if (threadIdx.x == 0) a.scan_sums[nblocks] = carry;
 }
 
 // --------------------------------------------------------------- scatter
-// Particles outside the grid (llpointer = -1 in the reference) take the
-// positions after the last cell; they have no neighbours and are never one.
-__global__ void k_cell_scatter(StepArgs a) {
+// The cells' first positions, and the particles into their cells.  Particles
+// outside the grid (llpointer = -1 in the reference) take the positions after
+// the last cell; they have no neighbours and are never one.
+__global__ void __launch_bounds__(256) k_cell_scatter(StepArgs a) {
     if (a.status->code) return;
-    const int base_out = a.cell_start[a.grid->ncells];
+    const int ncells = (int)a.grid->ncells;
+    const int base_out = a.scan_sums[(ncells + kScanChunk - 1) / kScanChunk];
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncells; c += gridDim.x * blockDim.x)
+        a.cell_start[c] = c < ncells ? a.cell_local[c] + a.scan_sums[c / kScanChunk] : base_out;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
         int key = a.key[i];
         const unsigned act = __activemask();
@@ -232,65 +229,11 @@ __global__ void k_cell_scatter(StepArgs a) {
         if (lane == lead) top = atomicSub(&a.cell_count[key], __popc(grp));
         top = __shfl_sync(grp, top, lead);
         int slot = top - 1 - __popc(grp & ((1u << lane) - 1u));
-        a.cell_list[a.cell_start[key] + slot] = i;
+        a.cell_list[a.cell_local[key] + a.scan_sums[key / kScanChunk] + slot] = i;
     }
 }
 
-// Candidate records in cell order (positions at neighbour time): FP64 position
-// and h, and the FP32 coordinates by which the search decides all but the
-// near-tie candidates: negated, one array each, x relative to the grid origin
-// (the candidates of a row's two or three cells share one frame in x), y and z
-// relative to the origin of the particle's own cell.  cposf (all three
-// relative to the cell, h) is kept for the searches that read it.
-__global__ void __launch_bounds__(256) k_cell_records(StepArgs a, int with_cposf) {
-    __shared__ unsigned long long smax[8], smin[8];
-    if (a.status->code) return;
-    const double *X = a.F.f[FX], *Y = a.F.f[FY], *Z = a.F.f[FZ], *H = a.F.f[FH];
-    const DevGrid g = *a.grid;
-    unsigned long long hbits = 0ull, lbits = ~0ull;   // h > 0: the bit pattern orders like the value
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x) {
-        int i = a.cell_list[p];
-        const double x = X[i], y = Y[i], z = Z[i], h = H[i];
-        a.cpos[p] = make_double4(x, y, z, h);
-        if (a.pos_of) a.pos_of[i] = p;
-        a.cmat[p] = a.F.mat[i];
-        const int key = a.key[i];
-        a.ckey[p] = key;
-        float4 r = make_float4(0.f, 0.f, 0.f, (float)h);
-        if (key >= 0) {
-            int bx, by, bz;
-            cell_coords(key, g.gridlim, bx, by, bz);
-            r.x = (float)(x - cell_origin(g, 0, bx));
-            r.y = (float)(y - cell_origin(g, 1, by));
-            r.z = (float)(z - cell_origin(g, 2, bz));
-            const unsigned long long hb = (unsigned long long)__double_as_longlong(h);
-            hbits = hb > hbits ? hb : hbits;
-            lbits = hb < lbits ? hb : lbits;
-        }
-        if (with_cposf) a.cposf[p] = r;
-        a.snx[p] = -(float)(x - g.gridmin[0]);
-        a.sny[p] = -r.y;
-        a.snz[p] = -r.z;
-        a.snh[p] = r.w;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long v = __shfl_xor_sync(0xffffffffu, hbits, o);
-        const unsigned long long u = __shfl_xor_sync(0xffffffffu, lbits, o);
-        hbits = v > hbits ? v : hbits;
-        lbits = u < lbits ? u : lbits;
-    }
-    if ((threadIdx.x & 31) == 0) { smax[threadIdx.x >> 5] = hbits; smin[threadIdx.x >> 5] = lbits; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-            hbits = smax[w] > hbits ? smax[w] : hbits;
-            lbits = smin[w] < lbits ? smin[w] : lbits;
-        }
-        atomicMax(reinterpret_cast<unsigned long long *>(&a.grid->hcut), hbits);
-        atomicMin(reinterpret_cast<unsigned long long *>(&a.grid->hmin), lbits);
-    }
-}
-
+// ------------------------------------------------------- order and records
 // Per-cell order: descending reference index (head insertion in
 // MCM/mcm_setuplist.f90:126-130 over i = 1..np ascending), the order of the
 // reference's lists.  (Ascending x, which lets a search window its rows,
@@ -302,16 +245,72 @@ __global__ void __launch_bounds__(256) k_cell_records(StepArgs a, int with_cposf
 // the ranks are a permutation); all ranks are known before any entry is
 // written back.  Cells of more than 32 * kSortPer particles are sorted by
 // insertion in one lane.
+//
+// The lane that has placed a particle writes its records: FP64 position and h,
+// the FP32 coordinates by which the search decides all but the near-tie
+// candidates (negated, one array each, x relative to the grid origin, so that
+// the candidates of a row's two or three cells share one frame in x, y and z
+// relative to the origin of the particle's own cell; cposf, all three relative
+// to the cell, for the searches that read it), and the strain gather's record
+// of the step's arithmetic REC: positions shifted back half a step
+// (MCM/mcm_strain.f90:27-31), velocities and V = m/rho
+// (MCM/mcm_oldstrain.f90:44).
+enum { kRecFP64 = 0, kRecMixed = 1 };
+template <int REC>
+__device__ __forceinline__ void write_records(const StepArgs &a, const DevGrid &g, int p, int i, int key, double dt,
+                                              bool with_cposf, unsigned long long &hbits, unsigned long long &lbits) {
+    const double *const *f = a.F.f;
+    const double x = f[FX][i], y = f[FY][i], z = f[FZ][i], h = f[FH][i];
+    const double vx = f[FVX][i], vy = f[FVY][i], vz = f[FVZ][i];
+    a.cpos[p] = make_double4(x, y, z, h);
+    if (a.pos_of) a.pos_of[i] = p;
+    a.cmat[p] = a.F.mat[i];
+    a.ckey[p] = key;
+    double o[3] = {0.0, 0.0, 0.0};
+    float4 r = make_float4(0.f, 0.f, 0.f, (float)h);
+    if (key >= 0) {
+        int b[3];
+        cell_coords(key, g.gridlim, b[0], b[1], b[2]);
+        for (int d = 0; d < 3; ++d) o[d] = cell_origin(g, d, b[d]);
+        r.x = (float)(x - o[0]);
+        r.y = (float)(y - o[1]);
+        r.z = (float)(z - o[2]);
+        const unsigned long long hb = (unsigned long long)__double_as_longlong(h);   // h > 0: bits order like values
+        hbits = hb > hbits ? hb : hbits;
+        lbits = hb < lbits ? hb : lbits;
+    }
+    if (with_cposf) a.cposf[p] = r;
+    a.snx[p] = -(float)(x - g.gridmin[0]);
+    a.sny[p] = -r.y;
+    a.snz[p] = -r.z;
+    a.snh[p] = r.w;
+    const double xs = x - 0.5 * vx * dt, ys = y - 0.5 * vy * dt, zs = z - 0.5 * vz * dt;
+    const double vol = f[FMASS][i] / f[FRHO][i];
+    if (REC == kRecMixed) {
+        a.frec0[2 * (size_t)p] = make_float4((float)(xs - o[0]), (float)(ys - o[1]), (float)(zs - o[2]), (float)h);
+        a.frec0[2 * (size_t)p + 1] = make_float4((float)vx, (float)vy, (float)vz, (float)vol);
+    } else {
+        a.rec0[p] = make_double4(xs, ys, zs, h);
+        a.rec1[p] = make_double4(vx, vy, vz, vol);
+    }
+}
+
 constexpr int kSortPer = 4;
-__global__ void __launch_bounds__(256) k_cell_sort(StepArgs a) {
+template <int REC>
+__global__ void __launch_bounds__(256) k_cell_order(StepArgs a, int with_cposf) {
+    __shared__ DevGrid g;
+    __shared__ unsigned long long smax[8], smin[8];
     if (a.status->code) return;
-    const long long ncells = a.grid->ncells;
+    if (threadIdx.x == 0) g = *a.grid;
+    __syncthreads();
+    const int ncells = (int)g.ncells;
+    const double dt = a.time->dt;
     const int lane = threadIdx.x & 31;
-    const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long c = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += nw) {
+    const int nw = gridDim.x * (blockDim.x >> 5);
+    unsigned long long hbits = 0ull, lbits = ~0ull;
+    for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += nw) {
         const int s = a.cell_start[c], e = a.cell_start[c + 1];
         const int n = e - s;
-        if (n < 2) continue;   // warp-uniform
         if (n <= 32) {
             // one particle per lane (the common case)
             const bool on = lane < n;
@@ -320,9 +319,14 @@ __global__ void __launch_bounds__(256) k_cell_sort(StepArgs a) {
             int rank = 0;
             for (int k = 0; k < n; ++k) rank += __shfl_sync(0xffffffffu, o, k) > o ? 1 : 0;
             __syncwarp();
-            if (on) a.cell_list[s + rank] = v;
+            if (on) {
+                a.cell_list[s + rank] = v;
+                write_records<REC>(a, g, s + rank, v, c, dt, with_cposf != 0, hbits, lbits);
+            }
             __syncwarp();
-        } else if (n <= 32 * kSortPer) {
+            continue;
+        }
+        if (n <= 32 * kSortPer) {
             int v[kSortPer], o[kSortPer], rank[kSortPer];
 #pragma unroll
             for (int u = 0; u < kSortPer; ++u) {
@@ -350,7 +354,6 @@ __global__ void __launch_bounds__(256) k_cell_sort(StepArgs a) {
 #pragma unroll
             for (int u = 0; u < kSortPer; ++u)
                 if (lane + 32 * u < n) a.cell_list[s + rank[u]] = v[u];
-            __syncwarp();
         } else if (lane == 0) {
             for (int k = s + 1; k < e; ++k) {
                 const int v = a.cell_list[k];
@@ -363,6 +366,29 @@ __global__ void __launch_bounds__(256) k_cell_sort(StepArgs a) {
                 a.cell_list[m + 1] = v;
             }
         }
+        __syncwarp();
+        for (int p = s + lane; p < e; p += 32)
+            write_records<REC>(a, g, p, a.cell_list[p], c, dt, with_cposf != 0, hbits, lbits);
+        __syncwarp();
+    }
+    // particles outside the grid
+    for (int p = a.cell_start[ncells] + blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x)
+        write_records<REC>(a, g, p, a.cell_list[p], kNoCell, dt, with_cposf != 0, hbits, lbits);
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long v = __shfl_xor_sync(0xffffffffu, hbits, o);
+        const unsigned long long u = __shfl_xor_sync(0xffffffffu, lbits, o);
+        hbits = v > hbits ? v : hbits;
+        lbits = u < lbits ? u : lbits;
+    }
+    if (lane == 0) { smax[threadIdx.x >> 5] = hbits; smin[threadIdx.x >> 5] = lbits; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
+            hbits = smax[w] > hbits ? smax[w] : hbits;
+            lbits = smin[w] < lbits ? smin[w] : lbits;
+        }
+        atomicMax(reinterpret_cast<unsigned long long *>(&a.grid->hcut), hbits);
+        atomicMin(reinterpret_cast<unsigned long long *>(&a.grid->hmin), lbits);
     }
 }
 
@@ -373,20 +399,18 @@ static int grid_blocks(long long work, int threads) {
     return (int)b;
 }
 
-void launch_grid_setup(const StepArgs &a, cudaStream_t s) { k_grid_setup<<<1, 32, 0, s>>>(a); }
-
+// Four launches: keys and counts, their scan, the scatter, the order within
+// the cells with everything that is written per particle in cell order.
 void launch_cell_build(const StepArgs &a, cudaStream_t s) {
-    cudaMemsetAsync(a.cell_count, 0, sizeof(int) * (size_t)a.cell_cap, s);
-    k_cell_keys<<<grid_blocks(a.n, 256), 256, 0, s>>>(a);
-    device_exclusive_scan(a.cell_count, a.cell_start, a.scan_sums, &a.grid->ncells, a.cell_cap, a.status, s);
-    k_cell_scatter<<<grid_blocks(a.n, 256), 256, 0, s>>>(a);
-    {
-        long long b = (a.cell_cap + 7) / 8;   // 8 warps (cells) per block
-        if (b > 148LL * 8) b = 148LL * 8;
-        k_cell_sort<<<(unsigned)(b < 1 ? 1 : b), 256, 0, s>>>(a);
-    }
-    k_cell_records<<<grid_blocks(a.n, 256) < 148 * 8 ? grid_blocks(a.n, 256) : 148 * 8, 256, 0, s>>>(
-        a, a.search_kind == 3 || a.prm.skin > 0.0 ? 1 : 0);
+    const int wide = grid_blocks(a.n, 256) < 148 * 8 ? grid_blocks(a.n, 256) : 148 * 8;
+    k_cell_keys<<<wide, 256, 0, s>>>(a);
+    k_cell_scan<<<(unsigned)((a.cell_cap + kScanChunk - 1) / kScanChunk), kScanThreads, 0, s>>>(a);
+    k_cell_scatter<<<wide, 256, 0, s>>>(a);
+    // about 8 particles to a lane's warp at the least: a warp per cell of a full body
+    const int ob = grid_blocks((long long)a.n * 2, 256) < 148 * 8 ? grid_blocks((long long)a.n * 2, 256) : 148 * 8;
+    const int with_cposf = a.search_kind == 3 || a.prm.skin > 0.0 ? 1 : 0;
+    if (a.frec0) k_cell_order<kRecMixed><<<ob, 256, 0, s>>>(a, with_cposf);
+    else k_cell_order<kRecFP64><<<ob, 256, 0, s>>>(a, with_cposf);
 }
 
 // ------------------------------------------------------------- re-sorting
@@ -641,12 +665,16 @@ __global__ void k_ghost_emit(StepArgs a) {
             a.gvx[g] = v[0];
             a.gvy[g] = v[1];
             a.gvz[g] = v[2];
+            // the strain gather's records: ghosts keep their unshifted positions
+            const double vol = a.F.f[FMASS][j] / a.F.f[FRHO][j];
+            a.grec0[g] = make_double4(x[0], x[1], x[2], a.F.f[FH][j]);
+            if (a.frec0) a.gfrec1[g] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)vol);
+            else a.grec1[g] = make_double4(v[0], v[1], v[2], vol);
         }
     }
 }
 
 void launch_ghosts(const StepArgs &a, cudaStream_t s) {
-    cudaMemsetAsync(a.gcell, 0, sizeof(int2) * (size_t)a.cell_cap, s);
     k_ghost_count<<<(unsigned)((a.layer_cap + kScanChunk - 1) / kScanChunk), kScanThreads, 0, s>>>(a);
     long long eb = ((long long)a.layer_cap + 7) / 8;   // 8 warps (layer cells) per block
     if (eb > 148LL * 4) eb = 148LL * 4;

@@ -29,7 +29,9 @@ struct StepArgs {
     // key order, each cell in descending reference index, particles outside
     // the grid last); cell_list[p] is its state index.
     int *key;         // per state index: cell key or -1
-    int *cell_count;  // cell_cap
+    int *cell_count;  // cell_cap; zero between steps
+    int *cell_local;  // cell_cap: first position within a chunk of cells
+    int *scan_ticket; // blocks of k_cell_scan that have ended
     int *cell_start;  // cell_cap + 1
     int *cell_list;   // npad: position -> state index
     int *n_inside;    // particles inside the grid (device counter)
@@ -93,7 +95,6 @@ struct StepArgs {
 };
 
 // cells.cu
-void launch_grid_setup(const StepArgs &a, cudaStream_t s);
 void launch_cell_build(const StepArgs &a, cudaStream_t s);
 void launch_ghosts(const StepArgs &a, cudaStream_t s);
 void launch_search(const StepArgs &a, cudaStream_t s);
@@ -118,7 +119,6 @@ void launch_finish_step(const StepArgs &a, cudaStream_t s);
 // step_mixed.cu: FP32 pair sums over FP32 gather records (the constitutive
 // update of the mixed path is the FP64 fast one)
 namespace mixed {
-void launch_strain_prep(const StepArgs &a, cudaStream_t s);
 void launch_strain(const StepArgs &a, cudaStream_t s);
 void launch_mom_prep(const StepArgs &a, cudaStream_t s);
 int launch_momentum(const StepArgs &a, cudaStream_t s, int integrate);
@@ -150,7 +150,6 @@ void launch_reverse_strain(const StepArgs &a, const AdjArgs &b, cudaStream_t s);
 // step kernels (one namespace per arithmetic flavour)
 #define MCM_DECLARE_STEP(NS)                                                        \
     namespace NS {                                                                  \
-    void launch_strain_prep(const StepArgs &a, cudaStream_t s);                     \
     void launch_strain(const StepArgs &a, cudaStream_t s);                          \
     int launch_constitutive(const StepArgs &a, cudaStream_t s);                     \
     void launch_mom_prep(const StepArgs &a, cudaStream_t s);                        \

@@ -173,32 +173,6 @@ __device__ __forceinline__ void store_state(const StepArgs &a, int i, const PSta
     }
 }
 
-// ------------------------------------------------------------ strain prep
-// Gather records for the strain loop: positions shifted back half a step
-// (MCM/mcm_strain.f90:27-31) and V_j = m_j/rho_j (MCM/mcm_oldstrain.f90:44).
-// Ghosts keep their unshifted positions, as in the reference.
-__global__ void k_strain_prep(StepArgs a) {
-    if (skip_step(a)) return;
-    const double dt = a.time->dt;
-    const double *const *f = a.F.f;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x) {
-        const int i = a.cell_list[p];
-        double vx = f[FVX][i], vy = f[FVY][i], vz = f[FVZ][i];
-        double x = f[FX][i] - 0.5 * vx * dt;
-        double y = f[FY][i] - 0.5 * vy * dt;
-        double z = f[FZ][i] - 0.5 * vz * dt;
-        a.rec0[p] = make_double4(x, y, z, f[FH][i]);
-        a.rec1[p] = make_double4(vx, vy, vz, f[FMASS][i] / f[FRHO][i]);
-    }
-    if (a.prm.boundary) {
-        const int ngp = *a.ngp;
-        for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ngp; g += gridDim.x * blockDim.x) {
-            a.grec0[g] = make_double4(a.gx[g], a.gy[g], a.gz[g], a.gh[g]);
-            a.grec1[g] = make_double4(a.gvx[g], a.gvy[g], a.gvz[g], a.gmass[g] / a.grho[g]);
-        }
-    }
-}
-
 __device__ __forceinline__ double block_min(double v, double *sm) {
     for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -228,7 +202,7 @@ __device__ __forceinline__ void update_h(const StepArgs &a, int i, PState<double
 // ---------------------------------------------------- constitutive update
 // MCM/mcm_rhoupd.f90, mcm_constitutive.f90:29-83 and mcm_calccritts.f90 for
 // the particle with state index i, and the forward half-step shift of
-// MCM/mcm_strain.f90:56-60 (x - v dt/2 recomputed exactly as k_strain_prep).
+// MCM/mcm_strain.f90:56-60 (x - v dt/2 recomputed as the strain records have it).
 // Two resident blocks per SM (128 registers, a few hundred bytes of spills)
 // measured faster than one at 154 registers: 0.27 against 0.43 ms per step
 // on the 2M bar.
@@ -712,10 +686,6 @@ static inline int gs_blocks(int n) { int b = nblk(n, 256); return b > 148 * 16 ?
 // that run at the same time fill the chip.
 static int seq_lanes(const StepArgs &a) { return (long long)a.n * a.share < kSeqLanesBelow ? 8 : 1; }
 #endif
-
-void launch_strain_prep(const StepArgs &a, cudaStream_t s) {
-    k_strain_prep<<<gs_blocks(a.n > a.ghost_cap ? a.n : a.ghost_cap), 256, 0, s>>>(a);
-}
 
 void launch_strain(const StepArgs &a, cudaStream_t s) {
 #if MCM_EXACT

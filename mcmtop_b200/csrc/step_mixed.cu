@@ -137,31 +137,6 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float term) {
     s = t;
 }
 
-// ------------------------------------------------------------ strain prep
-// MCM/mcm_strain.f90:27-31 (x - v dt/2) and V_j = m_j/rho_j, cell-relative.
-__global__ void k_strain_prep(StepArgs a) {
-    if (skip_step(a)) return;
-    const double dt = a.time->dt;
-    const Frame fr = make_frame(*a.grid);
-    const double *const *f = a.F.f;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x) {
-        const int i = a.cell_list[p];
-        double o[3];
-        frame_origin(fr, a.ckey[p], o);
-        const double vx = f[FVX][i], vy = f[FVY][i], vz = f[FVZ][i];
-        const double xs = f[FX][i] - 0.5 * vx * dt, ys = f[FY][i] - 0.5 * vy * dt, zs = f[FZ][i] - 0.5 * vz * dt;
-        a.frec0[2 * (size_t)p] = make_float4((float)(xs - o[0]), (float)(ys - o[1]), (float)(zs - o[2]), (float)f[FH][i]);
-        a.frec0[2 * (size_t)p + 1] = make_float4((float)vx, (float)vy, (float)vz, (float)(f[FMASS][i] / f[FRHO][i]));
-    }
-    if (a.prm.boundary) {
-        const int ngp = *a.ngp;
-        for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ngp; g += gridDim.x * blockDim.x) {
-            a.grec0[g] = make_double4(a.gx[g], a.gy[g], a.gz[g], a.gh[g]);
-            a.gfrec1[g] = make_float4((float)a.gvx[g], (float)a.gvy[g], (float)a.gvz[g], (float)(a.gmass[g] / a.grho[g]));
-        }
-    }
-}
-
 // ----------------------------------------------------------- strain rate
 // Neighbours a gather lane loads ahead before it uses the first (strain,
 // momentum), and the momentum gather's resident blocks per SM.
@@ -855,12 +830,6 @@ __global__ void __launch_bounds__(STAGED ? kStageThreads : 256, STAGED ? 4 : MCM
 }
 
 // ------------------------------------------------------------ launchers
-
-void launch_strain_prep(const StepArgs &a, cudaStream_t s) {
-    int n = a.n > a.ghost_cap ? a.n : a.ghost_cap;
-    int b = nblk(n, 256);
-    k_strain_prep<<<b < 148 * 16 ? b : 148 * 16, 256, 0, s>>>(a);
-}
 
 void launch_strain(const StepArgs &a, cudaStream_t s) {
     if (a.pair_kind == 2 && !a.prm.kahan) {
