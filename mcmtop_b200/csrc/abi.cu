@@ -299,7 +299,7 @@ int regrow(mcm_gpu_handle *h, int *grew) {
 }
 
 // ---------------------------------------------------------------- dispatch
-int launch_strain(mcm_gpu_handle *h) {
+void launch_strain(mcm_gpu_handle *h) {
     const int prec = h->cfg.precision;
     {
         Scope sc(h, R_STRAIN, 1);
@@ -308,10 +308,8 @@ int launch_strain(mcm_gpu_handle *h) {
         else fast::launch_strain(h->A, h->stream);
     }
     Scope sc(h, R_CONST, 1);
-    switch (prec) {
-        case MCM_PREC_FP64_EXACT: return exact::launch_constitutive(h->A, h->stream);
-        default: return fast::launch_constitutive(h->A, h->stream);
-    }
+    if (prec == MCM_PREC_FP64_EXACT) exact::launch_constitutive(h->A, h->stream);
+    else fast::launch_constitutive(h->A, h->stream);
 }
 int launch_mom(mcm_gpu_handle *h, int integrate) {
     const int prec = h->cfg.precision;
@@ -375,28 +373,26 @@ void enqueue_part_a(mcm_gpu_handle *h) {
         Scope sc(h, R_SEARCH, 1);
         launch_search(a, h->stream);
     }
-    int nb = launch_strain(h);
-    Scope sc(h, R_CRITTS, 1);
-    launch_critts_reduce(a, h->stream, nb);
+    launch_strain(h);
 }
 
 // momentum -> boundcond -> calctotale (-> update_velocity -> move)
-void enqueue_part_b(mcm_gpu_handle *h, int integrate) {
+void enqueue_part_b(mcm_gpu_handle *h, int integrate, int finish) {
     if (h->A.prm.veloc_opt && integrate) {
         // XSPH needs every updated velocity before any particle moves
         int nb = launch_mom(h, 0);
         {
-            Scope sc(h, R_REDUCE, 2);
+            Scope sc(h, R_REDUCE, 1);
             launch_energy_bbox_reduce(h->A, h->stream, nb, 1, 0);
         }
         nb = launch_move(h);
         Scope sc(h, R_REDUCE, 1);
-        launch_energy_bbox_reduce(h->A, h->stream, nb, 0, 1);
+        launch_energy_bbox_reduce(h->A, h->stream, nb, 0, 1, finish);
         return;
     }
     int nb = launch_mom(h, integrate);
-    Scope sc(h, R_REDUCE, 2);
-    launch_energy_bbox_reduce(h->A, h->stream, nb, 1, integrate);
+    Scope sc(h, R_REDUCE, 1);
+    launch_energy_bbox_reduce(h->A, h->stream, nb, 1, integrate, finish);
 }
 
 int check_handle(mcm_gpu_handle *h) {
@@ -723,6 +719,9 @@ int mcm_gpu_create(const mcm_gpu_config *cfg, const mcm_gpu_material *mats, int 
     h->A.hmax = (double *)p; p += 32;
     h->A.skin_d2 = (unsigned long long *)p; p += 32;
     h->A.skin_flags = (int *)p; p += 32;
+    h->A.crit_bits = (unsigned long long *)p;
+    h->A.crit_ticket = (int *)(p + 8);
+    h->A.reduce_ticket = (int *)(p + 12); p += 32;
     h->A.energy = (double *)p;
     cudaMallocHost((void **)&h->h_time, 4096);
     char *q = (char *)h->h_time;
@@ -1109,9 +1108,7 @@ int mcm_gpu_run(mcm_gpu_handle *h, int nsteps, mcm_gpu_time *t, int *done) {
         if ((st = reset_status(h))) return st;
         for (int k = 0; k < batch; ++k) {
             enqueue_part_a(h);
-            enqueue_part_b(h, 1);
-            Scope sc(h, R_MISC, 1);
-            launch_finish_step(h->A, h->stream);
+            enqueue_part_b(h, 1, 1);
         }
         if ((st = sync_status(h))) return st;
         int ran = h->h_time->steps_done;

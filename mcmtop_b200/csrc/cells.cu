@@ -14,6 +14,7 @@
 // and the predicate d^2 < (h_i+h_j)^2 are evaluated exactly as the reference
 // does in FP64, so borderline pairs resolve identically.
 #include "nbr_iter.cuh"
+#include "time_step.cuh"
 
 namespace mcm {
 
@@ -97,6 +98,8 @@ __global__ void __launch_bounds__(256) k_cell_keys(StepArgs a) {
             *a.n_inside = 0;
             *a.scan_ticket = 0;
             *a.ghost_ticket = 0;
+            *a.crit_ticket = 0;
+            *a.crit_bits = order_bits((unsigned long long)__double_as_longlong(1.0e20));
         }
     }
     __syncthreads();

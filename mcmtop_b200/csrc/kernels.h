@@ -82,6 +82,8 @@ struct StepArgs {
     float4 *frec0;                   // mixed path: 4 npad float4 (strain or momentum records)
     float4 *gfrec1, *gfrec2;         // mixed path, per ghost
     // reductions
+    unsigned long long *crit_bits;   // bits of the step's critical timestep so far
+    int *crit_ticket, *reduce_ticket;   // blocks of the constitutive and reduction kernels that have ended
     double *red;      // block partials
     int red_blocks;   // capacity of red in blocks (partial vectors)
     // launch shape, chosen by mcm_gpu_set_tuning or mcm_gpu_autotune (0: default)
@@ -106,15 +108,13 @@ constexpr int kReorderLaunches = (NFIELD + kReorderGroup - 1) / kReorderGroup + 
 void launch_reorder(const StepArgs &a, cudaStream_t s);
 
 // reduce.cu
-void launch_critts_reduce(const StepArgs &a, cudaStream_t s, int nblocks);
 void launch_init_critts_reduce(const StepArgs &a, cudaStream_t s, int nblocks);
-void launch_energy_bbox_reduce(const StepArgs &a, cudaStream_t s, int nblocks, int energy, int bbox);
+void launch_energy_bbox_reduce(const StepArgs &a, cudaStream_t s, int nblocks, int energy, int bbox, int finish = 0);
 void launch_set_time(const StepArgs &a, cudaStream_t s, double dt, double dtold, int set_dtold);
 // energy partials of several materials in the rows of the momentum kernel's nblocks blocks
 void launch_energy_step_partials(const StepArgs &a, cudaStream_t s, int nblocks);
 // per-material sums of mass x repulsion into out[3*nmat] (device memory)
 void launch_contact_forces(const StepArgs &a, cudaStream_t s, double *out);
-void launch_finish_step(const StepArgs &a, cudaStream_t s);
 
 // step_mixed.cu: FP32 pair sums over FP32 gather records (the constitutive
 // update of the mixed path is the FP64 fast one)
@@ -151,7 +151,7 @@ void launch_reverse_strain(const StepArgs &a, const AdjArgs &b, cudaStream_t s);
 #define MCM_DECLARE_STEP(NS)                                                        \
     namespace NS {                                                                  \
     void launch_strain(const StepArgs &a, cudaStream_t s);                          \
-    int launch_constitutive(const StepArgs &a, cudaStream_t s);                     \
+    void launch_constitutive(const StepArgs &a, cudaStream_t s);                     \
     void launch_mom_prep(const StepArgs &a, cudaStream_t s);                        \
     void launch_rep_cont(const StepArgs &a, cudaStream_t s);                        \
     int launch_momentum(const StepArgs &a, cudaStream_t s, int integrate);          \

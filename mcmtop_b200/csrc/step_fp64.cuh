@@ -12,6 +12,7 @@
 #pragma once
 #include "nbr_iter.cuh"
 #include "physics.cuh"
+#include "time_step.cuh"
 
 #ifndef MCM_FLAVOUR_NS
 #error "define MCM_FLAVOUR_NS (exact or fast)"
@@ -212,11 +213,10 @@ __device__ __forceinline__ void update_h(const StepArgs &a, int i, PState<double
 __global__ void __launch_bounds__(kRedThreads, MCM_CONST_MINBLOCKS) k_constitutive(StepArgs a) {
     __shared__ double sm[32];
     if (skip_step(a)) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const double dt = a.time->dt;
     double crit = 1.0e20;
-    int bad = 0;
-    if (i < a.n) {
+#pragma unroll 1
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
         double *const *f = a.F.f;
         const DevMaterial &M = a.mats[a.F.mat[i] - 1];
         PState<double> P;
@@ -229,12 +229,14 @@ __global__ void __launch_bounds__(kRedThreads, MCM_CONST_MINBLOCKS) k_constituti
         P.tracerod = f[FTR][i];
         if (a.prm.h_opt) update_h(a, i, P, dt);
         rhoupd(P, M, dt, 3);
-        bad = constitutive_particle(P, M, dt);
+        const int bad = constitutive_particle(P, M, dt);
+        if (bad) raise_status(a.status, bad, i);
         const double vx = f[FVX][i], vy = f[FVY][i], vz = f[FVZ][i];
         const double mindist = (a.prm.tcrit_opt == 2) ? f[FMINDIST][i] : 0.0;
-        crit = critts_particle(P, M, a.prm.tcrit_opt, 3, f[FVABS][i], mindist);
+        const double own = critts_particle(P, M, a.prm.tcrit_opt, 3, f[FVABS][i], mindist);
+        crit = fmin(crit, own);
         store_state(a, i, P, M.model);
-        if (a.prm.diag) f[FCRITTS][i] = crit;
+        if (a.prm.diag) f[FCRITTS][i] = own;
         const double xs = f[FX][i] - 0.5 * vx * dt;
         const double ys = f[FY][i] - 0.5 * vy * dt;
         const double zs = f[FZ][i] - 0.5 * vz * dt;
@@ -242,9 +244,8 @@ __global__ void __launch_bounds__(kRedThreads, MCM_CONST_MINBLOCKS) k_constituti
         f[FY][i] = ys + 0.5 * vy * dt;
         f[FZ][i] = zs + 0.5 * vz * dt;
     }
-    if (bad) raise_status(a.status, bad, i);
     double m = block_min(crit, sm);
-    if (threadIdx.x == 0) a.red[blockIdx.x] = m;
+    if (threadIdx.x == 0) finish_critts(a, m);
 }
 
 // ------------------------------------------------------ repulsive contact
@@ -701,10 +702,11 @@ void launch_strain(const StepArgs &a, cudaStream_t s) {
 #endif
 }
 
-int launch_constitutive(const StepArgs &a, cudaStream_t s) {
+void launch_constitutive(const StepArgs &a, cudaStream_t s) {
     int blocks = nblk(a.n, kRedThreads);
+    const int wave = 148 * resident_per_sm((const void *)k_constitutive, kRedThreads);
+    if (blocks > wave) blocks = wave;
     k_constitutive<<<blocks, kRedThreads, 0, s>>>(a);
-    return blocks;
 }
 
 void launch_mom_prep(const StepArgs &a, cudaStream_t s) {
