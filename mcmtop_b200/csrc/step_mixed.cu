@@ -42,7 +42,14 @@ __device__ __forceinline__ bool skip_step(const StepArgs &a) { return a.status->
 // Sum of one value per lane over the L lanes of a sub-warp, every addition
 // error-free transformed (TwoSum) and the errors added up; every lane gets it.
 // c: a correction the lane already carries (the compensation of a Kahan sum).
-__device__ __forceinline__ double lane_sum(float s, float c = 0.0f) {
+__device__ __forceinline__ double lane_sum(float s) {
+    static_assert(L == 2, "one exchange");
+    const float s2 = __shfl_xor_sync(0xffffffffu, s, 1, L);
+    const float t = s + s2;
+    const float bp = t - s;
+    return (double)t + (double)((s - (t - bp)) + (s2 - bp));
+}
+__device__ __forceinline__ double lane_sum(float s, float c) {
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) {
         const float s2 = __shfl_xor_sync(0xffffffffu, s, o, L);
@@ -79,13 +86,35 @@ __device__ __forceinline__ void frame_origin(const Frame &fr, int key, double o[
     for (int d = 0; d < 3; ++d) o[d] = fr.gmin[d] + (double)(b[d] - 1) * fr.cs[d];
 }
 
+#ifndef MCM_STRAIN_UNROLL
+#define MCM_STRAIN_UNROLL 4
+#endif
+#ifndef MCM_MOM_UNROLL
+#define MCM_MOM_UNROLL 1
+#endif
+#ifndef MCM_MOM_MINBLOCKS
+#define MCM_MOM_MINBLOCKS 4
+#endif
 // Offsets of the 27 neighbour cells (cell size times -1, 0, 1 per axis), by code.
-__device__ __forceinline__ void fill_offsets(float4 *tab, const Frame &fr) {
-    if (threadIdx.x < 27) {
-        const int c = threadIdx.x;
-        tab[c] = make_float4((float)(c % 3 - 1) * fr.csf[0], (float)((c / 3) % 3 - 1) * fr.csf[1],
-                             (float)(c / 9 - 1) * fr.csf[2], 0.0f);
-    }
+// The strain gather reads them as one 16-byte word, the momentum gather, whose
+// records already fill the shared-memory path, as three words that never meet
+// in a bank (685 824-particle bar: strain 228 us with the one and 236 with the
+// other, momentum 308 and 301).
+struct Offsets4 {
+    float4 v[27];
+    __device__ __forceinline__ float4 operator[](unsigned c) const { return v[c]; }
+    __device__ __forceinline__ void set(int c, float x, float y, float z) { v[c] = make_float4(x, y, z, 0.0f); }
+};
+struct Offsets3 {
+    float x[32], y[32], z[32];
+    __device__ __forceinline__ float4 operator[](unsigned c) const { return make_float4(x[c], y[c], z[c], 0.0f); }
+    __device__ __forceinline__ void set(int c, float u, float v, float w) { x[c] = u; y[c] = v; z[c] = w; }
+};
+template <typename T>
+__device__ __forceinline__ void fill_offsets(T &tab, const Frame &fr) {
+    const int c = threadIdx.x;
+    if (c < 27)
+        tab.set(c, (float)(c % 3 - 1) * fr.csf[0], (float)((c / 3) % 3 - 1) * fr.csf[1], (float)(c / 9 - 1) * fr.csf[2]);
 }
 
 // Gather records.  A strain record is 32 bytes {x, y, z, h, vx, vy, vz, V}
@@ -105,23 +134,34 @@ __device__ __forceinline__ Rec8 ld_rec8(const float4 *p) {
 }
 __device__ __forceinline__ float4 ld_rec4(const float4 *p) { return __ldg(p); }
 
-// Cubic B-spline gradient in FP32 (MCM/mcm_gradw.f90:64-101), ih = 1/havg.
-__device__ __forceinline__ void gradw_f(float x0, float x1, float x2, float ih, float &d0, float &d1, float &d2) {
-    const float r2 = fmaf(x0, x0, fmaf(x1, x1, x2 * x2));
-    if (r2 == 0.0f) { d0 = d1 = d2 = 0.0f; return; }
-    const float rinv = rsqrtf(r2);
-    const float z = r2 * rinv * ih;
-    const float const1 = (1.0f / kPiF) * ih * ih * ih;
-    float dw;
-    if (z < 1.0f) dw = const1 * ((2.25f * z - 3.0f) * z);
-    else if (z < 2.0f) { const float tt = 2.0f - z; dw = -0.75f * const1 * (tt * tt); }
-    else dw = 0.0f;
-    const float f = dw * ih * rinv;
-    d0 = f * x0; d1 = f * x1; d2 = f * x2;
+// A particle's own h and what every pair of one h has in common:
+// ih = 1/h and c3 = 1/(pi h^3).
+struct OwnH {
+    float h, ih, c3;
+};
+__device__ __forceinline__ OwnH own_h(float h) {
+    const float ih = 1.0f / h;
+    return {h, ih, (1.0f / kPiF) * ih * ih * ih};
 }
 
-__device__ __forceinline__ float inv_havg_f(float hi, float hj, float ihi) {
-    return (hi == hj) ? ihi : 2.0f / (hi + hj);
+// f with grad W = f (x_i - x_j): the cubic B-spline gradient in FP32
+// (MCM/mcm_gradw.f90:64-101).  No branches on the distance: coincident
+// particles get a finite f (the caller multiplies it by a zero difference), and
+// beyond 2h the spline's argument is held at its end, where it is zero.
+__device__ __forceinline__ float gradw_f(float x0, float x1, float x2, const OwnH &o, float hj) {
+    float ih = o.ih, c3 = o.c3;
+    if (hj != o.h) {
+        ih = 2.0f / (o.h + hj);
+        c3 = (1.0f / kPiF) * ih * ih * ih;
+    }
+    const float r2 = fmaxf(fmaf(x0, x0, fmaf(x1, x1, x2 * x2)), 1.0e-36f);
+    float rinv;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rinv) : "f"(r2));
+    const float q = rinv * ih;
+    const float z = r2 * q;
+    const float t = fmaxf(2.0f - z, 0.0f);
+    const float dw = z < 1.0f ? (2.25f * z - 3.0f) * z : -0.75f * (t * t);
+    return dw * c3 * q;
 }
 
 static inline int nblk(int n, int t) { return (n + t - 1) / t; }
@@ -140,15 +180,6 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float term) {
 // ----------------------------------------------------------- strain rate
 // Neighbours a gather lane loads ahead before it uses the first (strain,
 // momentum), and the momentum gather's resident blocks per SM.
-#ifndef MCM_STRAIN_UNROLL
-#define MCM_STRAIN_UNROLL 4
-#endif
-#ifndef MCM_MOM_UNROLL
-#define MCM_MOM_UNROLL 1
-#endif
-#ifndef MCM_MOM_MINBLOCKS
-#define MCM_MOM_MINBLOCKS 4
-#endif
 constexpr int kUnroll = MCM_STRAIN_UNROLL;
 
 // The list entries base[0 .. 2U) of one particle's two lanes, lane l getting
@@ -178,10 +209,10 @@ __device__ __forceinline__ void pair_entries(const unsigned *base, int lane, uns
 // One pair's terms of MCM/mcm_oldstrain.f90:42-53: V_j (v_j - v_i)_n dW/dx_m
 // added to gv[3n + m] (KAHAN: compensated, the low parts in gc).
 template <bool KAHAN>
-__device__ __forceinline__ void strain_term(float dx, float dy, float dz, float hj, float4 vj, float hi, float ihi,
-                                            float4 vi, float (&gv)[9], float (&gc)[9]) {
-    float d0, d1, d2;
-    gradw_f(dx, dy, dz, inv_havg_f(hi, hj, ihi), d0, d1, d2);
+__device__ __forceinline__ void strain_term(float dx, float dy, float dz, float hj, float4 vj, const OwnH &o, float4 vi,
+                                            float (&gv)[9], float (&gc)[9]) {
+    const float f = gradw_f(dx, dy, dz, o, hj);
+    const float d0 = f * dx, d1 = f * dy, d2 = f * dz;
     const float t0 = vj.w * (vj.x - vi.x), t1 = vj.w * (vj.y - vi.y), t2 = vj.w * (vj.z - vi.z);
     if (KAHAN) {
         const float tt[3] = {t0, t1, t2}, dd[3] = {d0, d1, d2};
@@ -196,11 +227,22 @@ __device__ __forceinline__ void strain_term(float dx, float dy, float dz, float 
     }
 }
 
+// MCM/mcm_oldstrain.f90:56-63: rod, spin and trace of particle i, which lie in
+// ten consecutive fields; each of the two lanes stores five of them.
+__device__ __forceinline__ void store_rates(const StepArgs &a, int i, int lane, const double (&r)[9]) {
+    static_assert(FTR == FR11 + 9 && FW12 == FR11 + 6, "rod, spin and trace in a row");
+    const double v[10] = {r[0], r[4], r[8], 0.5 * (r[1] + r[3]), 0.5 * (r[2] + r[6]), 0.5 * (r[5] + r[7]),
+                          0.5 * (r[1] - r[3]), 0.5 * (r[2] - r[6]), 0.5 * (r[5] - r[7]), r[0] + r[4] + r[8]};
+    double *f = a.F.f[FR11] + (size_t)(5 * lane) * a.npad + i;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) f[(size_t)q * a.npad] = lane ? v[5 + q] : v[q];
+}
+
 // MCM/mcm_oldstrain.f90:34-64 with FP32 pair sums (KAHAN: compensated per
 // lane, the compensation carried into the TwoSum lane combination).
 template <bool KAHAN>
 __global__ void __launch_bounds__(256, 3) k_strain(StepArgs a) {
-    __shared__ float4 offs[27];
+    __shared__ Offsets4 offs;
     if (skip_step(a)) return;
     const int sub = threadIdx.x / L, lane = threadIdx.x % L;
     const int per = blockDim.x / L;
@@ -231,7 +273,7 @@ __global__ void __launch_bounds__(256, 3) k_strain(StepArgs a) {
             xs[2] = a.F.f[FZ][i] - 0.5 * a.F.f[FVZ][i] * dt;
         }
         const int total = live ? nreal + gn : 0;
-        const float ihi = 1.0f / xi.w;
+        const OwnH own = own_h(xi.w);
         float gv[9], gc[9];
 #pragma unroll
         for (int u = 0; u < 9; ++u) { gv[u] = 0.0f; gc[u] = 0.0f; }
@@ -249,39 +291,26 @@ __global__ void __launch_bounds__(256, 3) k_strain(StepArgs a) {
             for (int u = 0; u < kUnroll; ++u) {
                 const float4 o = offs[e[u] >> 26];
                 strain_term<KAHAN>((xi.x - r[u].a.x) - o.x, (xi.y - r[u].a.y) - o.y, (xi.z - r[u].a.z) - o.z,
-                                   r[u].a.w, r[u].b, xi.w, ihi, vi, gv, gc);
+                                   r[u].a.w, r[u].b, own, vi, gv, gc);
             }
         }
         for (; k < nreal; k += L) {
             const unsigned e = spos[k];
             const float4 o = offs[e >> 26];
             const Rec8 r = ld_rec8(a.frec0 + 2 * (size_t)(e & kPosMask));
-            strain_term<KAHAN>((xi.x - r.a.x) - o.x, (xi.y - r.a.y) - o.y, (xi.z - r.a.z) - o.z, r.a.w, r.b, xi.w,
-                               ihi, vi, gv, gc);
+            strain_term<KAHAN>((xi.x - r.a.x) - o.x, (xi.y - r.a.y) - o.y, (xi.z - r.a.z) - o.z, r.a.w, r.b, own,
+                               vi, gv, gc);
         }
         for (; k < total; k += L) {
             const int q = a.gnbr[(size_t)(k - nreal) * a.npad + t];
             const double4 xj = a.grec0[q];
             strain_term<KAHAN>((float)(xs[0] - xj.x), (float)(xs[1] - xj.y), (float)(xs[2] - xj.z), (float)xj.w,
-                               a.gfrec1[q], xi.w, ihi, vi, gv, gc);
+                               a.gfrec1[q], own, vi, gv, gc);
         }
         double r[9];
 #pragma unroll
-        for (int u = 0; u < 9; ++u) r[u] = lane_sum(gv[u], KAHAN ? gc[u] : 0.0f);
-        if (live && lane == 0) {
-            // MCM/mcm_oldstrain.f90:56-63
-            double *const *f = a.F.f;
-            f[FR11][i] = r[0];
-            f[FR22][i] = r[4];
-            f[FR33][i] = r[8];
-            f[FR12][i] = 0.5 * (r[1] + r[3]);
-            f[FR13][i] = 0.5 * (r[2] + r[6]);
-            f[FR23][i] = 0.5 * (r[5] + r[7]);
-            f[FW12][i] = 0.5 * (r[1] - r[3]);
-            f[FW13][i] = 0.5 * (r[2] - r[6]);
-            f[FW23][i] = 0.5 * (r[5] - r[7]);
-            f[FTR][i] = r[0] + r[4] + r[8];
-        }
+        for (int u = 0; u < 9; ++u) r[u] = KAHAN ? lane_sum(gv[u], gc[u]) : lane_sum(gv[u]);
+        if (live) store_rates(a, i, lane, r);
         __syncwarp();
     }
 }
@@ -380,7 +409,7 @@ __device__ __forceinline__ int stage_index(const StageWin &W, int wbase, unsigne
 }
 
 __global__ void __launch_bounds__(kStageThreads, 6) k_strain_staged(StepArgs a) {
-    __shared__ float4 offs[27];
+    __shared__ Offsets4 offs;
     __shared__ float4 stage[2 * kStageCap];
     __shared__ StageWin W;
     if (skip_step(a)) return;
@@ -415,7 +444,7 @@ __global__ void __launch_bounds__(kStageThreads, 6) k_strain_staged(StepArgs a) 
             xs[2] = a.F.f[FZ][i] - 0.5 * a.F.f[FVZ][i] * dt;
         }
         const int total = live ? nreal + gn : 0;
-        const float ihi = 1.0f / xi.w;
+        const OwnH own = own_h(xi.w);
         float gv[9];
 #pragma unroll
         for (int u = 0; u < 9; ++u) gv[u] = 0.0f;
@@ -448,8 +477,8 @@ __global__ void __launch_bounds__(kStageThreads, 6) k_strain_staged(StepArgs a) 
                 dz = (float)(xs[2] - xj.z);
                 hj = (float)xj.w;
             }
-            float d0, d1, d2;
-            gradw_f(dx, dy, dz, inv_havg_f(xi.w, hj, ihi), d0, d1, d2);
+            const float f = gradw_f(dx, dy, dz, own, hj);
+            const float d0 = f * dx, d1 = f * dy, d2 = f * dz;
             const float t0 = vj.w * (vj.x - vi.x), t1 = vj.w * (vj.y - vi.y), t2 = vj.w * (vj.z - vi.z);
             gv[0] = fmaf(t0, d0, gv[0]); gv[1] = fmaf(t0, d1, gv[1]); gv[2] = fmaf(t0, d2, gv[2]);
             gv[3] = fmaf(t1, d0, gv[3]); gv[4] = fmaf(t1, d1, gv[4]); gv[5] = fmaf(t1, d2, gv[5]);
@@ -458,19 +487,7 @@ __global__ void __launch_bounds__(kStageThreads, 6) k_strain_staged(StepArgs a) 
         double r[9];
 #pragma unroll
         for (int u = 0; u < 9; ++u) r[u] = lane_sum(gv[u]);
-        if (live && lane == 0) {
-            double *const *f = a.F.f;
-            f[FR11][i] = r[0];
-            f[FR22][i] = r[4];
-            f[FR33][i] = r[8];
-            f[FR12][i] = 0.5 * (r[1] + r[3]);
-            f[FR13][i] = 0.5 * (r[2] + r[6]);
-            f[FR23][i] = 0.5 * (r[5] + r[7]);
-            f[FW12][i] = 0.5 * (r[1] - r[3]);
-            f[FW13][i] = 0.5 * (r[2] - r[6]);
-            f[FW23][i] = 0.5 * (r[5] - r[7]);
-            f[FTR][i] = r[0] + r[4] + r[8];
-        }
+        if (live) store_rates(a, i, lane, r);
         __syncthreads();   // the next round overwrites the windows
     }
 }
@@ -606,14 +623,13 @@ constexpr int kUnrollM = MCM_MOM_UNROLL;
 // a(n) += m_j sum_m (A_j + A_i)(m, n) dW/dx_m, A = (sigma - q I)/rho^2 packed
 // as r1 = (11 22 33 12), r2 = (13 23 m_j -).
 template <bool KAHAN>
-__device__ __forceinline__ void momentum_term(float dx, float dy, float dz, float hj, float4 r1, float4 r2, float hi,
-                                              float ihi, float4 r1i, float4 r2i, float (&acc)[3], float (&comp)[3]) {
-    float d0, d1, d2;
-    gradw_f(dx, dy, dz, inv_havg_f(hi, hj, ihi), d0, d1, d2);
+__device__ __forceinline__ void momentum_term(float dx, float dy, float dz, float hj, float4 r1, float4 r2,
+                                              const OwnH &o, float4 r1i, float4 r2i, float (&acc)[3],
+                                              float (&comp)[3]) {
+    const float f = gradw_f(dx, dy, dz, o, hj) * r2.z;
+    const float d0 = f * dx, d1 = f * dy, d2 = f * dz;
     const float s11 = r1.x + r1i.x, s22 = r1.y + r1i.y, s33 = r1.z + r1i.z;
     const float s12 = r1.w + r1i.w, s13 = r2.x + r2i.x, s23 = r2.y + r2i.y;
-    const float mj = r2.z;
-    d0 *= mj; d1 *= mj; d2 *= mj;
     if (KAHAN) {
         kahan_add(acc[0], comp[0], fmaf(s11, d0, fmaf(s12, d1, s13 * d2)));
         kahan_add(acc[1], comp[1], fmaf(s12, d0, fmaf(s22, d1, s23 * d2)));
@@ -628,7 +644,7 @@ __device__ __forceinline__ void momentum_term(float dx, float dy, float dz, floa
 template <bool ASYM, bool KAHAN, bool STAGED>
 __global__ void __launch_bounds__(STAGED ? kStageThreads : 256, STAGED ? 4 : MCM_MOM_MINBLOCKS) k_momentum(StepArgs a, int integrate_flag) {
     __shared__ double sm[32];
-    __shared__ float4 offs[27];
+    __shared__ Offsets3 offs;
     __shared__ float4 stage[STAGED ? 3 * kStageCapM : 1];
     __shared__ StageWin W;
     if (skip_step(a)) return;
@@ -667,7 +683,7 @@ __global__ void __launch_bounds__(STAGED ? kStageThreads : 256, STAGED ? 4 : MCM
         double xa[3] = {0.0, 0.0, 0.0};
         if (live && gn > 0) { xa[0] = a.F.f[FX][i]; xa[1] = a.F.f[FY][i]; xa[2] = a.F.f[FZ][i]; }
         const int total = live ? nreal + gn : 0;
-        const float ihi = 1.0f / xi.w;
+        const OwnH own = own_h(xi.w);
         float acc[3] = {0.0f, 0.0f, 0.0f}, comp[3] = {0.0f, 0.0f, 0.0f};
         int k0 = lane;
         if (!STAGED && !asym) {
@@ -684,7 +700,7 @@ __global__ void __launch_bounds__(STAGED ? kStageThreads : 256, STAGED ? 4 : MCM
                     const Rec8 r = ld_rec8(a.frec0 + 2 * p);
                     const float4 q2 = ld_rec4(mom_tail(a) + p);
                     momentum_term<KAHAN>((xi.x - r.a.x) - o.x, (xi.y - r.a.y) - o.y, (xi.z - r.a.z) - o.z, r.a.w,
-                                         r.b, q2, xi.w, ihi, r1i, r2i, acc, comp);
+                                         r.b, q2, own, r1i, r2i, acc, comp);
                     e[0] = e[1];
                     e[1] = e[2];
                     e[2] = e[3];
@@ -707,7 +723,7 @@ __global__ void __launch_bounds__(STAGED ? kStageThreads : 256, STAGED ? 4 : MCM
                 for (int u = 0; u < kUnrollM; ++u) {
                     const float4 o = offs[e[u] >> 26];
                     momentum_term<KAHAN>((xi.x - r[u].a.x) - o.x, (xi.y - r[u].a.y) - o.y, (xi.z - r[u].a.z) - o.z,
-                                         r[u].a.w, r[u].b, q2[u], xi.w, ihi, r1i, r2i, acc, comp);
+                                         r[u].a.w, r[u].b, q2[u], own, r1i, r2i, acc, comp);
                 }
             }
         }
@@ -749,14 +765,12 @@ __global__ void __launch_bounds__(STAGED ? kStageThreads : 256, STAGED ? 4 : MCM
                 dz = (float)(xa[2] - xj.z);
                 hj = (float)xj.w;
             }
-            float d0, d1, d2;
-            gradw_f(dx, dy, dz, inv_havg_f(xi.w, hj, ihi), d0, d1, d2);
+            const float f = gradw_f(dx, dy, dz, own, hj) * r2.z;
+            const float d0 = f * dx, d1 = f * dy, d2 = f * dz;
             const float s11 = r1.x + r1i.x, s22 = r1.y + r1i.y, s33 = r1.z + r1i.z;
             const float s12 = r1.w + r1i.w, s13 = r2.x + r2i.x, s23 = r2.y + r2i.y;
             float l21 = s12, l31 = s13, l32 = s23;
             if (asym) { l21 = r3.x + r3i.x; l31 = r3.y + r3i.y; l32 = r3.z + r3i.z; }
-            const float mj = r2.z;
-            d0 *= mj; d1 *= mj; d2 *= mj;
             // a(n) += m_j sum_m (A_j + A_i)(m,n) dW/dx_m (column n; rows for a symmetric A)
             if (KAHAN) {
                 kahan_add(acc[0], comp[0], fmaf(s11, d0, fmaf(l21, d1, l31 * d2)));
@@ -770,7 +784,7 @@ __global__ void __launch_bounds__(STAGED ? kStageThreads : 256, STAGED ? 4 : MCM
         }
         double ac[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) ac[c] = lane_sum(acc[c], KAHAN ? comp[c] : 0.0f);
+        for (int c = 0; c < 3; ++c) ac[c] = KAHAN ? lane_sum(acc[c], comp[c]) : lane_sum(acc[c]);
         if (live && lane == 0) {
             double *const *f = a.F.f;
             if (a.prm.contact)   // repulsive contact (MCM/mcm_oldacceleration.f90:49-51)
