@@ -84,6 +84,7 @@ __device__ __forceinline__ bool make_grid(const StepArgs &a, DevGrid &g) {
 // get none) and the cells' counts.  cell_count is zero on entry: the scatter
 // takes every count down to zero again.
 __global__ void __launch_bounds__(256) k_cell_keys(StepArgs a) {
+    chain_start();
     __shared__ DevGrid g;
     __shared__ int stop;
     if (a.status->code) return;
@@ -167,6 +168,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *smem, int &total
 
 
 __global__ void __launch_bounds__(kScanThreads) k_cell_scan(StepArgs a) {
+    chain_start();
     __shared__ int smem[32];
     __shared__ int last;
     if (a.status->code) return;
@@ -212,6 +214,7 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(StepArgs a) {
 // outside the grid (llpointer = -1 in the reference) take the positions after
 // the last cell; they have no neighbours and are never one.
 __global__ void __launch_bounds__(256) k_cell_scatter(StepArgs a) {
+    chain_start();
     if (a.status->code) return;
     const int ncells = (int)a.grid->ncells;
     const int base_out = a.scan_sums[(ncells + kScanChunk - 1) / kScanChunk];
@@ -301,6 +304,7 @@ __device__ __forceinline__ void write_records(const StepArgs &a, const DevGrid &
 constexpr int kSortPer = 4;
 template <int REC>
 __global__ void __launch_bounds__(256) k_cell_order(StepArgs a, int with_cposf) {
+    chain_start();
     __shared__ DevGrid g;
     __shared__ unsigned long long smax[8], smin[8];
     if (a.status->code) return;
@@ -406,14 +410,14 @@ static int grid_blocks(long long work, int threads) {
 // the cells with everything that is written per particle in cell order.
 void launch_cell_build(const StepArgs &a, cudaStream_t s) {
     const int wide = grid_blocks(a.n, 256) < 148 * 8 ? grid_blocks(a.n, 256) : 148 * 8;
-    k_cell_keys<<<wide, 256, 0, s>>>(a);
-    k_cell_scan<<<(unsigned)((a.cell_cap + kScanChunk - 1) / kScanChunk), kScanThreads, 0, s>>>(a);
-    k_cell_scatter<<<wide, 256, 0, s>>>(a);
+    launch_chained(k_cell_keys, wide, 256, 0, s, a);
+    launch_chained(k_cell_scan, (unsigned)((a.cell_cap + kScanChunk - 1) / kScanChunk), kScanThreads, 0, s, a);
+    launch_chained(k_cell_scatter, wide, 256, 0, s, a);
     // about 8 particles to a lane's warp at the least: a warp per cell of a full body
     const int ob = grid_blocks((long long)a.n * 2, 256) < 148 * 8 ? grid_blocks((long long)a.n * 2, 256) : 148 * 8;
     const int with_cposf = a.search_kind == 3 || a.prm.skin > 0.0 ? 1 : 0;
-    if (a.frec0) k_cell_order<kRecMixed><<<ob, 256, 0, s>>>(a, with_cposf);
-    else k_cell_order<kRecFP64><<<ob, 256, 0, s>>>(a, with_cposf);
+    if (a.frec0) launch_chained(k_cell_order<kRecMixed>, ob, 256, 0, s, a, with_cposf);
+    else launch_chained(k_cell_order<kRecFP64>, ob, 256, 0, s, a, with_cposf);
 }
 
 // ------------------------------------------------------------- re-sorting
@@ -558,6 +562,7 @@ __device__ __forceinline__ Origin origin_of(const StepArgs &a, const Layers &l, 
 // Counts of the layer cells and their prefix sums: within a chunk in
 // layer_off, over the chunks in layer_sums (by the block that ends last).
 __global__ void __launch_bounds__(kScanThreads) k_ghost_count(StepArgs a) {
+    chain_start();
     __shared__ int smem[32];
     __shared__ int last;
     if (a.status->code && a.status->code != MCM_EGHOST_LAYER) return;   // EGHOST_LAYER may be this launch's own
@@ -621,6 +626,7 @@ __global__ void __launch_bounds__(kScanThreads) k_ghost_count(StepArgs a) {
 
 // One warp per layer cell, its lanes over the cell's ghosts.
 __global__ void k_ghost_emit(StepArgs a) {
+    chain_start();
     if (a.status->code) return;
     const Layers l = make_layers(a);
     const int T = l.first[6];
@@ -678,10 +684,10 @@ __global__ void k_ghost_emit(StepArgs a) {
 }
 
 void launch_ghosts(const StepArgs &a, cudaStream_t s) {
-    k_ghost_count<<<(unsigned)((a.layer_cap + kScanChunk - 1) / kScanChunk), kScanThreads, 0, s>>>(a);
+    launch_chained(k_ghost_count, (unsigned)((a.layer_cap + kScanChunk - 1) / kScanChunk), kScanThreads, 0, s, a);
     long long eb = ((long long)a.layer_cap + 7) / 8;   // 8 warps (layer cells) per block
     if (eb > 148LL * 4) eb = 148LL * 4;
-    k_ghost_emit<<<(unsigned)(eb < 1 ? 1 : eb), 256, 0, s>>>(a);
+    launch_chained(k_ghost_emit, (unsigned)(eb < 1 ? 1 : eb), 256, 0, s, a);
 }
 
 // ------------------------------------------------------------------ search
@@ -796,10 +802,10 @@ __device__ __forceinline__ unsigned group_bits(const StepArgs &a, int g0, int m,
     for (int j = 0; j < turns; ++j) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-            const float4 x = __ldg(X + 2 * j + u), y = __ldg(Y + 2 * j + u), z = __ldg(Z + 2 * j + u);
+            const float4 x = X[2 * j + u], y = Y[2 * j + u], z = Z[2 * j + u];
             float2 t0 = thr, t1 = thr;
             if (!UNI) {
-                const float4 h = __ldg(H + 2 * j + u);
+                const float4 h = H[2 * j + u];
                 const float2 h0 = __fadd2_rn(hi2, make_float2(h.x, h.y)), h1 = __fadd2_rn(hi2, make_float2(h.z, h.w));
                 t0 = __ffma2_rn(__fmul2_rn(h0, rel), h0, band);
                 t1 = __ffma2_rn(__fmul2_rn(h1, rel), h1, band);
@@ -971,6 +977,7 @@ __device__ __forceinline__ void list_overflow(const StepArgs &a, int i, int nn, 
 constexpr int kSrchKeep = 36;   // entries a lane can hold
 template <int V>
 __global__ void __launch_bounds__(128, 8) k_search(StepArgs a) {
+    chain_wait();
     constexpr bool contact = (V & kSrchContact) != 0;   // contacttype > 0: other materials -> contact list
     constexpr bool two_pass = (V & kSrchTwoPass) != 0;  // kernel contact between materials: own material first
     constexpr unsigned kAll = 0xffffffffu;
@@ -1096,6 +1103,7 @@ __global__ void __launch_bounds__(128, 8) k_search(StepArgs a) {
 // loads overlap.
 template <int V, int G>
 __global__ void __launch_bounds__(128, 6) k_search_lanes(StepArgs a) {
+    chain_wait();
     constexpr bool contact = (V & kSrchContact) != 0;
     constexpr bool two_pass = (V & kSrchTwoPass) != 0;
     constexpr bool want_mind = (V & kSrchMind) != 0;
@@ -1266,6 +1274,7 @@ __global__ void __launch_bounds__(128, 6) k_search_lanes(StepArgs a) {
 // the lists are k_search's, entry for entry.
 constexpr int kCellWarps = 8;
 __global__ void __launch_bounds__(kCellWarps * 32, 3) k_search_cell(StepArgs a) {
+    chain_wait();
     __shared__ float4 stage[kCellWarps][32];
     __shared__ int stage_mat[kCellWarps][32];
     if (a.status->code) return;
@@ -1735,7 +1744,7 @@ void launch_skin_search(const StepArgs &a, cudaStream_t s) {
 constexpr int kSearch8Below = 24000, kSearch4Below = 64000;
 template <int V, int G>
 static void launch_lanes(const StepArgs &a, int threads, cudaStream_t s) {
-    k_search_lanes<V, G><<<(unsigned)(((long long)a.n * G + threads - 1) / threads), threads, 0, s>>>(a);
+    launch_chained(k_search_lanes<V, G>, (unsigned)(((long long)a.n * G + threads - 1) / threads), threads, 0, s, a);
 }
 template <int V>
 static void launch_search_v(const StepArgs &a, cudaStream_t s) {
@@ -1743,7 +1752,7 @@ static void launch_search_v(const StepArgs &a, cudaStream_t s) {
     const long long n = (long long)a.n * a.share;
     if (a.search_kind == 2 || n < kSearch8Below) launch_lanes<V, 8>(a, threads, s);
     else if (n < kSearch4Below) launch_lanes<V, 4>(a, threads, s);
-    else k_search<V><<<(a.n + threads - 1) / threads, threads, (threads / 32) * 33 * kSrchKeep * sizeof(unsigned), s>>>(a);
+    else launch_chained(k_search<V>, (a.n + threads - 1) / threads, threads, (threads / 32) * 33 * kSrchKeep * sizeof(unsigned), s, a);
 }
 
 void launch_search(const StepArgs &a, cudaStream_t s) {
@@ -1751,7 +1760,7 @@ void launch_search(const StepArgs &a, cudaStream_t s) {
         // grid-stride over the cells (ncells is on the device): up to 16 blocks per SM
         long long b = (a.cell_cap + kCellWarps - 1) / kCellWarps;
         if (b > 148LL * 16) b = 148LL * 16;
-        k_search_cell<<<(unsigned)(b < 1 ? 1 : b), kCellWarps * 32, 0, s>>>(a);
+        launch_chained(k_search_cell, (unsigned)(b < 1 ? 1 : b), kCellWarps * 32, 0, s, a);
         return;
     }
     const bool mind = a.prm.tcrit_opt == 2 || a.prm.diag;

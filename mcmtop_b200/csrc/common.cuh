@@ -116,6 +116,21 @@ __host__ __device__ inline double cell_origin(const DevGrid &g, int d, int b) {
     return g.gridmin[d] + (double)(b - 1) * g.cell[d];
 }
 
+// First statement of every kernel of the step's chain (launch_chained): waits
+// until the launch before it in the stream has completed and its memory is
+// visible.  Every path through such a kernel passes here, so the kernels still
+// follow one another; and none reads memory through the non-coherent path,
+// which assumes that nothing is written while the kernel is in place.
+// chain_start, of the short kernels, then lets the launch behind it begin, so
+// that its blocks are in place when this kernel ends.  The searches, gathers
+// and the constitutive update only wait (chain_wait): blocks that wait beside
+// them cost more than the launch (685 824 particles: 100.3 ms against 96.7).
+__device__ __forceinline__ void chain_start() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void raise_status(DevStatus *st, int code, int idx = -1) {
     if (atomicCAS(&st->code, 0, code) == 0) st->bad_index = idx;
 }

@@ -24,7 +24,7 @@ constexpr unsigned kPosMask = 0x3ffffffu;   // position bits of a neighbour entr
 // would each use half of every sector they touch.
 __device__ __forceinline__ double4 ld4(const double4 *p) {
     double4 r;
-    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
     return r;
 }
 

@@ -64,6 +64,7 @@ __device__ __forceinline__ void reduce_value(const StepArgs &a, int nblocks, int
 }
 
 __global__ void k_energy_bbox_reduce(StepArgs a, int nblocks, int energy, int bbox, int finish) {
+    chain_start();
     __shared__ double sm[32];
     if (a.status->code || a.time->ended >= 2) return;
     reduce_value(a, nblocks, energy, bbox, sm);
@@ -94,6 +95,7 @@ __global__ void k_energy_bbox_reduce(StepArgs a, int nblocks, int energy, int bb
 // b*T + tid + k*nblocks*T (T threads) and combines its threads in a fixed
 // order, so the sums do not depend on scheduling.
 __global__ void k_energy_step_partials(StepArgs a) {
+    chain_start();
     __shared__ double sm[32];
     if (a.status->code || a.time->ended >= 2) return;
     const int nv = 5 * a.nmat + 6;
@@ -155,6 +157,7 @@ __global__ void k_contact_forces(StepArgs a, double *out) {
 }
 
 __global__ void k_set_time(StepArgs a, double dt, double dtold, int set_dtold) {
+    chain_start();
     a.time->dt = dt;
     if (set_dtold) a.time->dtold = dtold;
 }
@@ -164,11 +167,11 @@ void launch_init_critts_reduce(const StepArgs &a, cudaStream_t s, int nblocks) {
 }
 
 void launch_energy_bbox_reduce(const StepArgs &a, cudaStream_t s, int nblocks, int energy, int bbox, int finish) {
-    k_energy_bbox_reduce<<<5 * a.nmat + 6, 256, 0, s>>>(a, nblocks, energy, bbox, finish);
+    launch_chained(k_energy_bbox_reduce, 5 * a.nmat + 6, 256, 0, s, a, nblocks, energy, bbox, finish);
 }
 
 void launch_energy_step_partials(const StepArgs &a, cudaStream_t s, int nblocks) {
-    k_energy_step_partials<<<nblocks, 256, 0, s>>>(a);
+    launch_chained(k_energy_step_partials, nblocks, 256, 0, s, a);
 }
 
 void launch_contact_forces(const StepArgs &a, cudaStream_t s, double *out) {
@@ -176,7 +179,7 @@ void launch_contact_forces(const StepArgs &a, cudaStream_t s, double *out) {
 }
 
 void launch_set_time(const StepArgs &a, cudaStream_t s, double dt, double dtold, int set_dtold) {
-    k_set_time<<<1, 1, 0, s>>>(a, dt, dtold, set_dtold);
+    launch_chained(k_set_time, 1, 1, 0, s, a, dt, dtold, set_dtold);
 }
 
 }  // namespace mcm

@@ -68,6 +68,7 @@ __device__ __forceinline__ Entry entry_at(const StepArgs &a, int t, int k, int n
 // ----------------------------------------------------------- strain rate
 template <int L, int DISC>
 __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_strain_coop(StepArgs a) {
+    chain_wait();
     if (skip_step(a)) return;
     const int sub = threadIdx.x / L, lane = threadIdx.x % L;
     const int per = blockDim.x / L;
@@ -202,6 +203,7 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_strain_coop(StepArgs
 // measured 382 and 561, two neighbours ahead 433 and 553).
 template <int L, int DISC, bool ASYM>
 __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepArgs a, int integrate) {
+    chain_wait();
     __shared__ double sm[32];
     if (skip_step(a)) return;
     const int sub = threadIdx.x / L, lane = threadIdx.x % L;

@@ -272,6 +272,7 @@ __device__ __forceinline__ void correction_of(const StepArgs &a, const Walk &w, 
 // state's diagnostic arrays, which the constitutive kernel reads.
 template <int DISC, int L>
 __global__ void __launch_bounds__(seq_threads(L), seq_blocks(DISC, L)) k_strain_seq(StepArgs a) {
+    chain_wait();
     constexpr int kSeqThreads = seq_threads(L), kPer = kSeqThreads / L;   // particles per block
     __shared__ double bufs[kSeqThreads / 32][L == 1 ? 1 : 64 * seq_pitch(9)];
     __shared__ double grad[9][L == 1 ? 1 : kPer + 1];
@@ -381,6 +382,7 @@ __device__ __forceinline__ void lower_from_rec(const double4 &r3, double A[3][3]
 // record.
 template <int DISC, bool ASYM, int L>
 __global__ void __launch_bounds__(seq_threads(L), seq_blocks(DISC, L)) k_momentum_seq(StepArgs a, int integrate) {
+    chain_wait();
     constexpr unsigned kAll = 0xffffffffu;
     constexpr int kSeqThreads = seq_threads(L), kPer = kSeqThreads / L, kWarps = kSeqThreads / 32;
     __shared__ double bufs[kWarps][L == 1 ? 1 : (DISC == 0 ? 64 * seq_pitch(3) : 32 * seq_pitch(18))];

@@ -211,6 +211,7 @@ __device__ __forceinline__ void update_h(const StepArgs &a, int i, PState<double
 #define MCM_CONST_MINBLOCKS 2
 #endif
 __global__ void __launch_bounds__(kRedThreads, MCM_CONST_MINBLOCKS) k_constitutive(StepArgs a) {
+    chain_wait();
     __shared__ double sm[32];
     if (skip_step(a)) return;
     const double dt = a.time->dt;
@@ -259,6 +260,7 @@ __global__ void __launch_bounds__(kRedThreads, MCM_CONST_MINBLOCKS) k_constituti
 // ghost contact list (the reference reads their ids from the real contact
 // list past ncont, :48 of mcm_get_j_cont_info.f90, entries no search wrote).
 __global__ void k_rep_cont(StepArgs a) {
+    chain_start();
     if (skip_step(a)) return;
     double *const *f = a.F.f;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < a.n; t += gridDim.x * blockDim.x) {
@@ -320,6 +322,7 @@ __global__ void k_rep_cont(StepArgs a) {
 // mass and V = m/rho (the corrected sums').  Ghost stresses follow MCM/mcm_update_ghost_stress.f90:28-41 (all
 // off-diagonals negated) with the ghost's own density from its creation.
 __global__ void k_mom_prep(StepArgs a) {
+    chain_start();
     if (skip_step(a)) return;
     const double *const *f = a.F.f;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x) {
@@ -420,6 +423,7 @@ __device__ __forceinline__ void integrate_particle(const StepArgs &a, int i, con
 
 // Split path: velocity and position update after the host's output phase.
 __global__ void __launch_bounds__(kRedThreads) k_update_move(StepArgs a) {
+    chain_start();
     __shared__ double sm[32];
     if (a.status->code) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -447,6 +451,7 @@ __global__ void __launch_bounds__(kRedThreads) k_update_move(StepArgs a) {
 // In a fused run the step that terminates skips all three, like the fused
 // momentum kernel.
 __global__ void k_velocity(StepArgs a) {
+    chain_start();
     if (skip_step(a) || a.time->ended) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
@@ -468,6 +473,7 @@ __global__ void k_velocity(StepArgs a) {
 // updated state, ghosts their copies from the start of the step; W takes the
 // neighbour's h and V_j = m_j / ((rho_j + rho_i) / 2).
 __global__ void k_xsph_sum(StepArgs a) {
+    chain_start();
     if (skip_step(a) || a.time->ended) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= a.n) return;
@@ -499,6 +505,7 @@ __global__ void k_xsph_sum(StepArgs a) {
 }
 
 __global__ void __launch_bounds__(kRedThreads) k_xsph_move(StepArgs a) {
+    chain_start();
     __shared__ double sm[32];
     if (skip_step(a) || a.time->ended) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -694,11 +701,11 @@ void launch_strain(const StepArgs &a, cudaStream_t s) {
     void (*kern)(StepArgs) = a.prm.disctype == 0 ? (lanes == 1 ? k_strain_seq<0, 1> : k_strain_seq<0, 8>)
                                                  : (lanes == 1 ? k_strain_seq<1, 1> : k_strain_seq<1, 8>);
     const int threads = seq_threads(lanes);
-    kern<<<nblk(a.n, threads / lanes), threads, 0, s>>>(a);
+    launch_chained(kern, nblk(a.n, threads / lanes), threads, 0, s, a);
 #else
     constexpr int L = kCoopLanes;
     void (*kern)(StepArgs) = a.prm.disctype == 0 ? k_strain_coop<L, 0> : k_strain_coop<L, 1>;
-    kern<<<pair_blocks_of(a, L, (const void *)kern), pair_threads_of(a), 0, s>>>(a);
+    launch_chained(kern, pair_blocks_of(a, L, (const void *)kern), pair_threads_of(a), 0, s, a);
 #endif
 }
 
@@ -706,14 +713,14 @@ void launch_constitutive(const StepArgs &a, cudaStream_t s) {
     int blocks = nblk(a.n, kRedThreads);
     const int wave = 148 * resident_per_sm((const void *)k_constitutive, kRedThreads);
     if (blocks > wave) blocks = wave;
-    k_constitutive<<<blocks, kRedThreads, 0, s>>>(a);
+    launch_chained(k_constitutive, blocks, kRedThreads, 0, s, a);
 }
 
 void launch_mom_prep(const StepArgs &a, cudaStream_t s) {
-    k_mom_prep<<<gs_blocks(a.n > a.ghost_cap ? a.n : a.ghost_cap), 256, 0, s>>>(a);
+    launch_chained(k_mom_prep, gs_blocks(a.n > a.ghost_cap ? a.n : a.ghost_cap), 256, 0, s, a);
 }
 
-void launch_rep_cont(const StepArgs &a, cudaStream_t s) { k_rep_cont<<<gs_blocks(a.n), 256, 0, s>>>(a); }
+void launch_rep_cont(const StepArgs &a, cudaStream_t s) { launch_chained(k_rep_cont, gs_blocks(a.n), 256, 0, s, a); }
 
 int launch_momentum(const StepArgs &a, cudaStream_t s, int integrate) {
 #if MCM_EXACT
@@ -726,7 +733,7 @@ int launch_momentum(const StepArgs &a, cudaStream_t s, int integrate) {
     int blocks = nblk(a.n, threads / lanes);
     const int wave = 148 * resident_per_sm((const void *)kern, threads);
     if (blocks > wave) blocks = wave;
-    kern<<<blocks, threads, 0, s>>>(a, integrate);
+    launch_chained(kern, blocks, threads, 0, s, a, integrate);
     return blocks;
 #else
     constexpr int L = kCoopLanes;
@@ -734,22 +741,22 @@ int launch_momentum(const StepArgs &a, cudaStream_t s, int integrate) {
                                   : (a.prm.asym ? k_momentum_coop<L, 0, true> : k_momentum_coop<L, 0, false>);
     const int blocks = pair_blocks_of(a, L, (const void *)kern);
     if (a.nmat > 1) launch_energy_step_partials(a, s, blocks);
-    kern<<<blocks, pair_threads_of(a), 0, s>>>(a, integrate);
+    launch_chained(kern, blocks, pair_threads_of(a), 0, s, a, integrate);
     return blocks;
 #endif
 }
 
 int launch_update_move(const StepArgs &a, cudaStream_t s) {
     int blocks = nblk(a.n, kRedThreads);
-    k_update_move<<<blocks, kRedThreads, 0, s>>>(a);
+    launch_chained(k_update_move, blocks, kRedThreads, 0, s, a);
     return blocks;
 }
 
 int launch_xsph_move(const StepArgs &a, cudaStream_t s) {
     const int blocks = nblk(a.n, kRedThreads);
-    k_velocity<<<blocks, kRedThreads, 0, s>>>(a);
-    k_xsph_sum<<<blocks, kRedThreads, 0, s>>>(a);
-    k_xsph_move<<<blocks, kRedThreads, 0, s>>>(a);
+    launch_chained(k_velocity, blocks, kRedThreads, 0, s, a);
+    launch_chained(k_xsph_sum, blocks, kRedThreads, 0, s, a);
+    launch_chained(k_xsph_move, blocks, kRedThreads, 0, s, a);
     return blocks;
 }
 

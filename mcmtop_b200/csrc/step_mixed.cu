@@ -126,13 +126,13 @@ struct __align__(32) Rec8 {
 };
 __device__ __forceinline__ Rec8 ld_rec8(const float4 *p) {
     Rec8 r;
-    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z),
                    "=f"(r.b.w)
                  : "l"(p));
     return r;
 }
-__device__ __forceinline__ float4 ld_rec4(const float4 *p) { return __ldg(p); }
+__device__ __forceinline__ float4 ld_rec4(const float4 *p) { return *p; }
 
 // A particle's own h and what every pair of one h has in common:
 // ih = 1/h and c3 = 1/(pi h^3).
@@ -196,7 +196,7 @@ __device__ __forceinline__ void pair_entries(const unsigned *base, int lane, uns
 #pragma unroll
     for (int v = 0; v < U / 4; ++v) {
         // lane 0 loads entries 8v .. 8v+3, lane 1 entries 8v+4 .. 8v+7
-        const uint4 w = __ldg(reinterpret_cast<const uint4 *>(base + 8 * v + 4 * lane));
+        const uint4 w = *reinterpret_cast<const uint4 *>(base + 8 * v + 4 * lane);
         const unsigned r0 = __shfl_xor_sync(pm, lane ? w.x : w.y, 1);
         const unsigned r1 = __shfl_xor_sync(pm, lane ? w.z : w.w, 1);
         e[4 * v + 0] = lane ? r0 : w.x;
@@ -242,6 +242,7 @@ __device__ __forceinline__ void store_rates(const StepArgs &a, int i, int lane, 
 // lane, the compensation carried into the TwoSum lane combination).
 template <bool KAHAN>
 __global__ void __launch_bounds__(256, 3) k_strain(StepArgs a) {
+    chain_wait();
     __shared__ Offsets4 offs;
     if (skip_step(a)) return;
     const int sub = threadIdx.x / L, lane = threadIdx.x % L;
@@ -409,6 +410,7 @@ __device__ __forceinline__ int stage_index(const StageWin &W, int wbase, unsigne
 }
 
 __global__ void __launch_bounds__(kStageThreads, 6) k_strain_staged(StepArgs a) {
+    chain_wait();
     __shared__ Offsets4 offs;
     __shared__ float4 stage[2 * kStageCap];
     __shared__ StageWin W;
@@ -506,6 +508,7 @@ __device__ __forceinline__ float4 *mom_lower(const StepArgs &a) { return a.frec0
 // stresses with every off-diagonal negated (MCM/mcm_update_ghost_stress.f90:
 // 272-285) over the ghost's own density.
 __global__ void k_mom_prep(StepArgs a) {
+    chain_start();
     if (skip_step(a)) return;
     const Frame fr = make_frame(*a.grid);
     const double *const *f = a.F.f;
@@ -643,6 +646,7 @@ __device__ __forceinline__ void momentum_term(float dx, float dy, float dz, floa
 
 template <bool ASYM, bool KAHAN, bool STAGED>
 __global__ void __launch_bounds__(STAGED ? kStageThreads : 256, STAGED ? 4 : MCM_MOM_MINBLOCKS) k_momentum(StepArgs a, int integrate_flag) {
+    chain_wait();
     __shared__ double sm[32];
     __shared__ Offsets3 offs;
     __shared__ float4 stage[STAGED ? 3 * kStageCapM : 1];
@@ -849,20 +853,20 @@ void launch_strain(const StepArgs &a, cudaStream_t s) {
     if (a.pair_kind == 2 && !a.prm.kahan) {
         int b = nblk(a.n, kStageThreads / L);
         if (b > 148 * 6) b = 148 * 6;
-        k_strain_staged<<<b, kStageThreads, 0, s>>>(a);
+        launch_chained(k_strain_staged, b, kStageThreads, 0, s, a);
         return;
     }
     if (a.prm.kahan) {
-        k_strain<true><<<pair_blocks_of(a, L, (const void *)k_strain<true>), pair_threads_of(a), 0, s>>>(a);
+        launch_chained(k_strain<true>, pair_blocks_of(a, L, (const void *)k_strain<true>), pair_threads_of(a), 0, s, a);
     } else {
-        k_strain<false><<<pair_blocks_of(a, L, (const void *)k_strain<false>), pair_threads_of(a), 0, s>>>(a);
+        launch_chained(k_strain<false>, pair_blocks_of(a, L, (const void *)k_strain<false>), pair_threads_of(a), 0, s, a);
     }
 }
 
 void launch_mom_prep(const StepArgs &a, cudaStream_t s) {
     int n = a.n > a.ghost_cap ? a.n : a.ghost_cap;
     int b = nblk(n, 256);
-    k_mom_prep<<<b < 148 * 16 ? b : 148 * 16, 256, 0, s>>>(a);
+    launch_chained(k_mom_prep, b < 148 * 16 ? b : 148 * 16, 256, 0, s, a);
 }
 
 int launch_momentum(const StepArgs &a, cudaStream_t s, int integrate_flag) {
@@ -871,15 +875,15 @@ int launch_momentum(const StepArgs &a, cudaStream_t s, int integrate_flag) {
         if (blocks > 148 * 4) blocks = 148 * 4;
         if (a.red_blocks > 0 && blocks > a.red_blocks) blocks = a.red_blocks;
         if (a.nmat > 1) launch_energy_step_partials(a, s, blocks);
-        if (a.prm.asym) k_momentum<true, false, true><<<blocks, kStageThreads, 0, s>>>(a, integrate_flag);
-        else k_momentum<false, false, true><<<blocks, kStageThreads, 0, s>>>(a, integrate_flag);
+        if (a.prm.asym) launch_chained(k_momentum<true, false, true>, blocks, kStageThreads, 0, s, a, integrate_flag);
+        else launch_chained(k_momentum<false, false, true>, blocks, kStageThreads, 0, s, a, integrate_flag);
         return blocks;
     }
     void (*kern)(StepArgs, int) = a.prm.asym ? (a.prm.kahan ? k_momentum<true, true, false> : k_momentum<true, false, false>)
                                              : (a.prm.kahan ? k_momentum<false, true, false> : k_momentum<false, false, false>);
     const int blocks = pair_blocks_of(a, L, (const void *)kern);
     if (a.nmat > 1) launch_energy_step_partials(a, s, blocks);
-    kern<<<blocks, pair_threads_of(a), 0, s>>>(a, integrate_flag);
+    launch_chained(kern, blocks, pair_threads_of(a), 0, s, a, integrate_flag);
     return blocks;
 }
 
