@@ -121,6 +121,8 @@ int alloc_particles(mcm_gpu_handle *h) {
     h->A.sny = h->A.snx + (np + 32);
     h->A.snz = h->A.sny + (np + 32);
     h->A.snh = h->A.snz + (np + 32);
+    if ((st = dalloc(h, &h->A.pos_of, np))) return st;
+    if (h->A.prm.boundary && (st = dalloc(h, &h->A.ghost_of, np))) return st;
     if ((st = dalloc(h, &h->A.cmat, np))) return st;
     if ((st = dalloc(h, &h->A.ckey, np))) return st;
     if ((st = dalloc(h, &h->A.reorder_tmp, np))) return st;
@@ -130,7 +132,6 @@ int alloc_particles(mcm_gpu_handle *h) {
     CK(cudaMemsetAsync(h->A.nnbr, 0, sizeof(int) * np, h->stream));
     CK(cudaMemsetAsync(h->A.gnnbr, 0, sizeof(int) * np, h->stream));
     if (h->A.prm.skin > 0.0) {
-        if ((st = dalloc(h, &h->A.pos_of, np))) return st;
         if ((st = dalloc(h, &h->A.supn, np))) return st;
         if ((st = dalloc(h, &h->A.xref, 3 * np))) return st;
     }
@@ -185,6 +186,7 @@ int alloc_ghosts(mcm_gpu_handle *h, int cap) {
     for (double **p : dd)
         if ((st = dalloc(h, p, (size_t)cap))) return st;
     if ((st = dalloc(h, &h->A.gpar, (size_t)cap))) return st;
+    if ((st = dalloc(h, &h->A.gnext, (size_t)cap))) return st;
     if ((st = dalloc(h, &h->A.gmat, (size_t)cap))) return st;
     if ((st = dalloc(h, &h->A.gflip, (size_t)cap))) return st;
     if ((st = dalloc(h, &h->A.grec0, (size_t)cap))) return st;
@@ -311,7 +313,9 @@ void launch_strain(mcm_gpu_handle *h) {
     if (prec == MCM_PREC_FP64_EXACT) exact::launch_constitutive(h->A, h->stream);
     else fast::launch_constitutive(h->A, h->stream);
 }
-int launch_mom(mcm_gpu_handle *h, int integrate) {
+// prep: form the gather records, which the constitutive update has written,
+// once more (the state may have changed since)
+int launch_mom(mcm_gpu_handle *h, int integrate, int prep) {
     const int prec = h->cfg.precision;
     if (h->A.prm.contact) {
         // MCM/mcm_solution.f90:64: repulsive contact before the momentum sum
@@ -319,10 +323,9 @@ int launch_mom(mcm_gpu_handle *h, int integrate) {
         if (prec == MCM_PREC_FP64_EXACT) exact::launch_rep_cont(h->A, h->stream);
         else fast::launch_rep_cont(h->A, h->stream);
     }
-    {
+    if (prep) {
         Scope sc(h, R_MOM_PREP, 1);
         if (prec == MCM_PREC_FP64_EXACT) exact::launch_mom_prep(h->A, h->stream);
-        else if (prec == MCM_PREC_MIXED) mixed::launch_mom_prep(h->A, h->stream);
         else fast::launch_mom_prep(h->A, h->stream);
     }
     // the cooperative gathers of several materials add a fixed-order energy-partials kernel
@@ -377,10 +380,10 @@ void enqueue_part_a(mcm_gpu_handle *h) {
 }
 
 // momentum -> boundcond -> calctotale (-> update_velocity -> move)
-void enqueue_part_b(mcm_gpu_handle *h, int integrate, int finish) {
+void enqueue_part_b(mcm_gpu_handle *h, int integrate, int finish, int prep) {
     if (h->A.prm.veloc_opt && integrate) {
         // XSPH needs every updated velocity before any particle moves
-        int nb = launch_mom(h, 0);
+        int nb = launch_mom(h, 0, prep);
         {
             Scope sc(h, R_REDUCE, 1);
             launch_energy_bbox_reduce(h->A, h->stream, nb, 1, 0);
@@ -390,7 +393,7 @@ void enqueue_part_b(mcm_gpu_handle *h, int integrate, int finish) {
         launch_energy_bbox_reduce(h->A, h->stream, nb, 0, 1, finish);
         return;
     }
-    int nb = launch_mom(h, integrate);
+    int nb = launch_mom(h, integrate, prep);
     Scope sc(h, R_REDUCE, 1);
     launch_energy_bbox_reduce(h->A, h->stream, nb, 1, integrate, finish);
 }
@@ -753,10 +756,10 @@ int mcm_gpu_destroy(mcm_gpu_handle *h) {
                     h->A.cpos, h->A.snx, h->A.cmat, h->A.ckey, h->A.reorder_tmp, h->A.reorder_grp, h->A.nidx,
                     h->A.red, h->A.cell_count, h->A.cell_start, h->A.scan_sums, h->A.gcell,
                     h->A.layer_count, h->A.gx, h->A.gy, h->A.gz, h->A.gvx, h->A.gvy,
-                    h->A.gvz, h->A.gmass, h->A.gh, h->A.ghold, h->A.grho, h->A.gpar, h->A.gmat, h->A.gflip,
+                    h->A.gvz, h->A.gmass, h->A.gh, h->A.ghold, h->A.grho, h->A.gpar, h->A.gnext, h->A.gmat, h->A.gflip,
                     h->A.grec0, h->A.grec1, h->A.grec2, h->A.gnbr, h->A.rec3, h->A.grec3,
                     h->A.cidx, h->A.gcont, h->A.ncont, h->A.gncont,
-                    h->A.sup, h->A.supn, h->A.pos_of, h->A.xref};
+                    h->A.sup, h->A.supn, h->A.pos_of, h->A.ghost_of, h->A.xref};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (double *p : h->adj_ckpt)
@@ -1055,7 +1058,7 @@ int mcm_gpu_step_b(mcm_gpu_handle *h, double *energies) {
     h->A.split_mode = 1;
     if (!h->part_b_enqueued) {   // step_a has not enqueued it (a call out of the usual order)
         if ((st = reset_status(h))) return st;
-        enqueue_part_b(h, 0);
+        enqueue_part_b(h, 0, 0, 1);
     }
     h->part_b_enqueued = false;
     if (!energies) return MCM_OK;   // nothing to wait for: errors surface at the next waiting call

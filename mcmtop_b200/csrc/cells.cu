@@ -261,7 +261,6 @@ __global__ void __launch_bounds__(256) k_cell_scatter(StepArgs a) {
 // of the step's arithmetic REC: positions shifted back half a step
 // (MCM/mcm_strain.f90:27-31), velocities and V = m/rho
 // (MCM/mcm_oldstrain.f90:44).
-enum { kRecFP64 = 0, kRecMixed = 1 };
 template <int REC>
 __device__ __forceinline__ void write_records(const StepArgs &a, const DevGrid &g, int p, int i, int key, double dt,
                                               bool with_cposf, unsigned long long &hbits, unsigned long long &lbits) {
@@ -269,7 +268,8 @@ __device__ __forceinline__ void write_records(const StepArgs &a, const DevGrid &
     const double x = f[FX][i], y = f[FY][i], z = f[FZ][i], h = f[FH][i];
     const double vx = f[FVX][i], vy = f[FVY][i], vz = f[FVZ][i];
     a.cpos[p] = make_double4(x, y, z, h);
-    if (a.pos_of) a.pos_of[i] = p;
+    a.pos_of[i] = p;
+    if (a.prm.boundary) a.ghost_of[i] = -1;
     a.cmat[p] = a.F.mat[i];
     a.ckey[p] = key;
     double o[3] = {0.0, 0.0, 0.0};
@@ -662,6 +662,7 @@ __global__ void k_ghost_emit(StepArgs a) {
                 }
             }
             a.gpar[g] = j;
+            a.gnext[g] = atomicExch(&a.ghost_of[j], g);
             a.gflip[g] = flips;
             a.gmat[g] = a.F.mat[j];
             a.gmass[g] = a.F.f[FMASS][j];

@@ -139,7 +139,8 @@ int sync_status(mcm_gpu_handle *h);
 int regrow(mcm_gpu_handle *h, int *grew);
 int alloc_table(mcm_gpu_handle *h, int nstride, int gstride);
 void enqueue_part_a(mcm_gpu_handle *h);
-void enqueue_part_b(mcm_gpu_handle *h, int integrate, int finish = 0);   // finish: ends the fused step
+// finish: ends the fused step; prep: not directly after enqueue_part_a
+void enqueue_part_b(mcm_gpu_handle *h, int integrate, int finish = 0, int prep = 0);
 int check_handle(mcm_gpu_handle *h);
 size_t snap_doubles(const mcm_gpu_handle *h);
 int snap_save(mcm_gpu_handle *h, double *buf);

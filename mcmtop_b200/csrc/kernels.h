@@ -34,6 +34,7 @@ struct StepArgs {
     int *scan_ticket; // blocks of k_cell_scan that have ended
     int *cell_start;  // cell_cap + 1
     int *cell_list;   // npad: position -> state index
+    int *pos_of;      // npad: state index -> position
     int *n_inside;    // particles inside the grid (device counter)
     double4 *cpos;    // per position: x, y, z, h at neighbour time
     float4 *cposf;    // per position: x, y, z relative to the cell origin (FP32), h (for search_kind 3 and the skin lists)
@@ -45,6 +46,7 @@ struct StepArgs {
     // ghosts (SoA, ghost_cap each)
     double *gx, *gy, *gz, *gvx, *gvy, *gvz, *gmass, *gh, *ghold, *grho;
     int *gpar, *gmat;
+    int *ghost_of, *gnext;   // npad: a particle's ghosts as a list: one of them or -1; per ghost: the next or -1
     int *gflip;       // per ghost: bit d set if its position is the parent's mirrored along axis d
     int *ngp;         // device ghost counter
     int *ghost_ticket;                           // blocks of k_ghost_count that have ended
@@ -66,9 +68,8 @@ struct StepArgs {
     int cstride, gcstride;
     // skin lists (prm.skin > 0): per STATE index i, the state indices of the
     // particles within h_i + h_j + skin at the last build, sup[i*sstride + k],
-    // supn[i] of them; the positions x at that build (xref, 3 x npad); pos_of[i]
-    // the cell-order position of state index i in the current cell list
-    int *sup, *supn, *pos_of;
+    // supn[i] of them; the positions x at that build (xref, 3 x npad)
+    int *sup, *supn;
     int sstride;
     double *xref;
     int *skin_flags;                 // [0] force a build, [1] this step builds, [2] builds so far
@@ -96,6 +97,9 @@ struct StepArgs {
     double *energy;   // 5*nmat + 3
 };
 
+// Whose gathers read the strain and momentum records: the FP64 steps', the mixed step's.
+enum { kRecFP64 = 0, kRecMixed = 1 };
+
 // cells.cu
 void launch_cell_build(const StepArgs &a, cudaStream_t s);
 void launch_ghosts(const StepArgs &a, cudaStream_t s);
@@ -120,7 +124,6 @@ void launch_contact_forces(const StepArgs &a, cudaStream_t s, double *out);
 // update of the mixed path is the FP64 fast one)
 namespace mixed {
 void launch_strain(const StepArgs &a, cudaStream_t s);
-void launch_mom_prep(const StepArgs &a, cudaStream_t s);
 int launch_momentum(const StepArgs &a, cudaStream_t s, int integrate);
 }  // namespace mixed
 

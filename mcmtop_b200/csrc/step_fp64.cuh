@@ -186,6 +186,72 @@ __device__ __forceinline__ double block_min(double v, double *sm) {
     return v;
 }
 
+// --------------------------------------------------------- momentum records
+// Gather record of position p: x, h; (sigma - q)/rho^2
+// (MCM/mcm_oldacceleration.f90:79-80); mass and V = m/rho (the corrected
+// sums').  The mixed step's is FP32, formed in FP64, its x relative to the
+// origin of the particle's cell `key`.
+struct Moment {
+    double h, mass, rho, q;
+    const double *sig, *sigl;   // 11 22 33 12 13 23; 21 31 32
+};
+template <int REC>
+__device__ __forceinline__ void write_momentum(const StepArgs &a, const DevGrid &g, int p, int key, double x, double y,
+                                               double z, const Moment &s) {
+    if (REC == kRecMixed) {
+        double o[3] = {0.0, 0.0, 0.0};
+        if (key >= 0) {
+            int b[3];
+            cell_coords(key, g.gridlim, b[0], b[1], b[2]);
+            for (int d = 0; d < 3; ++d) o[d] = cell_origin(g, d, b[d]);
+        }
+        const double ir2 = 1.0 / (s.rho * s.rho);
+        const float4 f0 = make_float4((float)(x - o[0]), (float)(y - o[1]), (float)(z - o[2]), (float)s.h);
+        const float4 f1 = make_float4((float)((s.sig[T11] - s.q) * ir2), (float)((s.sig[T22] - s.q) * ir2),
+                                      (float)((s.sig[T33] - s.q) * ir2), (float)(s.sig[T12] * ir2));
+        a.frec0[2 * (size_t)p] = f0;
+        a.frec0[2 * (size_t)p + 1] = f1;
+        a.frec0[2 * (size_t)a.npad + p] =
+            make_float4((float)(s.sig[T13] * ir2), (float)(s.sig[T23] * ir2), (float)s.mass, (float)s.rho);
+        // the cap model's lower triangle (21 31 32), read only when a material has it
+        if (a.prm.asym)
+            a.frec0[3 * (size_t)a.npad + p] =
+                make_float4((float)(s.sigl[0] * ir2), (float)(s.sigl[1] * ir2), (float)(s.sigl[2] * ir2), 0.0f);
+    } else {
+        const double r2 = s.rho * s.rho;
+        a.rec0[p] = make_double4(x, y, z, s.h);
+        a.rec1[p] = make_double4((s.sig[T11] - s.q) / r2, (s.sig[T22] - s.q) / r2, (s.sig[T33] - s.q) / r2,
+                                 (s.sig[T12] - 0.0) / r2);
+        a.rec2[p] = make_double4((s.sig[T13] - 0.0) / r2, (s.sig[T23] - 0.0) / r2, s.mass, s.mass / s.rho);
+        if (a.prm.asym)
+            a.rec3[p] = make_double4((s.sigl[0] - 0.0) / r2, (s.sigl[1] - 0.0) / r2, (s.sigl[2] - 0.0) / r2, 0.0);
+    }
+}
+
+// Ghost q's record: its parent's stress after the constitutive update
+// (MCM/mcm_update_ghost_stress.f90:28-41, all off-diagonals negated) with the
+// ghost's own density from its creation.
+template <int REC>
+__device__ __forceinline__ void write_ghost_momentum(const StepArgs &a, int q, const Moment &s) {
+    const double rho = a.grho[q], m = a.gmass[q];
+    const double r2 = rho * rho;
+    a.grec0[q] = make_double4(a.gx[q], a.gy[q], a.gz[q], a.gh[q]);
+    if (REC == kRecMixed) {
+        const double ir2 = 1.0 / r2;
+        a.gfrec1[q] = make_float4((float)((s.sig[T11] - s.q) * ir2), (float)((s.sig[T22] - s.q) * ir2),
+                                  (float)((s.sig[T33] - s.q) * ir2), (float)(-s.sig[T12] * ir2));
+        a.gfrec2[q] = make_float4((float)(-s.sig[T13] * ir2), (float)(-s.sig[T23] * ir2), (float)m, (float)rho);
+        if (a.prm.asym) a.grec3[q] = make_double4(-s.sigl[0] * ir2, -s.sigl[1] * ir2, -s.sigl[2] * ir2, 0.0);
+    } else {
+        a.grec1[q] = make_double4((s.sig[T11] - s.q) / r2, (s.sig[T22] - s.q) / r2, (s.sig[T33] - s.q) / r2,
+                                  ((-s.sig[T12]) - (-0.0)) / r2);
+        a.grec2[q] = make_double4(((-s.sig[T13]) - (-0.0)) / r2, ((-s.sig[T23]) - (-0.0)) / r2, m, m / rho);
+        if (a.prm.asym)
+            a.grec3[q] = make_double4(((-s.sigl[0]) - (-0.0)) / r2, ((-s.sigl[1]) - (-0.0)) / r2,
+                                      ((-s.sigl[2]) - (-0.0)) / r2, 0.0);
+    }
+}
+
 // ------------------------------------------------- variable smoothing length
 // MCM/mcm_update_h.f90:25-55 (after mcm_strain, before the constitutive
 // update): particles at or above their cut-off pressure take a new h and
@@ -207,13 +273,25 @@ __device__ __forceinline__ void update_h(const StepArgs &a, int i, PState<double
 // Two resident blocks per SM (128 registers, a few hundred bytes of spills)
 // measured faster than one at 154 registers: 0.27 against 0.43 ms per step
 // on the 2M bar.
+//
+// Writes the momentum gather's records of the particle, at its position in cell
+// order, and of its ghosts too: whole 32-byte sectors, while the state they are
+// made of is in registers.  685 824 particles, this kernel and a kernel of its
+// own for the records: 105 + 33 us (mixed), 105 + 43 (FP64); as one 123 and
+// 132.  16 848: 18 + 11 and 20.
 #ifndef MCM_CONST_MINBLOCKS
 #define MCM_CONST_MINBLOCKS 2
 #endif
+template <int REC>
 __global__ void __launch_bounds__(kRedThreads, MCM_CONST_MINBLOCKS) k_constitutive(StepArgs a) {
     chain_wait();
     __shared__ double sm[32];
+    __shared__ DevGrid g;
     if (skip_step(a)) return;
+    if (REC == kRecMixed) {
+        if (threadIdx.x == 0) g = *a.grid;
+        __syncthreads();
+    }
     const double dt = a.time->dt;
     double crit = 1.0e20;
 #pragma unroll 1
@@ -241,9 +319,14 @@ __global__ void __launch_bounds__(kRedThreads, MCM_CONST_MINBLOCKS) k_constituti
         const double xs = f[FX][i] - 0.5 * vx * dt;
         const double ys = f[FY][i] - 0.5 * vy * dt;
         const double zs = f[FZ][i] - 0.5 * vz * dt;
-        f[FX][i] = xs + 0.5 * vx * dt;
-        f[FY][i] = ys + 0.5 * vy * dt;
-        f[FZ][i] = zs + 0.5 * vz * dt;
+        const double x = xs + 0.5 * vx * dt, y = ys + 0.5 * vy * dt, z = zs + 0.5 * vz * dt;
+        f[FX][i] = x;
+        f[FY][i] = y;
+        f[FZ][i] = z;
+        const Moment s = {P.h, P.mass, P.rho, P.q, P.sig, P.sigl};
+        write_momentum<REC>(a, g, a.pos_of[i], a.key[i], x, y, z, s);
+        if (a.prm.boundary)
+            for (int q = a.ghost_of[i]; q >= 0; q = a.gnext[q]) write_ghost_momentum<REC>(a, q, s);
     }
     double m = block_min(crit, sm);
     if (threadIdx.x == 0) finish_critts(a, m);
@@ -318,41 +401,26 @@ __global__ void k_rep_cont(StepArgs a) {
 }
 
 // --------------------------------------------------------- momentum prep
-// Gather records: x, h; (sigma - q)/rho^2 (MCM/mcm_oldacceleration.f90:79-80);
-// mass and V = m/rho (the corrected sums').  Ghost stresses follow MCM/mcm_update_ghost_stress.f90:28-41 (all
-// off-diagonals negated) with the ghost's own density from its creation.
+// The records of a momentum sum that does not directly follow the constitutive
+// update (a call of the split loop out of its usual order).
+template <int REC>
 __global__ void k_mom_prep(StepArgs a) {
     chain_start();
+    __shared__ DevGrid grid;
     if (skip_step(a)) return;
+    if (REC == kRecMixed) {
+        if (threadIdx.x == 0) grid = *a.grid;
+        __syncthreads();
+    }
     const double *const *f = a.F.f;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x) {
         const int i = a.cell_list[p];
-        double rho = f[FRHO][i];
-        double r2 = rho * rho;
-        double q = f[FQ][i];
-        a.rec0[p] = make_double4(f[FX][i], f[FY][i], f[FZ][i], f[FH][i]);
-        a.rec1[p] = make_double4((f[FS11][i] - q) / r2, (f[FS22][i] - q) / r2, (f[FS33][i] - q) / r2,
-                                 (f[FS12][i] - 0.0) / r2);
-        a.rec2[p] = make_double4((f[FS13][i] - 0.0) / r2, (f[FS23][i] - 0.0) / r2, f[FMASS][i], f[FMASS][i] / rho);
-        if (a.prm.asym)
-            a.rec3[p] = make_double4((f[FL21][i] - 0.0) / r2, (f[FL31][i] - 0.0) / r2, (f[FL32][i] - 0.0) / r2, 0.0);
-    }
-    if (a.prm.boundary) {
-        const int ngp = *a.ngp;
-        for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ngp; g += gridDim.x * blockDim.x) {
-            int j = a.gpar[g];
-            double rho = a.grho[g];
-            double r2 = rho * rho;
-            double q = f[FQ][j];
-            a.grec0[g] = make_double4(a.gx[g], a.gy[g], a.gz[g], a.gh[g]);
-            a.grec1[g] = make_double4((f[FS11][j] - q) / r2, (f[FS22][j] - q) / r2, (f[FS33][j] - q) / r2,
-                                      ((-f[FS12][j]) - (-0.0)) / r2);
-            a.grec2[g] = make_double4(((-f[FS13][j]) - (-0.0)) / r2, ((-f[FS23][j]) - (-0.0)) / r2, a.gmass[g],
-                                      a.gmass[g] / rho);
-            if (a.prm.asym)
-                a.grec3[g] = make_double4(((-f[FL21][j]) - (-0.0)) / r2, ((-f[FL31][j]) - (-0.0)) / r2,
-                                          ((-f[FL32][j]) - (-0.0)) / r2, 0.0);
-        }
+        const double sig[6] = {f[FS11][i], f[FS22][i], f[FS33][i], f[FS12][i], f[FS13][i], f[FS23][i]};
+        const double sigl[3] = {f[FL21][i], f[FL31][i], f[FL32][i]};
+        const Moment s = {f[FH][i], f[FMASS][i], f[FRHO][i], f[FQ][i], sig, sigl};
+        write_momentum<REC>(a, grid, p, a.ckey[p], f[FX][i], f[FY][i], f[FZ][i], s);
+        if (a.prm.boundary)
+            for (int q = a.ghost_of[i]; q >= 0; q = a.gnext[q]) write_ghost_momentum<REC>(a, q, s);
     }
 }
 
@@ -711,13 +779,14 @@ void launch_strain(const StepArgs &a, cudaStream_t s) {
 
 void launch_constitutive(const StepArgs &a, cudaStream_t s) {
     int blocks = nblk(a.n, kRedThreads);
-    const int wave = 148 * resident_per_sm((const void *)k_constitutive, kRedThreads);
+    void (*kern)(StepArgs) = a.frec0 ? k_constitutive<kRecMixed> : k_constitutive<kRecFP64>;
+    const int wave = 148 * resident_per_sm((const void *)kern, kRedThreads);
     if (blocks > wave) blocks = wave;
-    launch_chained(k_constitutive, blocks, kRedThreads, 0, s, a);
+    launch_chained(kern, blocks, kRedThreads, 0, s, a);
 }
 
 void launch_mom_prep(const StepArgs &a, cudaStream_t s) {
-    launch_chained(k_mom_prep, gs_blocks(a.n > a.ghost_cap ? a.n : a.ghost_cap), 256, 0, s, a);
+    launch_chained(a.frec0 ? k_mom_prep<kRecMixed> : k_mom_prep<kRecFP64>, gs_blocks(a.n), 256, 0, s, a);
 }
 
 void launch_rep_cont(const StepArgs &a, cudaStream_t s) { launch_chained(k_rep_cont, gs_blocks(a.n), 256, 0, s, a); }

@@ -64,28 +64,6 @@ __device__ __forceinline__ double lane_sum(float s, float c) {
 }
 
 // ------------------------------------------------------------ geometry
-struct Frame {
-    double gmin[3], cs[3];
-    float csf[3];
-    int gl[3];
-};
-__device__ __forceinline__ Frame make_frame(const DevGrid &g) {
-    Frame fr;
-    for (int d = 0; d < 3; ++d) {
-        fr.gmin[d] = g.gridmin[d];
-        fr.cs[d] = 1.0 / g.gridsize[d];
-        fr.csf[d] = (float)fr.cs[d];
-        fr.gl[d] = g.gridlim[d];
-    }
-    return fr;
-}
-__device__ __forceinline__ void frame_origin(const Frame &fr, int key, double o[3]) {
-    if (key < 0) { o[0] = o[1] = o[2] = 0.0; return; }
-    int b[3];
-    cell_coords(key, fr.gl, b[0], b[1], b[2]);
-    for (int d = 0; d < 3; ++d) o[d] = fr.gmin[d] + (double)(b[d] - 1) * fr.cs[d];
-}
-
 #ifndef MCM_STRAIN_UNROLL
 #define MCM_STRAIN_UNROLL 4
 #endif
@@ -111,10 +89,11 @@ struct Offsets3 {
     __device__ __forceinline__ void set(int c, float u, float v, float w) { x[c] = u; y[c] = v; z[c] = w; }
 };
 template <typename T>
-__device__ __forceinline__ void fill_offsets(T &tab, const Frame &fr) {
+__device__ __forceinline__ void fill_offsets(T &tab, const DevGrid &g) {
     const int c = threadIdx.x;
     if (c < 27)
-        tab.set(c, (float)(c % 3 - 1) * fr.csf[0], (float)((c / 3) % 3 - 1) * fr.csf[1], (float)(c / 9 - 1) * fr.csf[2]);
+        tab.set(c, (float)(c % 3 - 1) * (float)g.cell[0], (float)((c / 3) % 3 - 1) * (float)g.cell[1],
+                (float)(c / 9 - 1) * (float)g.cell[2]);
 }
 
 // Gather records.  A strain record is 32 bytes {x, y, z, h, vx, vy, vz, V}
@@ -248,9 +227,7 @@ __global__ void __launch_bounds__(256, 3) k_strain(StepArgs a) {
     const int sub = threadIdx.x / L, lane = threadIdx.x % L;
     const int per = blockDim.x / L;
     const int rounds = (a.n + per * gridDim.x - 1) / (per * gridDim.x);
-    const DevGrid g = *a.grid;
-    const Frame fr = make_frame(g);
-    fill_offsets(offs, fr);
+    fill_offsets(offs, *a.grid);
     __syncthreads();
     const double dt = a.time->dt;
     for (int round = 0; round < rounds; ++round) {
@@ -418,9 +395,7 @@ __global__ void __launch_bounds__(kStageThreads, 6) k_strain_staged(StepArgs a) 
     const int sub = threadIdx.x / L, lane = threadIdx.x % L;
     constexpr int per = kStageThreads / L;
     const int rounds = (a.n + per * gridDim.x - 1) / (per * gridDim.x);
-    const DevGrid g = *a.grid;
-    const Frame fr = make_frame(g);
-    fill_offsets(offs, fr);
+    fill_offsets(offs, *a.grid);
     const double dt = a.time->dt;
     for (int round = 0; round < rounds; ++round) {
         const int tb = (round * gridDim.x + blockIdx.x) * per;
@@ -501,52 +476,6 @@ __global__ void __launch_bounds__(kStageThreads, 6) k_strain_staged(StepArgs a) 
 // next to each other in every array.
 __device__ __forceinline__ float4 *mom_tail(const StepArgs &a) { return a.frec0 + 2 * (size_t)a.npad; }
 __device__ __forceinline__ float4 *mom_lower(const StepArgs &a) { return a.frec0 + 3 * (size_t)a.npad; }
-
-// --------------------------------------------------------- momentum prep
-// Records: cell-relative x, h; (sigma - q)/rho^2 (formed in FP64,
-// MCM/mcm_oldacceleration.f90:79-80) and m (FP32).  Ghosts: FP64 positions,
-// stresses with every off-diagonal negated (MCM/mcm_update_ghost_stress.f90:
-// 272-285) over the ghost's own density.
-__global__ void k_mom_prep(StepArgs a) {
-    chain_start();
-    if (skip_step(a)) return;
-    const Frame fr = make_frame(*a.grid);
-    const double *const *f = a.F.f;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x) {
-        const int i = a.cell_list[p];
-        double o[3];
-        frame_origin(fr, a.ckey[p], o);
-        const double rho = f[FRHO][i];
-        const double ir2 = 1.0 / (rho * rho);
-        const double q = f[FQ][i];
-        float4 *rec = a.frec0 + 2 * (size_t)p;
-        rec[0] = make_float4((float)(f[FX][i] - o[0]), (float)(f[FY][i] - o[1]), (float)(f[FZ][i] - o[2]),
-                             (float)f[FH][i]);
-        rec[1] = make_float4((float)((f[FS11][i] - q) * ir2), (float)((f[FS22][i] - q) * ir2),
-                                 (float)((f[FS33][i] - q) * ir2), (float)(f[FS12][i] * ir2));
-        mom_tail(a)[p] = make_float4((float)(f[FS13][i] * ir2), (float)(f[FS23][i] * ir2), (float)f[FMASS][i], (float)rho);
-        // the cap model's lower triangle (21 31 32), read only when a material has it
-        if (a.prm.asym)
-            mom_lower(a)[p] =
-                make_float4((float)(f[FL21][i] * ir2), (float)(f[FL31][i] * ir2), (float)(f[FL32][i] * ir2), 0.0f);
-    }
-    if (a.prm.boundary) {
-        const int ngp = *a.ngp;
-        for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ngp; g += gridDim.x * blockDim.x) {
-            const int j = a.gpar[g];
-            const double rho = a.grho[g];
-            const double ir2 = 1.0 / (rho * rho);
-            const double q = f[FQ][j];
-            a.grec0[g] = make_double4(a.gx[g], a.gy[g], a.gz[g], a.gh[g]);
-            a.gfrec1[g] = make_float4((float)((f[FS11][j] - q) * ir2), (float)((f[FS22][j] - q) * ir2),
-                                      (float)((f[FS33][j] - q) * ir2), (float)(-f[FS12][j] * ir2));
-            a.gfrec2[g] = make_float4((float)(-f[FS13][j] * ir2), (float)(-f[FS23][j] * ir2), (float)a.gmass[g],
-                                      (float)rho);
-            if (a.prm.asym)
-                a.grec3[g] = make_double4(-f[FL21][j] * ir2, -f[FL31][j] * ir2, -f[FL32][j] * ir2, 0.0);
-        }
-    }
-}
 
 __device__ __forceinline__ double block_sum(double v, double *sm) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -655,9 +584,7 @@ __global__ void __launch_bounds__(STAGED ? kStageThreads : 256, STAGED ? 4 : MCM
     const int sub = threadIdx.x / L, lane = threadIdx.x % L;
     const int per = blockDim.x / L;
     const int rounds = (a.n + per * gridDim.x - 1) / (per * gridDim.x);
-    const DevGrid g = *a.grid;
-    const Frame fr = make_frame(g);
-    fill_offsets(offs, fr);
+    fill_offsets(offs, *a.grid);
     __syncthreads();
     const int nm = a.nmat;
     constexpr bool asym = ASYM;   // the cap model: sigma's lower triangle in the record's 4th slot
@@ -861,12 +788,6 @@ void launch_strain(const StepArgs &a, cudaStream_t s) {
     } else {
         launch_chained(k_strain<false>, pair_blocks_of(a, L, (const void *)k_strain<false>), pair_threads_of(a), 0, s, a);
     }
-}
-
-void launch_mom_prep(const StepArgs &a, cudaStream_t s) {
-    int n = a.n > a.ghost_cap ? a.n : a.ghost_cap;
-    int b = nblk(n, 256);
-    launch_chained(k_mom_prep, b < 148 * 16 ? b : 148 * 16, 256, 0, s, a);
 }
 
 int launch_momentum(const StepArgs &a, cudaStream_t s, int integrate_flag) {
