@@ -650,10 +650,12 @@ int mcm_gpu_create(const mcm_gpu_config *cfg, const mcm_gpu_material *mats, int 
     if (cfg->tcrit_opt < 0 || cfg->tcrit_opt > 2) return MCM_EINVAL;
     if (cfg->precision < 0 || cfg->precision > 2) return MCM_EINVAL;
     bool cap_model = false;
+    int model = mats[0].model;
     for (int m = 0; m < nmat; ++m) {
         int md = mats[m].model;
         if (md != 1 && md != 3 && md != 4 && md != 9 && md != 10) return MCM_EINVAL;
         cap_model = cap_model || md == 4;
+        if (md != model) model = 0;
     }
     // the cap model leaves sigma asymmetric: the simple-SPH momentum sums of
     // every precision read both triangles; the corrected-SPH sum carries 6 components
@@ -684,6 +686,7 @@ int mcm_gpu_create(const mcm_gpu_config *cfg, const mcm_gpu_material *mats, int 
     h->A.n = np;
     h->A.npad = h->npad;
     h->A.nmat = nmat;
+    h->A.model = model;
     h->A.split_mode = 1;
     h->A.share = 1;
     h->A.prm = make_params(h->cfg, nmat);

@@ -411,7 +411,7 @@ __device__ __forceinline__ void constitutive_pass(int pass, const StepArgs &a, c
     P.etry = D(0.0); P.einc = D(0.0); P.rhoold = P.rho;
     const D dt = D(b.dt_prev);
     rhoupd(P, M, dt, 3);
-    constitutive_particle(P, M, dt);
+    constitutive_particle(P, M, dt, M.model);
 #pragma unroll
     for (int k = 0; k < kND; ++k) {
         const int s = pass * kND + k;

@@ -10,6 +10,7 @@ struct StepArgs {
     int n;            // particles
     int npad;         // column pitch of per-particle arrays (multiple of 32)
     int nmat;
+    int model;        // the constitutive model of every material, 0 if they differ
     int nstride;      // neighbour-list capacity per position (entries, multiple of 4)
     int gstride;      // ghost-neighbour table width (int32 entries)
     int ghost_cap;    // ghost storage

@@ -1024,9 +1024,9 @@ __device__ __forceinline__ T critts_particle(const PState<T> &P, const Mat &M, i
 // Returns 0, MCM_ECOMPLEX_C (the EOS reported a complex sound speed) or
 // MCM_ECAP_NOCONV (the cap model's iterated return did not converge).
 template <typename T, typename Mat>
-__device__ __forceinline__ int constitutive_particle(PState<T> &P, const Mat &M, T dt) {
+__device__ __forceinline__ int constitutive_particle(PState<T> &P, const Mat &M, T dt, int model) {
     int code = 0;
-    switch (M.model) {
+    switch (model) {
         case 1:
             stress_rot1(P, dt); f3dm1(P, M, dt); sym_lower(P); aviscosity(P, M); lieupd(P, dt);
             break;

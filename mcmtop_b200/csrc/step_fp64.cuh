@@ -146,8 +146,7 @@ __device__ __forceinline__ void load_state(const StepArgs &a, int i, PState<doub
 
 __device__ __forceinline__ void store_state(const StepArgs &a, int i, const PState<double> &P, int model) {
     double *const *f = a.F.f;
-    f[FH][i] = P.h;
-    if (a.prm.h_opt) f[FHOLD][i] = P.hold;
+    if (a.prm.h_opt) { f[FH][i] = P.h; f[FHOLD][i] = P.hold; }
     f[FRHO][i] = P.rho; f[FE][i] = P.e; f[FP][i] = P.p; f[FC][i] = P.c;
     f[FEFPS][i] = P.efps; f[FPCUT][i] = P.pcut; f[FPCUT2][i] = P.p_cut; f[FFAIL][i] = P.fail;
 #pragma unroll
@@ -270,20 +269,22 @@ __device__ __forceinline__ void update_h(const StepArgs &a, int i, PState<double
 // MCM/mcm_rhoupd.f90, mcm_constitutive.f90:29-83 and mcm_calccritts.f90 for
 // the particle with state index i, and the forward half-step shift of
 // MCM/mcm_strain.f90:56-60 (x - v dt/2 recomputed as the strain records have it).
-// Two resident blocks per SM (128 registers, a few hundred bytes of spills)
-// measured faster than one at 154 registers: 0.27 against 0.43 ms per step
-// on the 2M bar.
+// MODEL: the model of every material, 0 if they differ or it is none of those
+// with an instance of their own.  All models in one kernel need 164 registers,
+// most of them for the cap model's call; two resident blocks per SM (128
+// registers, spills) measured faster than one.  Model 9 or 10 alone, 140
+// registers and no loads of what they do not read, run three blocks per SM (80
+// registers).  685 824 particles, all models / one with two blocks / one with
+// three: 123 / 101 / 98 us (mixed), 132 / 112 / 102 us (FP64), and 38 880 mixed
+// 20 / 19 / 19.
 //
 // Writes the momentum gather's records of the particle, at its position in cell
 // order, and of its ghosts too: whole 32-byte sectors, while the state they are
-// made of is in registers.  685 824 particles, this kernel and a kernel of its
-// own for the records: 105 + 33 us (mixed), 105 + 43 (FP64); as one 123 and
-// 132.  16 848: 18 + 11 and 20.
-#ifndef MCM_CONST_MINBLOCKS
-#define MCM_CONST_MINBLOCKS 2
-#endif
-template <int REC>
-__global__ void __launch_bounds__(kRedThreads, MCM_CONST_MINBLOCKS) k_constitutive(StepArgs a) {
+// made of is in registers.  685 824 particles, this kernel (all models) and a
+// kernel of its own for the records: 105 + 33 us (mixed), 105 + 43 (FP64); as
+// one 123 and 132.  16 848: 18 + 11 and 20.
+template <int REC, int MODEL>
+__global__ void __launch_bounds__(kRedThreads, MODEL ? 3 : 2) k_constitutive(StepArgs a) {
     chain_wait();
     __shared__ double sm[32];
     __shared__ DevGrid g;
@@ -298,8 +299,9 @@ __global__ void __launch_bounds__(kRedThreads, MCM_CONST_MINBLOCKS) k_constituti
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
         double *const *f = a.F.f;
         const DevMaterial &M = a.mats[a.F.mat[i] - 1];
+        const int model = MODEL ? MODEL : M.model;
         PState<double> P;
-        load_state(a, i, P, M.model);
+        load_state(a, i, P, model);
 #pragma unroll
         for (int u = 0; u < 6; ++u) P.rod[u] = f[FR11 + u][i];
         P.spin[0] = f[FW12][i];
@@ -308,13 +310,13 @@ __global__ void __launch_bounds__(kRedThreads, MCM_CONST_MINBLOCKS) k_constituti
         P.tracerod = f[FTR][i];
         if (a.prm.h_opt) update_h(a, i, P, dt);
         rhoupd(P, M, dt, 3);
-        const int bad = constitutive_particle(P, M, dt);
+        const int bad = constitutive_particle(P, M, dt, model);
         if (bad) raise_status(a.status, bad, i);
         const double vx = f[FVX][i], vy = f[FVY][i], vz = f[FVZ][i];
         const double mindist = (a.prm.tcrit_opt == 2) ? f[FMINDIST][i] : 0.0;
         const double own = critts_particle(P, M, a.prm.tcrit_opt, 3, f[FVABS][i], mindist);
         crit = fmin(crit, own);
-        store_state(a, i, P, M.model);
+        store_state(a, i, P, model);
         if (a.prm.diag) f[FCRITTS][i] = own;
         const double xs = f[FX][i] - 0.5 * vx * dt;
         const double ys = f[FY][i] - 0.5 * vy * dt;
@@ -777,9 +779,18 @@ void launch_strain(const StepArgs &a, cudaStream_t s) {
 #endif
 }
 
+template <int REC>
+static void (*constitutive_kernel(const StepArgs &a))(StepArgs) {
+    switch (a.model) {
+        case 9: return k_constitutive<REC, 9>;
+        case 10: return k_constitutive<REC, 10>;
+        default: return k_constitutive<REC, 0>;
+    }
+}
+
 void launch_constitutive(const StepArgs &a, cudaStream_t s) {
     int blocks = nblk(a.n, kRedThreads);
-    void (*kern)(StepArgs) = a.frec0 ? k_constitutive<kRecMixed> : k_constitutive<kRecFP64>;
+    void (*kern)(StepArgs) = a.frec0 ? constitutive_kernel<kRecMixed>(a) : constitutive_kernel<kRecFP64>(a);
     const int wave = 148 * resident_per_sm((const void *)kern, kRedThreads);
     if (blocks > wave) blocks = wave;
     launch_chained(kern, blocks, kRedThreads, 0, s, a);
