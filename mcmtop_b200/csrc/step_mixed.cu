@@ -27,7 +27,7 @@
 // The error is that of the FP32 pair terms rather than of their sum, and the
 // Kahan registers cost occupancy, so the lanes sum plainly.  Two lanes (about
 // 40 neighbours in flight per lane, one shuffle level) hide the record-gather
-// latency best: strain/momentum 0.78/1.11 ms per step.
+// latency best (now 0.62/0.81 ms per step of that bar).
 #include "nbr_iter.cuh"
 
 namespace mcm {
