@@ -87,8 +87,10 @@ __global__ void __launch_bounds__(256) k_cell_keys(StepArgs a) {
     chain_start();
     __shared__ DevGrid g;
     __shared__ int stop;
-    if (a.status->code) return;
-    if (threadIdx.x == 0) {
+    // block 0 raises the status in this launch, so only thread 0 reads it: the
+    // block stops or goes on as a whole
+    if (threadIdx.x == 0) stop = a.status->code;
+    if (threadIdx.x == 0 && !stop) {
         const bool bad = make_grid(a, g);
         stop = (bad || g.ncells >= (1LL << 31)) ? MCM_EGRID_TOO_LARGE : g.ncells > a.cell_cap ? MCM_EGRID_OVERFLOW : 0;
         if (blockIdx.x == 0) {
@@ -565,7 +567,8 @@ __global__ void __launch_bounds__(kScanThreads) k_ghost_count(StepArgs a) {
     chain_start();
     __shared__ int smem[32];
     __shared__ int last;
-    if (a.status->code && a.status->code != MCM_EGHOST_LAYER) return;   // EGHOST_LAYER may be this launch's own
+    // EGHOST_LAYER may be this launch's own
+    if (__syncthreads_or(a.status->code && a.status->code != MCM_EGHOST_LAYER)) return;
     const Layers l = make_layers(a);
     const int T = l.first[6];
     if (T < 0 || T > a.layer_cap) {
