@@ -288,11 +288,9 @@ __global__ void __launch_bounds__(kRedThreads, MODEL ? 3 : 2) k_constitutive(Ste
     chain_wait();
     __shared__ double sm[32];
     __shared__ DevGrid g;
-    if (skip_step(a)) return;
-    if (REC == kRecMixed) {
-        if (threadIdx.x == 0) g = *a.grid;
-        __syncthreads();
-    }
+    if (REC == kRecMixed && threadIdx.x == 0) g = *a.grid;
+    // other blocks may raise the status in this launch: the block leaves as a whole
+    if (__syncthreads_or(skip_step(a))) return;
     const double dt = a.time->dt;
     double crit = 1.0e20;
 #pragma unroll 1

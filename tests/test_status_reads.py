@@ -62,3 +62,7 @@ def test_the_reading_finds_kernels():
 
 def test_cell_and_ghost_kernels_leave_as_blocks():
     assert offenders("cells.cu") == []
+
+
+def test_every_kernel_leaves_as_blocks():
+    assert offenders(*os.listdir(CSRC)) == []
