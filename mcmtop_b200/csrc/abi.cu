@@ -170,9 +170,9 @@ int alloc_cells(mcm_gpu_handle *h, long long cap) {
     long long nsum = (cap + 4095) / 4096 + 2;
     if ((st = dalloc(h, &h->A.scan_sums, (size_t)nsum))) return st;
     if ((st = dalloc(h, &h->A.gcell, (size_t)cap))) return st;
-    // the planes' layers (a grid all of whose cells lie near planes may need more: the arrays grow then)
-    h->A.layer_cap = h->A.prm.boundary ? (int)std::min<long long>(cap, 1LL << 30) : 1;
-    if ((st = dalloc(h, &h->A.layer_count, 2 * (size_t)h->A.layer_cap + (size_t)h->A.layer_cap / 4096 + 2))) return st;
+    // the planes' layers hold at most twice the grid's cells (a grid has less than 2^31)
+    h->A.layer_cap = h->A.prm.boundary ? (unsigned)std::min<long long>(2 * cap, (1LL << 32) - 1) : 1u;
+    if ((st = dalloc(h, &h->A.layer_count, 2 * (size_t)h->A.layer_cap + scan_chunks(h->A.layer_cap) + 1))) return st;
     h->A.layer_off = h->A.layer_count + h->A.layer_cap;
     h->A.layer_sums = h->A.layer_off + h->A.layer_cap;
     return MCM_OK;

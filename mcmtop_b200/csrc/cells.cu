@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) k_cell_keys(StepArgs a) {
     __syncthreads();
     if (stop) return;
     if (a.prm.boundary)
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < (int)g.ncells; c += gridDim.x * blockDim.x)
+        for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < (unsigned)g.ncells; c += gridDim.x * blockDim.x)
             a.gcell[c] = make_int2(0, 0);
     const int ndim = a.prm.ndim;
     const double *X[3] = {a.F.f[FX], a.F.f[FY], a.F.f[FZ]};
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(256) k_cell_keys(StepArgs a) {
 // arrays have grown).
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
-constexpr int kScanChunk = kScanThreads * kScanItems;
+static_assert(kScanChunk == kScanThreads * kScanItems, "a chunk per block");
 
 __device__ __forceinline__ int block_exclusive_scan(int v, int *smem, int &total) {
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -174,10 +174,10 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(StepArgs a) {
     __shared__ int smem[32];
     __shared__ int last;
     if (a.status->code) return;
-    const int n = (int)a.grid->ncells;
-    const int nblocks = (n + kScanChunk - 1) / kScanChunk;
+    const unsigned n = (unsigned)a.grid->ncells;
+    const int nblocks = scan_chunks(n);
     if ((int)blockIdx.x >= nblocks) return;
-    const int base = blockIdx.x * kScanChunk + threadIdx.x * kScanItems;
+    const unsigned base = blockIdx.x * kScanChunk + threadIdx.x * kScanItems;
     int v[kScanItems];
     int local = 0;
 #pragma unroll
@@ -218,9 +218,9 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(StepArgs a) {
 __global__ void __launch_bounds__(256) k_cell_scatter(StepArgs a) {
     chain_start();
     if (a.status->code) return;
-    const int ncells = (int)a.grid->ncells;
-    const int base_out = a.scan_sums[(ncells + kScanChunk - 1) / kScanChunk];
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncells; c += gridDim.x * blockDim.x)
+    const unsigned ncells = (unsigned)a.grid->ncells;
+    const int base_out = a.scan_sums[scan_chunks(ncells)];
+    for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncells; c += gridDim.x * blockDim.x)
         a.cell_start[c] = c < ncells ? a.cell_local[c] + a.scan_sums[c / kScanChunk] : base_out;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
         int key = a.key[i];
@@ -312,12 +312,12 @@ __global__ void __launch_bounds__(256) k_cell_order(StepArgs a, int with_cposf) 
     if (a.status->code) return;
     if (threadIdx.x == 0) g = *a.grid;
     __syncthreads();
-    const int ncells = (int)g.ncells;
+    const unsigned ncells = (unsigned)g.ncells;
     const double dt = a.time->dt;
     const int lane = threadIdx.x & 31;
-    const int nw = gridDim.x * (blockDim.x >> 5);
+    const unsigned nw = gridDim.x * (blockDim.x >> 5);
     unsigned long long hbits = 0ull, lbits = ~0ull;
-    for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += nw) {
+    for (unsigned c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += nw) {
         const int s = a.cell_start[c], e = a.cell_start[c + 1];
         const int n = e - s;
         if (n <= 32) {
@@ -474,7 +474,7 @@ void launch_reorder(const StepArgs &a, cudaStream_t s) {
 
 // The layer cells of the active planes, plane after plane.
 struct Layers {
-    int first[7];   // of each plane's cells in the sequence
+    unsigned first[7];   // of each plane's cells in the sequence
     int gl[3];
 };
 __device__ __forceinline__ bool plane_active(const StepArgs &a, int plane) {
@@ -484,13 +484,10 @@ __device__ __forceinline__ bool plane_active(const StepArgs &a, int plane) {
 __device__ __forceinline__ Layers make_layers(const StepArgs &a) {
     Layers l;
     for (int d = 0; d < 3; ++d) l.gl[d] = a.grid->gridlim[d];
-    l.first[0] = 0;
+    unsigned active = 0u;
 #pragma unroll
-    for (int p = 0; p < 6; ++p) {
-        const int d = p >> 1;
-        const int area = l.gl[d == 0 ? 1 : 0] * l.gl[d == 2 ? 1 : 2];   // below 2^31 / 2: an active axis has two layers
-        l.first[p + 1] = l.first[p] + (plane_active(a, p) ? area : 0);
-    }
+    for (int p = 0; p < 6; ++p) active |= plane_active(a, p) ? 1u << p : 0u;
+    layer_starts(l.gl, active, l.first);
     return l;
 }
 __device__ __forceinline__ int layer_key(const Layers &l, const int *c) {
@@ -508,14 +505,14 @@ __device__ __forceinline__ int source_layer(const StepArgs &a, const Layers &l, 
 struct Origin {
     int from, to, count, depth, planes[3];
 };
-__device__ __forceinline__ Origin origin_of(const StepArgs &a, const Layers &l, int t) {
+__device__ __forceinline__ Origin origin_of(const StepArgs &a, const Layers &l, unsigned t) {
     int plane = 0;
 #pragma unroll
     for (int p = 1; p < 6; ++p)
         if (t >= l.first[p]) plane = p;
     const int d = plane >> 1, side = plane & 1;
     const int ad = d == 2 ? 1 : 2, bd = d == 0 ? 1 : 0;   // the layer's outer and inner axis
-    const int r = t - l.first[plane];
+    const int r = (int)(t - l.first[plane]);   // a layer has less than 2^31 cells
     const int nb = l.gl[bd];
     int c[3];
     c[ad] = r / nb + 1;
@@ -570,19 +567,19 @@ __global__ void __launch_bounds__(kScanThreads) k_ghost_count(StepArgs a) {
     // EGHOST_LAYER may be this launch's own
     if (__syncthreads_or(a.status->code && a.status->code != MCM_EGHOST_LAYER)) return;
     const Layers l = make_layers(a);
-    const int T = l.first[6];
-    if (T < 0 || T > a.layer_cap) {
+    const unsigned T = l.first[6];
+    if (T > a.layer_cap) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_status(a.status, MCM_EGRID_OVERFLOW);
         return;
     }
-    const int base = blockIdx.x * kScanChunk;
-    const int nblocks = (T + kScanChunk - 1) / kScanChunk;   // blocks that hold layer cells
+    const unsigned base = blockIdx.x * kScanChunk;
+    const int nblocks = scan_chunks(T);   // blocks that hold layer cells
     if ((int)blockIdx.x >= nblocks) return;
     int v[kScanItems];
     int local = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        const int t = base + threadIdx.x * kScanItems + k;
+        const unsigned t = base + threadIdx.x * kScanItems + k;
         v[k] = t < T ? origin_of(a, l, t).count : 0;
         local += v[k];
     }
@@ -590,7 +587,7 @@ __global__ void __launch_bounds__(kScanThreads) k_ghost_count(StepArgs a) {
     int pre = block_exclusive_scan(local, smem, total);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        const int t = base + threadIdx.x * kScanItems + k;
+        const unsigned t = base + threadIdx.x * kScanItems + k;
         if (t < T) {
             a.layer_count[t] = v[k];
             a.layer_off[t] = pre;
@@ -632,10 +629,10 @@ __global__ void k_ghost_emit(StepArgs a) {
     chain_start();
     if (a.status->code) return;
     const Layers l = make_layers(a);
-    const int T = l.first[6];
+    const unsigned T = l.first[6];
     const int lane = threadIdx.x & 31;
-    const int nw = gridDim.x * (blockDim.x >> 5);
-    for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < T; t += nw) {
+    const unsigned nw = gridDim.x * (blockDim.x >> 5);
+    for (unsigned t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < T; t += nw) {
         const int cnt = a.layer_count[t];
         if (cnt == 0) continue;
         const Origin o = origin_of(a, l, t);
@@ -688,7 +685,7 @@ __global__ void k_ghost_emit(StepArgs a) {
 }
 
 void launch_ghosts(const StepArgs &a, cudaStream_t s) {
-    launch_chained(k_ghost_count, (unsigned)((a.layer_cap + kScanChunk - 1) / kScanChunk), kScanThreads, 0, s, a);
+    launch_chained(k_ghost_count, scan_chunks(a.layer_cap), kScanThreads, 0, s, a);
     long long eb = ((long long)a.layer_cap + 7) / 8;   // 8 warps (layer cells) per block
     if (eb > 148LL * 4) eb = 148LL * 4;
     launch_chained(k_ghost_emit, (unsigned)(eb < 1 ? 1 : eb), 256, 0, s, a);

@@ -111,6 +111,24 @@ __host__ __device__ inline long long cell_key(int bx, int by, int bz, const int 
     return (long long)(bx - 1) + (long long)gl[0] * ((long long)(by - 1) + (long long)gl[1] * (long long)(bz - 1));
 }
 
+// The grid check lets up to 2^31 - 1 cells through, and their planes' layers
+// hold up to twice as many (an axis with a plane has at least two cells, one
+// with two planes three): counts of either are unsigned, so that no index or
+// loop counter that steps past them wraps.
+constexpr unsigned kScanChunk = 4096;   // cells or layer cells per block of their scans
+__host__ __device__ inline unsigned scan_chunks(unsigned n) { return n / kScanChunk + (n % kScanChunk ? 1u : 0u); }
+// The layer cells of the planes in `active` (bit 2 * axis + side), plane after
+// plane: first[p] is where plane p's begin, first[6] their number.
+__host__ __device__ inline void layer_starts(const int *gl, unsigned active, unsigned *first) {
+    first[0] = 0;
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+        const int d = p >> 1;
+        const unsigned area = (unsigned)gl[d == 0 ? 1 : 0] * (unsigned)gl[d == 2 ? 1 : 2];
+        first[p + 1] = first[p] + ((active >> p & 1u) ? area : 0u);
+    }
+}
+
 // Lower corner of cell b (1-based) along axis d of the grid.
 __host__ __device__ inline double cell_origin(const DevGrid &g, int d, int b) {
     return g.gridmin[d] + (double)(b - 1) * g.cell[d];

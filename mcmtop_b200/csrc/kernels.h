@@ -15,7 +15,7 @@ struct StepArgs {
     int gstride;      // ghost-neighbour table width (int32 entries)
     int ghost_cap;    // ghost storage
     long long cell_cap;   // cell-array storage
-    int layer_cap;    // scratch for the planes' layer cells
+    unsigned layer_cap;   // scratch for the planes' layer cells
     int share;        // bodies of this one's size that run on the GPU at the same time (a batch's lanes)
     int split_mode;   // 1: step_a/b/c entry points (dt supplied by the host); 0: fused run
     DevParams prm;
