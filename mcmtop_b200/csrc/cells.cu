@@ -501,7 +501,15 @@ __device__ __forceinline__ int source_layer(const StepArgs &a, const Layers &l, 
 
 // Where layer cell t's ghosts come from: the real particles of cell `from`,
 // mirrored through planes[depth - 1], ..., planes[0] in turn; `to` receives
-// them.  Reals in a cell that also receives ghosts raise MCM_EGHOST_LAYER.
+// them.
+//
+// The source cell may lie in the layers of earlier axes; it then holds the
+// ghosts of the last of them whose own source held anything, and so on down.
+// With one hop per such axis, from the layer to the cell it mirrors, what the
+// cell holds are the reals of the one cell of {no hop, first axis, second axis,
+// both} that has any.  Two that have some mean that a cell holds both reals and
+// ghosts, or the ghosts of two planes, and so does one of the four around `to`
+// when it receives any: MCM_EGHOST_LAYER.
 struct Origin {
     int from, to, count, depth, planes[3];
 };
@@ -521,40 +529,46 @@ __device__ __forceinline__ Origin origin_of(const StepArgs &a, const Layers &l, 
     c[d] = side == 0 ? 1 : l.gl[d];
     o.to = layer_key(l, c);
     c[d] = source_layer(a, l, d, side);
-    o.depth = 1;
-    o.planes[0] = plane;
-    o.count = 0;
-    bool found = false, mixed = false;
-    // down through the earlier planes whose layer the cell lies in
+    const int source = layer_key(l, c);
+    unsigned in = 0u;          // earlier axes along which the cell lies in a layer
+    int hop[2] = {0, 0}, via[2] = {0, 0};
 #pragma unroll
-    for (int e = 2; e >= 0; --e) {
+    for (int e = 0; e < 2; ++e) {
         if (e >= d) continue;
         const int es = c[e] == 1 && plane_active(a, 2 * e) ? 0 : (c[e] == l.gl[e] && plane_active(a, 2 * e + 1) ? 1 : -1);
         if (es < 0) continue;
-        const int k = layer_key(l, c);
-        const int n = a.cell_start[k + 1] - a.cell_start[k];
-        if (n > 0 && !found) {   // reals in a layer cell: they are what is mirrored
-            o.from = k;
-            o.count = n;
-            found = true;
-        }
-        c[e] = source_layer(a, l, e, es);
-        if (!found) {
-            if (o.depth == 1) o.planes[1] = 2 * e + es;
-            else o.planes[2] = 2 * e + es;
-            ++o.depth;
-        }
+        in |= 1u << e;
+        via[e] = 2 * e + es;
+        hop[e] = (source_layer(a, l, e, es) - c[e]) * (e == 0 ? 1 : l.gl[0]);
     }
-    const int k = layer_key(l, c);
-    const int n = a.cell_start[k + 1] - a.cell_start[k];
-    if (found) {
-        mixed = n > 0;
-    } else {
+    o.from = source;
+    o.count = 0;
+    unsigned taken = 0u;
+    bool clash = false;
+#pragma unroll
+    for (unsigned m = 0u; m < 4u; ++m) {
+        if (m & ~in) continue;
+        const int k = source + (m & 1u ? hop[0] : 0) + (m & 2u ? hop[1] : 0);
+        const int n = a.cell_start[k + 1] - a.cell_start[k];
+        if (n == 0) continue;
+        clash = clash || o.count > 0;
         o.from = k;
         o.count = n;
+        taken = m;
     }
-    if (o.count > 0 && (mixed || a.cell_start[o.to + 1] > a.cell_start[o.to]))
-        raise_status(a.status, MCM_EGHOST_LAYER, mixed ? o.from : o.to);
+    if (o.count > 0) {
+#pragma unroll
+        for (unsigned m = 0u; m < 4u; ++m) {
+            if (m & ~in) continue;
+            const int k = o.to + (m & 1u ? hop[0] : 0) + (m & 2u ? hop[1] : 0);
+            clash = clash || a.cell_start[k + 1] > a.cell_start[k];
+        }
+        if (clash) raise_status(a.status, MCM_EGHOST_LAYER, o.to);
+    }
+    o.depth = 1 + __popc(taken);
+    o.planes[0] = plane;
+    o.planes[1] = taken & 2u ? via[1] : via[0];
+    o.planes[2] = via[0];
     return o;
 }
 
