@@ -19,7 +19,10 @@
 namespace mcm {
 
 // ------------------------------------------------------------- grid set-up
-// MCM/mcm_setuplist.f90:30-81; true when a span has no finite cell count.
+// MCM/mcm_setuplist.f90:30-81; true when a span has no finite cell count (no
+// particle with a finite position leaves the box at 1e20 to -1e20).  A box that
+// lies wholly beyond a plane gives an axis less than one cell: such a grid has
+// none.
 __device__ __forceinline__ bool make_grid(const StepArgs &a, DevGrid &g) {
     const DevParams &P = a.prm;
     const double factor = 2.0;
@@ -36,25 +39,25 @@ __device__ __forceinline__ bool make_grid(const StepArgs &a, DevGrid &g) {
             case 1:
                 g.gridmin[i] = a.bbox[i] - 0.01 * hmax;
                 span = g.gridsize[i] * (a.bbox[3 + i] - g.gridmin[i]);
-                if (!(span < 1.0e9)) { bad = true; span = 0; }
+                if (!(fabs(span) < 1.0e9)) { bad = true; span = 0; }
                 g.gridlim[i] = (int)span + 1;
                 break;
             case 2:
                 g.gridmin[i] = P.planes.bx[0][i];
                 span = g.gridsize[i] * (a.bbox[3 + i] - g.gridmin[i]);
-                if (!(span < 1.0e9)) { bad = true; span = 0; }
+                if (!(fabs(span) < 1.0e9)) { bad = true; span = 0; }
                 g.gridlim[i] = (int)span + 1;
                 break;
             case 3:
                 span = g.gridsize[i] * (P.planes.bx[1][i] - a.bbox[i]);
-                if (!(span < 1.0e9)) { bad = true; span = 0; }
+                if (!(fabs(span) < 1.0e9)) { bad = true; span = 0; }
                 g.gridlim[i] = (int)span + 1;
                 g.gridmin[i] = P.planes.bx[1][i] - g.gridlim[i] * factor * hmax;
                 break;
             case 4:
                 g.gridmin[i] = P.planes.bx[0][i];
                 span = g.gridsize[i] * (P.planes.bx[1][i] - P.planes.bx[0][i]);
-                if (!(span < 1.0e9)) { bad = true; span = 0; }
+                if (!(fabs(span) < 1.0e9)) { bad = true; span = 0; }
                 g.gridlim[i] = (int)span;
                 g.gridlim[i] = g.gridlim[i] > 1 ? g.gridlim[i] : 1;
                 g.gridsize[i] = (double)(float)g.gridlim[i] / (P.planes.bx[1][i] - P.planes.bx[0][i]);
@@ -72,7 +75,11 @@ __device__ __forceinline__ bool make_grid(const StepArgs &a, DevGrid &g) {
     }
     g.pad = 0;
     for (int i = 0; i < 3; ++i) g.cell[i] = 1.0 / g.gridsize[i];
-    g.ncells = (long long)g.gridlim[0] * g.gridlim[1] * g.gridlim[2];
+    g.ncells = 1;   // held at 2^31, which is too many: three axes of 10^9 would wrap
+    for (int i = 0; i < 3; ++i) {
+        g.ncells = g.gridlim[i] < 1 ? 0 : g.ncells * g.gridlim[i];
+        if (g.ncells > (1LL << 31)) g.ncells = 1LL << 31;
+    }
     g.hcut = 0.0;                                          // raised by k_cell_order
     g.hmin = __longlong_as_double(0x7fffffffffffffffll);   // lowered by k_cell_order
     return bad;
@@ -176,6 +183,7 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(StepArgs a) {
     if (a.status->code) return;
     const unsigned n = (unsigned)a.grid->ncells;
     const int nblocks = scan_chunks(n);
+    if (n == 0 && blockIdx.x == 0 && threadIdx.x == 0) a.scan_sums[0] = 0;
     if ((int)blockIdx.x >= nblocks) return;
     const unsigned base = blockIdx.x * kScanChunk + threadIdx.x * kScanItems;
     int v[kScanItems];
@@ -475,19 +483,20 @@ void launch_reorder(const StepArgs &a, cudaStream_t s) {
 // The layer cells of the active planes, plane after plane.
 struct Layers {
     unsigned first[7];   // of each plane's cells in the sequence
+    unsigned active;     // bit 2 * axis + side
     int gl[3];
 };
-__device__ __forceinline__ bool plane_active(const StepArgs &a, int plane) {
-    const int code = a.prm.planes.code[plane & 1][plane >> 1];
-    return (code == 1 || code == 2) && (plane >> 1) < a.prm.ndim;
-}
 __device__ __forceinline__ Layers make_layers(const StepArgs &a) {
     Layers l;
     for (int d = 0; d < 3; ++d) l.gl[d] = a.grid->gridlim[d];
-    unsigned active = 0u;
+    l.active = 0u;
+    // an axis of one cell has no layer to mirror; a grid without cells has none
 #pragma unroll
-    for (int p = 0; p < 6; ++p) active |= plane_active(a, p) ? 1u << p : 0u;
-    layer_starts(l.gl, active, l.first);
+    for (int p = 0; p < 6; ++p) {
+        const int code = a.prm.planes.code[p & 1][p >> 1];
+        if ((code == 1 || code == 2) && (p >> 1) < a.prm.ndim && l.gl[p >> 1] > 1 && a.grid->ncells > 0) l.active |= 1u << p;
+    }
+    layer_starts(l.gl, l.active, l.first);
     return l;
 }
 __device__ __forceinline__ int layer_key(const Layers &l, const int *c) {
@@ -535,7 +544,7 @@ __device__ __forceinline__ Origin origin_of(const StepArgs &a, const Layers &l, 
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
         if (e >= d) continue;
-        const int es = c[e] == 1 && plane_active(a, 2 * e) ? 0 : (c[e] == l.gl[e] && plane_active(a, 2 * e + 1) ? 1 : -1);
+        const int es = c[e] == 1 && (l.active >> (2 * e) & 1u) ? 0 : (c[e] == l.gl[e] && (l.active >> (2 * e + 1) & 1u) ? 1 : -1);
         if (es < 0) continue;
         in |= 1u << e;
         via[e] = 2 * e + es;
