@@ -895,6 +895,8 @@ int run_search_only(mcm_gpu_handle *h) {
 int finish_upload(mcm_gpu_handle *h, const double *coord_maxmin) {
     int st;
     k_iota<<<256, 256, 0, h->stream>>>(h->A.F.orig, h->np);
+    // the box below is not formed while an error is raised or the run has ended
+    CK(cudaMemsetAsync(&h->A.time->ended, 0, sizeof(int), h->stream));
     const double hm[2] = {h->A.prm.hmax, 0.0};
     CK(cudaMemcpyAsync(h->A.hmax, hm, sizeof(hm), cudaMemcpyHostToDevice, h->stream));
     if (coord_maxmin) {
@@ -948,6 +950,7 @@ int mcm_gpu_upload(mcm_gpu_handle *h, const mcm_gpu_fields *f, const double *coo
     if (f->dispbc) CK(scopy(h, h->A.F.dispbc, f->dispbc, sizeof(int) * n, cudaMemcpyHostToDevice));
     else CK(cudaMemsetAsync(h->A.F.dispbc, 0, sizeof(int) * n, h->stream));
     if (f->ptype) CK(scopy(h, h->A.F.ptype, f->ptype, sizeof(int) * n, cudaMemcpyHostToDevice));
+    if ((st = reset_status(h))) return st;   // of the state before this one
     return finish_upload(h, coord_maxmin);
 }
 
