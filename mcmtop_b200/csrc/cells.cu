@@ -786,10 +786,7 @@ __device__ __forceinline__ Seeker make_seeker(const StepArgs &a, const DevGrid &
     k.uy = -a.sny[t];
     k.uz = -a.snz[t];
     k.ux = (float)(k.xi.x - cell_origin(g, 0, k.bx));
-    // With u = 2^-24 the coordinates, their differences and the sum of squares
-    // round by less than (4 gridlim(1) + 30) u cell^2 and the cutoff by 5 u of
-    // itself: the band is 4 and 8 times that.
-    k.kb = (1.52587890625e-5f + (float)g.gridlim[0] * 9.5367431640625e-7f) * csm * csm;
+    k.kb = search_band(g.gridlim[0], csm);
     const float reach = k.hi + (float)g.hcut;
     k.reach2 = reach * reach * 1.0009765625f + 9.765625e-4f * csm * csm;
     k.uni = g.hmin == g.hcut;

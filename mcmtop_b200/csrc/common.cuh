@@ -134,6 +134,18 @@ __host__ __device__ inline double cell_origin(const DevGrid &g, int d, int b) {
     return g.gridmin[d] + (double)(b - 1) * g.cell[d];
 }
 
+// Half-width of the band around the cutoff within which the search's FP32
+// distances do not decide.  With u = 2^-24 and N cells of size cell along x,
+// whose coordinates are relative to the grid's origin, two of them differ from
+// the true difference by e = 2 N u cell at most: the squared distance is off by
+// less than (2 e / cell + (e / cell)^2 + 30 u) cell^2, and the cutoff by 5 u of
+// itself.  The band is 4 times the terms in e (16 in e^2, which counts from
+// some 10^7 cells on) and 8 times the rest.
+__host__ __device__ inline float search_band(int n, float cell) {
+    const float e4 = (float)n * 4.76837158203125e-7f;   // 4 e / cell
+    return (1.52587890625e-5f + 2.0f * e4 + e4 * e4) * cell * cell;
+}
+
 // First statement of every kernel of the step's chain (launch_chained): waits
 // until the launch before it in the stream has completed and its memory is
 // visible.  Every path through such a kernel passes here, so the kernels still
