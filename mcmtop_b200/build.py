@@ -34,7 +34,7 @@ UNITS = [
     ("batch.cu", False),
     ("transfer.cu", False),
 ]
-HEADERS = ["common.cuh", "kernels.h", "handle.h", "physics.cuh", "step_fp64.cuh", "step_coop.cuh", "step_exact.cuh", "time_step.cuh", "nbr_iter.cuh", "dual.cuh"]
+HEADERS = ["common.cuh", "kernels.h", "handle.h", "physics.cuh", "step_fp64.cuh", "step_coop.cuh", "step_exact.cuh", "quotient.cuh", "time_step.cuh", "nbr_iter.cuh", "dual.cuh"]
 
 
 def _newer(target: str, deps: list[str]) -> bool:

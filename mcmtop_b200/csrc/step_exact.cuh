@@ -9,16 +9,14 @@
 // order.  A thread that owns a particle alone walks a chain of 80 square roots
 // and divisions, 62 us at the least however few particles there are.
 //
-// Bound: the latency of the FP64 chain and then the FP64 pipe.  Divisions by a number that several quotients share
-// (h, the gradient's denominator, the corrected form's sum squared) multiply
-// by its correctly rounded reciprocal and correct the quotient twice
-// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990: from a quotient within one ulp and a correctly rounded
-// reciprocal the fused-multiply-add correction rounds correctly), so every
-// quotient is the one that the division gives.
+// Bound: the latency of the FP64 chain and then the FP64 pipe.  Divisions by a
+// number that several quotients share (h, the gradient's denominator, the
+// corrected form's sum squared) multiply by its reciprocal and correct the
+// quotient (quotient.cuh), so every quotient is the one that the division gives.
 #pragma once
 #include "nbr_iter.cuh"
 #include "physics.cuh"
+#include "quotient.cuh"
 
 namespace mcm {
 namespace MCM_FLAVOUR_NS {
@@ -36,24 +34,6 @@ constexpr int seq_threads(int lanes) { return lanes == 1 ? 128 : 256; }
 // Neighbours whose records a lane fetches ahead, and the blocks an SM is to hold.
 constexpr int seq_ahead(int lanes) { return lanes == 1 ? 1 : 2; }
 constexpr int seq_blocks(int disc, int lanes) { return lanes == 1 ? (disc ? 4 : 5) : 2; }
-
-// a / b, y = RN(1 / b), for a and b well inside the exponent range (in_range).
-__device__ __forceinline__ double quotient(double a, double b, double y) {
-    double q = a * y;
-    double r = fma(-b, q, a);
-    q = fma(r, y, q);
-    r = fma(-b, q, a);
-    return fma(r, y, q);
-}
-// |v| in about [2^-500, 2^500], or zero: neither the quotient nor the
-// remainders of `quotient` overflow or lose bits.
-__device__ __forceinline__ bool in_range(double v) {
-    const unsigned h = (unsigned)__double2hiint(v) << 1;
-    return h - (523u << 21) < (1000u << 21) || (h | (unsigned)__double2loint(v)) == 0u;
-}
-__device__ __forceinline__ double divide(double a, double b, double y) {
-    return in_range(a) && in_range(b) ? quotient(a, b, y) : a / b;
-}
 
 // What a particle's own h gives every pair with a neighbour of the same h.
 struct OwnH {
@@ -94,7 +74,7 @@ __device__ __forceinline__ void pair_kernel(double x0, double x1, double x2, con
     }
     const double den = rad * havg;
     const double n0 = dw * x0, n1 = dw * x1, n2 = dw * x2;
-    if (in_range(den) && in_range(n0) && in_range(n1) && in_range(n2)) {
+    if (divisor_in_range(den) && dividend_in_range(n0) && dividend_in_range(n1) && dividend_in_range(n2)) {
         const double y = 1.0 / den;
         d[0] = quotient(n0, den, y);
         d[1] = quotient(n1, den, y);
