@@ -308,7 +308,7 @@ int mcm_gpu_adjoint_backward(mcm_gpu_handle *h, const double *xbar, const double
  * combined over a different number of block partials.  Zero fields keep the
  * current value. */
 typedef struct {
-    int search_threads;      /* threads per block of the search: 64 or 128 (256 runs as 128) */
+    int search_threads;      /* threads per block of the search: 64, 128 or 256 */
     int pair_threads;        /* threads per block of the gathers: 64, 128 or 256 */
     int pair_blocks_per_sm;  /* blocks per SM the gathers' persistent grid is sized for: 1..16 (reported as
                                 0 while it is the blocks resident per SM, the default) */

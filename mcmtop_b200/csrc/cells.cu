@@ -995,9 +995,10 @@ __device__ __forceinline__ void list_overflow(const StepArgs &a, int i, int nn, 
 // for the next mask the whole warp moves the collected entries on, eight lanes
 // to a particle, each with one 16-byte store per four entries (rows start at
 // multiples of 4); up to three stay behind.
+constexpr int kSearchThreads = 256;   // the most a block of a search may have (128 unless the caller asks)
 constexpr int kSrchKeep = 36;   // entries a lane can hold
 template <int V>
-__global__ void __launch_bounds__(128, 8) k_search(StepArgs a) {
+__global__ void __launch_bounds__(kSearchThreads, 4) k_search(StepArgs a) {
     chain_wait();
     constexpr bool contact = (V & kSrchContact) != 0;   // contacttype > 0: other materials -> contact list
     constexpr bool two_pass = (V & kSrchTwoPass) != 0;  // kernel contact between materials: own material first
@@ -1123,7 +1124,7 @@ __global__ void __launch_bounds__(128, 8) k_search(StepArgs a) {
 // The three rows of a plane are decided before any is written, so that their
 // loads overlap.
 template <int V, int G>
-__global__ void __launch_bounds__(128, 6) k_search_lanes(StepArgs a) {
+__global__ void __launch_bounds__(kSearchThreads, 3) k_search_lanes(StepArgs a) {
     chain_wait();
     constexpr bool contact = (V & kSrchContact) != 0;
     constexpr bool two_pass = (V & kSrchTwoPass) != 0;
@@ -1769,7 +1770,7 @@ static void launch_lanes(const StepArgs &a, int threads, cudaStream_t s) {
 }
 template <int V>
 static void launch_search_v(const StepArgs &a, cudaStream_t s) {
-    const int threads = search_threads_of(a) < 128 ? search_threads_of(a) : 128;
+    const int threads = search_threads_of(a);
     const long long n = (long long)a.n * a.share;
     if (a.search_kind == 2 || n < kSearch8Below) launch_lanes<V, 8>(a, threads, s);
     else if (n < kSearch4Below) launch_lanes<V, 4>(a, threads, s);
