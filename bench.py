@@ -87,7 +87,7 @@ def parse():
                     help="run only the long accuracy run on this device and print its JSON (the child process "
                          "that the long-run leg starts)")
     ap.add_argument("--search-kind", type=int, default=0, choices=[0, 1, 2, 3],
-                    help="neighbour search: 1 one thread per particle, 2 one warp per particle, 3 one warp per cell (0: default)")
+                    help="neighbour search: 1 lanes per particle by size, 2 eight lanes per particle, 3 one warp per cell (0: default)")
     return ap.parse_args()
 
 

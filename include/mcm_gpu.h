@@ -381,7 +381,10 @@ int mcm_gpu_set_diagnostics(mcm_gpu_handle *h, int enable);
  * its only timing is the commented-out MCM/mcm_write_timings.f90. */
 int mcm_gpu_profile(mcm_gpu_handle *h, int enable);
 /* Device time and launches of kernel group `region` (0..14) since
- * mcm_gpu_profile; returns MCM_EINVAL past the last group. */
+ * mcm_gpu_profile; returns MCM_EINVAL past the last group.  Groups 3 and 6
+ * (strain_prep, critts_dt) are empty: the strain records are written with the
+ * cell list and the ghosts, the critical timestep is formed by the
+ * constitutive update. */
 int mcm_gpu_profile_report(mcm_gpu_handle *h, int region, char *name, int name_len, double *total_ms,
                            int *launches);
 /* Kernels launched by this handle since the last mcm_gpu_profile call. */

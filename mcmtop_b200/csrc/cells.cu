@@ -1,5 +1,5 @@
-// cells.cu -- device cell list, boundary ghosts and the warp-cooperative
-// neighbour search of the MCM explicit step.
+// cells.cu -- device cell list, boundary ghosts and the neighbour search of
+// the MCM explicit step.
 //
 // Replaces MCM/mcm_setuplist.f90 (linked-list grid), MCM/mcm_ghost_setup.f90
 // (ghost particles) and MCM/mcm_ll_neighbours.f90 (27-cell search).  The cell
@@ -988,7 +988,8 @@ __device__ __forceinline__ void list_overflow(const StepArgs &a, int i, int nn, 
     }
 }
 
-// One thread per particle (bodies that fill the chip).  The lanes of a warp walk
+// One thread per particle (bodies that fill the chip; 64 registers for 32 warps
+// per SM, with 52 to 72 bytes spilled).  The lanes of a warp walk
 // the nine rows together (they lie in one or two cells, so their rows mostly
 // are the same ones), 32 candidates to a mask, and collect their entries in
 // shared memory, entry k of lane l at word 33 k + l.  When a lane has no room
@@ -1119,7 +1120,7 @@ __global__ void __launch_bounds__(kSearchThreads, 4) k_search(StepArgs a) {
 }
 
 // G lanes per particle (bodies too small to fill the chip with one thread per
-// particle).  A row's three cells are one contiguous range; each lane takes a
+// particle; 80 registers, 72 to 132 bytes spilled).  A row's three cells are one contiguous range; each lane takes a
 // run of its groups, and the lanes' counts give each where its entries begin.
 // The three rows of a plane are decided before any is written, so that their
 // loads overlap.
@@ -1292,8 +1293,10 @@ __global__ void __launch_bounds__(kSearchThreads, 3) k_search_lanes(StepArgs a) 
 // row's contiguous candidate range is staged 32 records at a time in shared
 // memory by one coalesced load per lane and then read by every lane as a
 // broadcast, so the inner loop has no global load.  Candidates are visited in
-// k_search's order and tested with its FP32 decision and FP64 tie test, so
-// the lists are k_search's, entry for entry.
+// k_search's order.  The FP32 decision is its own: coordinates relative to the
+// cells (cposf) and a band of 2^-12 of the cutoff and of the cell's square; the
+// band is left to the same FP64 expression, so the lists are k_search's, entry
+// for entry.
 constexpr int kCellWarps = 8;
 __global__ void __launch_bounds__(kCellWarps * 32, 3) k_search_cell(StepArgs a) {
     chain_wait();
@@ -1501,8 +1504,8 @@ __global__ void __launch_bounds__(kCellWarps * 32, 3) k_search_cell(StepArgs a) 
 // at the build; while every particle has moved less than skin/2 since then,
 // it is still at least h_i + h_j apart, so it cannot be a neighbour.  The
 // step rebuilds the skin lists when the largest displacement reaches skin/2
-// (or on request), and filters them every step with k_search's FP32 decision
-// and FP64 tie test, among the candidates in the 27 cells around the
+// (or on request), and filters them every step with k_search_cell's FP32
+// decision and the FP64 tie test, among the candidates in the 27 cells around the
 // particle's cell of the current grid (the only ones the reference examines),
 // so the neighbour sets are the reference's; their order is the skin list's.
 
@@ -1605,7 +1608,7 @@ __global__ void __launch_bounds__(256) k_skin_build(StepArgs a) {
     }
 }
 
-// The step's neighbour lists from the skin lists: k_search's decisions on
+// The step's neighbour lists from the skin lists: k_search_cell's decisions on
 // the candidates that lie in the 27 cells around the particle's cell, in
 // skin-list order; ghosts, contacts, minimum distances and counts as k_search.
 __global__ void __launch_bounds__(256, 4) k_skin_filter(StepArgs a) {
@@ -1757,12 +1760,14 @@ void launch_skin_search(const StepArgs &a, cudaStream_t s) {
 }
 
 // Lanes per particle of the search: one thread per particle is the cheapest
-// walk where it fills the chip, but its chain of nine rows takes 65 us however
+// walk where it fills the chip, but its chain of nine rows takes 62 us however
 // few particles there are.  Measured (us a search, 1 / 4 / 8 lanes, taylor
-// bars, mixed): 16 848 particles 62 / 48 / 34, 38 880: 70 / 53 / 55, 68 120:
-// 75 / 68 / 85, 131 544: 89 / 115 / 152, 685 824: 340 / 546 / 766.  Bodies of a
-// batch fill the chip together, so the particles of all that run at the same
-// time count.
+// bars, mixed): 16 848 particles 62 / 48 / 34, 38 880: 70 / 53 / 55, 685 824:
+// 340 / 546 / 766.  Around the line between four lanes and one (1 / 4): 62 484:
+// 72 / 62, 68 120: 72 / 65, 80 592: 76 / 72, 91 008: 77 / 80, 131 544: 86 / 108.
+// The two meet near 85 000: the line is on the safe side of that, and bodies
+// between the two pay up to 8 us.  Bodies of a batch fill the chip together, so
+// the particles of all that run at the same time count.
 constexpr int kSearch8Below = 24000, kSearch4Below = 64000;
 template <int V, int G>
 static void launch_lanes(const StepArgs &a, int threads, cudaStream_t s) {

@@ -154,7 +154,7 @@ __host__ __device__ inline float search_band(int n, float cell) {
 // chain_start, of the short kernels, then lets the launch behind it begin, so
 // that its blocks are in place when this kernel ends.  The searches, gathers
 // and the constitutive update only wait (chain_wait): blocks that wait beside
-// them cost more than the launch (685 824 particles: 100.3 ms against 96.7).
+// them cost more than the launch (685 824 particles: 100.6 ms against 96.7).
 __device__ __forceinline__ void chain_start() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

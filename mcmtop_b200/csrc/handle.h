@@ -94,7 +94,10 @@ inline int dalloc(mcm_gpu_handle *h, T **p, size_t count) {
 
 inline int round_up(int x, int m) { return ((x + m - 1) / m) * m; }
 
-// Kernel groups that the profiler times separately.
+// Kernel groups that the profiler times separately.  The strain records and the
+// critical timestep have no launches of their own (they are part of R_CELLS,
+// R_GHOSTS and of R_CONST): their groups stay empty and keep the numbering, by
+// which callers ask for a group.
 enum Region {
     R_CELLS = 0, R_GHOSTS, R_SEARCH, R_STRAIN_PREP, R_STRAIN, R_CONST, R_CRITTS, R_MOM_PREP, R_MOMENTUM,
     R_REDUCE, R_MOVE, R_MISC, R_ADJ_MOM, R_ADJ_CONST, R_ADJ_STRAIN, R_NREG

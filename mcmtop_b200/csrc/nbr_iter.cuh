@@ -35,8 +35,7 @@ __device__ __forceinline__ int stored_neighbours(const StepArgs &a, int t) {
 
 // FR: void(int position, bool is_self); FG: void(int ghost)
 template <typename FR, typename FG>
-__device__ __forceinline__ void for_each_neighbour(const StepArgs &a, const DevGrid &g, int t, FR &&real, FG &&ghost) {
-    (void)g;
+__device__ __forceinline__ void for_each_neighbour(const StepArgs &a, int t, FR &&real, FG &&ghost) {
     const unsigned *list = a.nidx + (size_t)t * a.nstride;
     const int nreal = stored_neighbours(a, t);
     for (int k = 0; k < nreal; ++k) real((int)(list[k] & kPosMask), false);

@@ -73,8 +73,6 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_strain_coop(StepArgs
     const int sub = threadIdx.x / L, lane = threadIdx.x % L;
     const int per = blockDim.x / L;
     const int rounds = (a.n + per * gridDim.x - 1) / (per * gridDim.x);
-    const DevGrid g = *a.grid;
-    (void)g;
     for (int round = 0; round < rounds; ++round) {
     const int t = (round * gridDim.x + blockIdx.x) * per + sub;
     const bool live = t < a.n;
@@ -200,7 +198,8 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_strain_coop(StepArgs
 // 1.58 against 1.87 ms for the strain gather above).  Records come in 32-byte
 // loads and real neighbours in a loop of their own: strain 437 -> 413 us,
 // momentum 590 -> 561 us on the 685 824-particle bar (one thread per particle
-// measured 382 and 561, two neighbours ahead 433 and 553).
+// measured 382 and 561, two neighbours ahead 433 and 553).  At 64 registers the
+// momentum gather spills 240 bytes a thread.
 template <int L, int DISC, bool ASYM>
 __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepArgs a, int integrate) {
     chain_wait();
@@ -209,8 +208,6 @@ __global__ void __launch_bounds__(256, DISC == 0 ? 4 : 1) k_momentum_coop(StepAr
     const int sub = threadIdx.x / L, lane = threadIdx.x % L;
     const int per = blockDim.x / L;
     const int rounds = (a.n + per * gridDim.x - 1) / (per * gridDim.x);
-    const DevGrid g = *a.grid;
-    (void)g;
     const int nm = a.nmat;
     // sums of material 1 in registers; other materials go to the block's partials
     double e1[5] = {0.0, 0.0, 0.0, 0.0, 0.0};

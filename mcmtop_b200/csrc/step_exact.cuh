@@ -26,9 +26,11 @@ namespace MCM_FLAVOUR_NS {
 // handing terms over.  Measured (us, strain / momentum, 8 lanes and 1; the
 // walk before, one thread per particle with a division per quotient, in
 // brackets): 2 080 particles 19/22 and 62/64 (83/88), 16 848: 37/40 and 66/66
-// (93/102), 38 880: 72/81 and 74/79, 131 544: 209/238 and 151/181 (177/206),
-// 685 824: 1092/1180 and 602/705 (796/946).  Corrected form, 68 120: 357/395
-// and 242/265 (339/367).
+// (93/102), 35 192: 64/69 and 68/72, 41 360: 76/81 and 72/77, 131 544: 209/238
+// and 151/181 (177/206), 685 824: 1092/1180 and 602/705 (796/946).  The
+// corrected form meets a little later, at the same line for all that: 35 192:
+// 184/206 and 213/229, 41 360: 223/238 and 228/247, 47 328: 238/256 and
+// 229/246, 68 120: 357/395 and 242/265 (339/367).
 constexpr int kSeqLanesBelow = 36000;
 constexpr int seq_threads(int lanes) { return lanes == 1 ? 128 : 256; }
 // Neighbours whose records a lane fetches ahead, and the blocks an SM is to hold.

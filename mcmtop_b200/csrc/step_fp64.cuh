@@ -1,14 +1,13 @@
-// step_fp64.cuh -- FP64 kernels of the MCM explicit step: strain-rate gather
-// fused with the constitutive update and the critical-timestep reduction, and
-// the momentum gather fused with boundary conditions, energy sums, velocity
-// update and position update.
+// step_fp64.cuh -- FP64 kernels of the MCM explicit step with one thread per
+// particle: the constitutive update, which forms the critical timestep and the
+// momentum gather's records too, repulsive contact, the split path's and XSPH's
+// velocity and position updates, and the initial state.
 //
 // Included by two translation units: MCM_FLAVOUR_EXACT (compiled without
 // fused multiply-add; reference expression order and divisions, so the
 // result follows the reference arithmetic) and MCM_FLAVOUR_FAST (fused
-// multiply-add and reciprocals).  Each thread owns one particle and walks its
-// neighbours in the reference order; the sums are sequential, so there are no
-// atomics and the FP64-exact flavour accumulates in the reference's order.
+// multiply-add and reciprocals).  The strain and momentum gathers are those of
+// step_exact.cuh (terms added in the reference's order) and step_coop.cuh.
 #pragma once
 #include "nbr_iter.cuh"
 #include "physics.cuh"
@@ -276,7 +275,10 @@ __device__ __forceinline__ void update_h(const StepArgs &a, int i, PState<double
 // registers and no loads of what they do not read, run three blocks per SM (80
 // registers).  685 824 particles, all models / one with two blocks / one with
 // three: 123 / 101 / 98 us (mixed), 132 / 112 / 102 us (FP64), and 38 880 mixed
-// 20 / 19 / 19.
+// 20 / 19 / 19.  The 80 registers spill 230 to 300 bytes a thread, the 128 of the
+// kernel for all models 150 to 240 besides the 512 bytes of the cap model's
+// arrays.  Bodies of model 1, 3 or 4 alone take the kernel for all models, as
+// those of several models do: no instance of theirs has been measured.
 //
 // Writes the momentum gather's records of the particle, at its position in cell
 // order, and of its ghosts too: whole 32-byte sectors, while the state they are
@@ -560,7 +562,7 @@ __global__ void k_xsph_sum(StepArgs a) {
         sv[2] = sv[2] + volj * (vj2 - vi[2]) * w;
     };
     for_each_neighbour(
-        a, *a.grid, t,
+        a, t,
         [&](int p, bool) {
             const int j = a.cell_list[p];
             body(f[FX][j], f[FY][j], f[FZ][j], f[FVX][j], f[FVY][j], f[FVZ][j], f[FMASS][j], f[FRHO][j], f[FH][j]);
