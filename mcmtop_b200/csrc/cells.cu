@@ -313,6 +313,71 @@ __device__ __forceinline__ void write_records(const StepArgs &a, const DevGrid &
 
 constexpr int kSortPer = 4;
 template <int REC>
+__device__ __forceinline__ void order_cell(const StepArgs &a, const DevGrid &g, int c, int s, int e, double dt,
+                                           bool with_cposf, unsigned long long &hbits, unsigned long long &lbits) {
+    const int lane = threadIdx.x & 31, n = e - s;
+    if (n <= 32) {
+        // one particle per lane (the common case)
+        const bool on = lane < n;
+        const int v = on ? a.cell_list[s + lane] : 0;
+        const int o = on ? a.F.orig[v] : 0;
+        int rank = 0;
+        for (int k = 0; k < n; ++k) rank += __shfl_sync(0xffffffffu, o, k) > o ? 1 : 0;
+        __syncwarp();
+        if (on) {
+            a.cell_list[s + rank] = v;
+            write_records<REC>(a, g, s + rank, v, c, dt, with_cposf, hbits, lbits);
+        }
+        __syncwarp();
+        return;
+    }
+    if (n <= 32 * kSortPer) {
+        int v[kSortPer], o[kSortPer], rank[kSortPer];
+#pragma unroll
+        for (int u = 0; u < kSortPer; ++u) {
+            const int j = lane + 32 * u;
+            v[u] = j < n ? a.cell_list[s + j] : 0;
+            o[u] = j < n ? a.F.orig[v[u]] : 0;
+            rank[u] = 0;
+        }
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            // the chunk's keys, one per lane, broadcast by shuffles
+            const int uk = k0 >> 5;
+            int ok = 0;
+#pragma unroll
+            for (int u = 0; u < kSortPer; ++u)
+                if (u == uk) ok = o[u];
+            const int m = n - k0 < 32 ? n - k0 : 32;
+            for (int k = 0; k < m; ++k) {
+                const int ob = __shfl_sync(0xffffffffu, ok, k);
+#pragma unroll
+                for (int u = 0; u < kSortPer; ++u)
+                    if (lane + 32 * u < n && ob > o[u]) ++rank[u];
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < kSortPer; ++u)
+            if (lane + 32 * u < n) a.cell_list[s + rank[u]] = v[u];
+    } else if (lane == 0) {
+        for (int k = s + 1; k < e; ++k) {
+            const int v = a.cell_list[k];
+            const int ov = a.F.orig[v];
+            int m = k - 1;
+            while (m >= s && a.F.orig[a.cell_list[m]] < ov) {
+                a.cell_list[m + 1] = a.cell_list[m];
+                --m;
+            }
+            a.cell_list[m + 1] = v;
+        }
+    }
+    __syncwarp();
+    for (int p = s + lane; p < e; p += 32)
+        write_records<REC>(a, g, p, a.cell_list[p], c, dt, with_cposf, hbits, lbits);
+    __syncwarp();
+}
+
+template <int REC>
 __global__ void __launch_bounds__(256) k_cell_order(StepArgs a, int with_cposf) {
     chain_start();
     __shared__ DevGrid g;
@@ -325,68 +390,16 @@ __global__ void __launch_bounds__(256) k_cell_order(StepArgs a, int with_cposf) 
     const int lane = threadIdx.x & 31;
     const unsigned nw = gridDim.x * (blockDim.x >> 5);
     unsigned long long hbits = 0ull, lbits = ~0ull;
-    for (unsigned c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += nw) {
-        const int s = a.cell_start[c], e = a.cell_start[c + 1];
-        const int n = e - s;
-        if (n <= 32) {
-            // one particle per lane (the common case)
-            const bool on = lane < n;
-            const int v = on ? a.cell_list[s + lane] : 0;
-            const int o = on ? a.F.orig[v] : 0;
-            int rank = 0;
-            for (int k = 0; k < n; ++k) rank += __shfl_sync(0xffffffffu, o, k) > o ? 1 : 0;
-            __syncwarp();
-            if (on) {
-                a.cell_list[s + rank] = v;
-                write_records<REC>(a, g, s + rank, v, c, dt, with_cposf != 0, hbits, lbits);
-            }
-            __syncwarp();
-            continue;
+    // a warp takes every nw-th cell and reads the ends of 32 of them at once: of a
+    // sparse grid only the cells that hold particles are walked
+    for (unsigned c0 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c0 < ncells; c0 += 32u * nw) {
+        const unsigned c = c0 + lane * nw;
+        const int s = c < ncells ? a.cell_start[c] : 0, e = c < ncells ? a.cell_start[c + 1] : 0;
+        for (unsigned todo = __ballot_sync(0xffffffffu, e > s); todo; todo &= todo - 1u) {
+            const int at = __ffs(todo) - 1;
+            order_cell<REC>(a, g, (int)(c0 + at * nw), __shfl_sync(0xffffffffu, s, at), __shfl_sync(0xffffffffu, e, at), dt,
+                            with_cposf != 0, hbits, lbits);
         }
-        if (n <= 32 * kSortPer) {
-            int v[kSortPer], o[kSortPer], rank[kSortPer];
-#pragma unroll
-            for (int u = 0; u < kSortPer; ++u) {
-                const int j = lane + 32 * u;
-                v[u] = j < n ? a.cell_list[s + j] : 0;
-                o[u] = j < n ? a.F.orig[v[u]] : 0;
-                rank[u] = 0;
-            }
-            for (int k0 = 0; k0 < n; k0 += 32) {
-                // the chunk's keys, one per lane, broadcast by shuffles
-                const int uk = k0 >> 5;
-                int ok = 0;
-#pragma unroll
-                for (int u = 0; u < kSortPer; ++u)
-                    if (u == uk) ok = o[u];
-                const int m = n - k0 < 32 ? n - k0 : 32;
-                for (int k = 0; k < m; ++k) {
-                    const int ob = __shfl_sync(0xffffffffu, ok, k);
-#pragma unroll
-                    for (int u = 0; u < kSortPer; ++u)
-                        if (lane + 32 * u < n && ob > o[u]) ++rank[u];
-                }
-            }
-            __syncwarp();
-#pragma unroll
-            for (int u = 0; u < kSortPer; ++u)
-                if (lane + 32 * u < n) a.cell_list[s + rank[u]] = v[u];
-        } else if (lane == 0) {
-            for (int k = s + 1; k < e; ++k) {
-                const int v = a.cell_list[k];
-                const int ov = a.F.orig[v];
-                int m = k - 1;
-                while (m >= s && a.F.orig[a.cell_list[m]] < ov) {
-                    a.cell_list[m + 1] = a.cell_list[m];
-                    --m;
-                }
-                a.cell_list[m + 1] = v;
-            }
-        }
-        __syncwarp();
-        for (int p = s + lane; p < e; p += 32)
-            write_records<REC>(a, g, p, a.cell_list[p], c, dt, with_cposf != 0, hbits, lbits);
-        __syncwarp();
     }
     // particles outside the grid
     for (int p = a.cell_start[ncells] + blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x)
@@ -417,14 +430,26 @@ static int grid_blocks(long long work, int threads) {
 }
 
 // Four launches: keys and counts, their scan, the scatter, the order within
-// the cells with everything that is written per particle in cell order.
+// the cells with everything that is written per particle in cell order.  All
+// but the scan loop over the cells as well as over the particles, and a few
+// particles may lie in a large grid: their blocks follow both, the cells by
+// the arrays' length (the host does not know the grid).  At the most 4 cells to
+// a thread of the short kernels and 16 to a warp that orders them, up to the
+// full chip.  (us a cell list, with blocks by the particles alone and a cell at
+// a time, and now: 2 080 particles in 153 cells 23 and 20, in 54 972 264 and 24,
+// in 4 million 18 700 and 122; 16 848 in 1 152 25 and 21, in 55 440 54 and 26;
+// 685 824 in 53 240 71 and 72; 450 604 in 117 120 61 and 55.)
+static int blocks_for(long long particles, long long cells) {
+    const long long b = grid_blocks(particles, 256) > cells ? grid_blocks(particles, 256) : cells;
+    return (int)(b < 148 * 8 ? b : 148 * 8);
+}
 void launch_cell_build(const StepArgs &a, cudaStream_t s) {
-    const int wide = grid_blocks(a.n, 256) < 148 * 8 ? grid_blocks(a.n, 256) : 148 * 8;
+    const int wide = blocks_for(a.n, a.cell_cap / (4 * 256));
     launch_chained(k_cell_keys, wide, 256, 0, s, a);
     launch_chained(k_cell_scan, (unsigned)((a.cell_cap + kScanChunk - 1) / kScanChunk), kScanThreads, 0, s, a);
     launch_chained(k_cell_scatter, wide, 256, 0, s, a);
-    // about 8 particles to a lane's warp at the least: a warp per cell of a full body
-    const int ob = grid_blocks((long long)a.n * 2, 256) < 148 * 8 ? grid_blocks((long long)a.n * 2, 256) : 148 * 8;
+    // about 16 particles to a warp, a cell of a full body
+    const int ob = blocks_for((long long)a.n * 2, a.cell_cap / (16 * 8));
     const int with_cposf = a.search_kind == 3 || a.prm.skin > 0.0 ? 1 : 0;
     if (a.frec0) launch_chained(k_cell_order<kRecMixed>, ob, 256, 0, s, a, with_cposf);
     else launch_chained(k_cell_order<kRecFP64>, ob, 256, 0, s, a, with_cposf);
