@@ -160,6 +160,17 @@ int alloc_particles(mcm_gpu_handle *h) {
     return MCM_OK;
 }
 
+// Scratch for the planes' layer cells: as many as the grid's cells at first,
+// twice as many, which is the most there can be, once a thin grid asks for it.
+int alloc_layers(mcm_gpu_handle *h, long long cap) {
+    int st;
+    h->A.layer_cap = h->A.prm.boundary ? (unsigned)std::min<long long>(cap, (1LL << 32) - 1) : 1u;
+    if ((st = dalloc(h, &h->A.layer_count, 2 * (size_t)h->A.layer_cap + scan_chunks(h->A.layer_cap) + 1))) return st;
+    h->A.layer_off = h->A.layer_count + h->A.layer_cap;
+    h->A.layer_sums = h->A.layer_off + h->A.layer_cap;
+    return MCM_OK;
+}
+
 int alloc_cells(mcm_gpu_handle *h, long long cap) {
     int st;
     h->A.cell_cap = cap;
@@ -170,12 +181,7 @@ int alloc_cells(mcm_gpu_handle *h, long long cap) {
     long long nsum = (cap + 4095) / 4096 + 2;
     if ((st = dalloc(h, &h->A.scan_sums, (size_t)nsum))) return st;
     if ((st = dalloc(h, &h->A.gcell, (size_t)cap))) return st;
-    // the planes' layers hold at most twice the grid's cells (a grid has less than 2^31)
-    h->A.layer_cap = h->A.prm.boundary ? (unsigned)std::min<long long>(2 * cap, (1LL << 32) - 1) : 1u;
-    if ((st = dalloc(h, &h->A.layer_count, 2 * (size_t)h->A.layer_cap + scan_chunks(h->A.layer_cap) + 1))) return st;
-    h->A.layer_off = h->A.layer_count + h->A.layer_cap;
-    h->A.layer_sums = h->A.layer_off + h->A.layer_cap;
-    return MCM_OK;
+    return alloc_layers(h, cap);
 }
 
 int alloc_ghosts(mcm_gpu_handle *h, int cap) {
@@ -289,6 +295,11 @@ int regrow(mcm_gpu_handle *h, int *grew) {
             break;
         }
         case MCM_EGRID_OVERFLOW: {
+            if (s.req_cells <= h->A.cell_cap) {   // the grid has room, its planes' layers have not
+                if ((st = alloc_layers(h, 2 * h->A.cell_cap))) return st;
+                *grew = 1;
+                break;
+            }
             long long need = std::max<long long>(s.req_cells, h->A.cell_cap * 2);
             long long cap = need + need / 2 + 1024;
             if ((st = alloc_cells(h, cap))) return st;
