@@ -160,6 +160,7 @@ __global__ void k_set_time(StepArgs a, double dt, double dtold, int set_dtold) {
     chain_start();
     a.time->dt = dt;
     if (set_dtold) a.time->dtold = dtold;
+    a.time->ended = 0;   // the caller's loop decides when it ends; a fused run before it may have ended
 }
 
 void launch_init_critts_reduce(const StepArgs &a, cudaStream_t s, int nblocks) {
